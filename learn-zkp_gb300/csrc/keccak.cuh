@@ -314,35 +314,38 @@ __device__ __forceinline__ Digest digest_bytes(const Digest& d) {
 // ---------------------------------------------------------------------------
 // Keccak-f[1600] spread over a warp, for latency-bound hashing (the top
 // levels of a Merkle tree, the transcript): lane j < 25 holds state word
-// A[x][y], j = x + 5y; lanes 25..31 only take part in the shuffles.  One
-// round is nine 64-bit shuffles (theta column sums and neighbours, pi, chi)
-// and a per-lane rotation.  Measured on GB300: 2.9 us per permutation on one
-// warp, against 4.25 us for one thread (whose ~4450 instructions issue at
-// the half-rate ALU pipe's pace) — so it pays only when each warp has a
-// single permutation to do (a level of at most as many nodes as warps).
+// A[x][y], j = x + 5y; lanes 25..31 only take part in the shuffles.  A round
+// is three dependent shuffle stages: theta's column sum (the other four words
+// of the column), theta's neighbour columns, and pi with chi, which reads the
+// three rotated words that end up in a row straight from the lanes that
+// rotated them.  Measured on GB300 (one block, clock64): 3,920 cycles per
+// permutation on one warp per scheduler and 4,250 on two, against 4,680 and
+// 5,140 with pi and chi as stages of their own.  A shuffle issues about every
+// 4.4 cycles per scheduler, so four warps per scheduler (7,650 cycles) are
+// bound by its 18 shuffles per round; a whole permutation on one thread takes
+// 8,500 cycles (its 173 instructions per round issue at the half-rate ALU
+// pipe's pace) and on a pair of lanes 5,330 (PairKeccak), so a level runs one
+// warp per node only while it has at most two nodes per scheduler.
 struct WarpKeccak {
-  int lane, x, y;
-  int col[4];      // theta: the other four lanes of this column
-  int xm1, xp1;    // theta: lanes of columns x-1, x+1 in this row
-  int pi_src;      // pi: B[x][y] = A[x'][y'] with x = y', y = 2x' + 3y'
-  int chi1, chi2;  // chi: lanes of columns x+1, x+2 in this row
-  int rho;         // rotation of this lane
+  int lane;
+  int col[4];            // theta: the other four lanes of this column
+  int xm1, xp1;          // theta: lanes of columns x-1, x+1 in this row
+  int src0, src1, src2;  // pi and chi: the lanes whose rotated words become B[x], B[x+1], B[x+2] of this row
+  int rho;               // rotation of this lane, applied before pi moves the word
 
   __device__ __forceinline__ WarpKeccak() {
     lane = threadIdx.x & 31;
     const int j = lane < 25 ? lane : 0;
-    x = j % 5;
-    y = j / 5;
+    const int x = j % 5, y = j / 5;
 #pragma unroll
     for (int k = 0; k < 4; ++k) col[k] = x + 5 * ((y + 1 + k) % 5);
     xm1 = (x + 4) % 5 + 5 * y;
     xp1 = (x + 1) % 5 + 5 * y;
-    // lane (X, Y) receives A[x'][y'] with y' = X, x' = 3 (Y - 3X) mod 5
-    const int xs = (3 * ((y - 3 * x) % 5 + 5)) % 5;
-    pi_src = xs + 5 * x;
-    chi1 = (x + 1) % 5 + 5 * y;
-    chi2 = (x + 2) % 5 + 5 * y;
-    // rotation of A[x][y] (FIPS 202 rho offsets), applied before pi moves it
+    // B[X][y] = A[x'][X] with x' = 3 (y - 3X) mod 5 (pi: x = y', y = 2x' + 3y')
+    auto pi_lane = [&](int X) { return (3 * ((y - 3 * X) % 5 + 10)) % 5 + 5 * X; };
+    src0 = pi_lane(x);
+    src1 = pi_lane((x + 1) % 5);
+    src2 = pi_lane((x + 2) % 5);
     constexpr int kRho[25] = {0,  1,  62, 28, 27, 36, 44, 6,  55, 20, 3,  10, 43,
                               25, 39, 41, 45, 15, 21, 8,  18, 2,  61, 56, 14};
     int r = 0;
@@ -355,48 +358,211 @@ struct WarpKeccak {
   static __device__ __forceinline__ uint2 shfl(uint2 v, int src) {
     return make_uint2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
   }
-  static __device__ __forceinline__ uint2 rolv(uint2 v, int r) {
-    if (r & 32) v = make_uint2(v.y, v.x);
-    const int s = r & 31;
-    return make_uint2(__funnelshift_l(v.y, v.x, s), __funnelshift_l(v.x, v.y, s));
-  }
-  // the same on an interleaved lane
-  static __device__ __forceinline__ uint2 rolv_bi(uint2 v, int r) {
-    if (r & 1) return make_uint2(rotl32(v.y, (r + 1) >> 1), rotl32(v.x, r >> 1));
-    return make_uint2(rotl32(v.x, r >> 1), rotl32(v.y, r >> 1));
-  }
 
   // All 32 lanes call this; `a` is this lane's word (interleaved when BI).
   template <bool BI>
   __device__ __forceinline__ uint2 permute(uint2 a) const {
-#pragma unroll 1
+    // the lane's rotation: swap the halves or not, then a 32-bit (BI) or a
+    // funnel shift per half
+    const bool swap = BI ? (rho & 1) != 0 : (rho & 32) != 0;
+    const int k0 = BI ? (rho + 1) >> 1 : rho & 31, k1 = BI ? rho >> 1 : rho & 31;
+#pragma unroll 4
     for (int r = 0; r < 24; ++r) {
+      uint2 rc = keccak_rc<BI>(r);
+      if (lane != 0) rc = make_uint2(0, 0);
       const uint2 c1 = shfl(a, col[0]), c2 = shfl(a, col[1]), c3 = shfl(a, col[2]), c4 = shfl(a, col[3]);
       const uint2 c = kx5(a, c1, c2, c3, c4);  // C[x]
       const uint2 cm = shfl(c, xm1), cp = shfl(c, xp1);
-      a = kx3(a, cm, krot<1, BI>(cp));         // theta
-      a = BI ? rolv_bi(a, rho) : rolv(a, rho);  // rho
-      const uint2 b = shfl(a, pi_src);         // pi
-      const uint2 b1 = shfl(b, chi1), b2 = shfl(b, chi2);
-      a = kchi(b, b1, b2);                     // chi
-      if (lane == 0) a = kx2(a, keccak_rc<BI>(r));  // iota
+      const uint2 t = kx3(a, cm, krot<1, BI>(cp));  // theta
+      const uint32_t u = swap ? t.y : t.x, v = swap ? t.x : t.y;
+      const uint2 q = BI ? make_uint2(rotl32(u, k0), rotl32(v, k1))
+                         : make_uint2(__funnelshift_l(v, u, k0), __funnelshift_l(u, v, k1));  // rho
+      const uint2 b0 = shfl(q, src0), b1 = shfl(q, src1), b2 = shfl(q, src2);  // pi, chi's row
+      a = kx2(kchi(b0, b1, b2), rc);                                           // chi, iota
     }
     return a;
   }
 };
 
-// keccak256(left || right) of node `s` by one warp: lanes 0..7 read the 64
-// message bytes, lanes 0..3 write the digest.
-__device__ __forceinline__ void warp_hash_node(const WarpKeccak& wk, const uint4* cur, size_t s, size_t h, uint4* nxt) {
-  const uint2* left = reinterpret_cast<const uint2*>(cur + 2 * s);
-  const uint2* right = reinterpret_cast<const uint2*>(cur + 2 * (s + h));
-  uint2 a = make_uint2(0, 0);
-  if (wk.lane < 4) a = left[wk.lane];
-  else if (wk.lane < 8) a = right[wk.lane - 4];
-  if (wk.lane == 8) a.x ^= 0x01u;         // pad10*1 after 64 bytes
-  if (wk.lane == 16) a.y ^= 0x80000000u;  // last byte of the 136-byte rate
-  a = wk.permute<true>(a);  // interleaved digests in, interleaved digest out
-  if (wk.lane < 4) reinterpret_cast<uint2*>(nxt + 2 * s)[wk.lane] = a;
+// Interleaved Keccak-f[1600] on a pair of lanes: the even lane holds the even
+// bits of all 25 words, the odd lane the odd bits (s[i], 32 bits).  Only theta's
+// rotation by one and the odd rotations of rho cross between them (18 shuffles
+// per round); the rest is half of a one-thread permutation's work per lane.
+// Measured on GB300: 5,330 cycles per permutation on one warp per scheduler
+// (16 states per warp) against 8,500 for one thread per state, 9,290 on two
+// warps per scheduler, so it serves levels of 9 to 64 nodes per block.
+struct PairKeccak {
+  bool odd;
+  __device__ __forceinline__ PairKeccak() { odd = (threadIdx.x & 1u) != 0; }
+
+  template <int R>
+  __device__ __forceinline__ uint32_t rot(uint32_t v) const {
+    if constexpr (R == 0) {
+      return v;
+    } else if constexpr ((R & 1) == 0) {
+      return rotl32(v, R / 2);
+    } else {  // even bits take rotl(odd bits, (R + 1) / 2), odd bits rotl(even bits, (R - 1) / 2)
+      const uint32_t o = __shfl_xor_sync(0xffffffffu, v, 1);
+      return __funnelshift_l(o, o, odd ? (R - 1) / 2 : (R + 1) / 2);
+    }
+  }
+
+  __device__ __forceinline__ void round(uint32_t s[25], int r) const {
+    const uint2 rc = c_keccak_rc_bi[r];
+    uint32_t C[5], D[5], b[25];
+#pragma unroll
+    for (int x = 0; x < 5; ++x) C[x] = s[x] ^ s[x + 5] ^ s[x + 10] ^ s[x + 15] ^ s[x + 20];
+#pragma unroll
+    for (int x = 0; x < 5; ++x) D[x] = rot<1>(C[(x + 1) % 5]);
+#pragma unroll
+    for (int i = 0; i < 25; ++i) s[i] ^= C[(i + 4) % 5] ^ D[i % 5];
+    b[0] = s[0];
+    b[10] = rot<1>(s[1]);
+    b[20] = rot<62>(s[2]);
+    b[5] = rot<28>(s[3]);
+    b[15] = rot<27>(s[4]);
+    b[16] = rot<36>(s[5]);
+    b[1] = rot<44>(s[6]);
+    b[11] = rot<6>(s[7]);
+    b[21] = rot<55>(s[8]);
+    b[6] = rot<20>(s[9]);
+    b[7] = rot<3>(s[10]);
+    b[17] = rot<10>(s[11]);
+    b[2] = rot<43>(s[12]);
+    b[12] = rot<25>(s[13]);
+    b[22] = rot<39>(s[14]);
+    b[23] = rot<41>(s[15]);
+    b[8] = rot<45>(s[16]);
+    b[18] = rot<15>(s[17]);
+    b[3] = rot<21>(s[18]);
+    b[13] = rot<8>(s[19]);
+    b[14] = rot<18>(s[20]);
+    b[24] = rot<2>(s[21]);
+    b[9] = rot<61>(s[22]);
+    b[19] = rot<56>(s[23]);
+    b[4] = rot<14>(s[24]);
+#pragma unroll
+    for (int y = 0; y < 25; y += 5) {
+#pragma unroll
+      for (int x = 0; x < 5; ++x) s[y + x] = b[y + x] ^ (~b[y + (x + 1) % 5] & b[y + (x + 2) % 5]);
+    }
+    s[0] ^= odd ? rc.y : rc.x;
+  }
+
+  // Pads the `nlanes` message lanes in s[0 .. nlanes) and permutes; the
+  // digest is s[0 .. 4).  All 32 lanes of the warp call this.
+  __device__ __forceinline__ void keccak256(uint32_t s[25], int nlanes) const {
+#pragma unroll
+    for (int i = 0; i < 25; ++i)
+      if (i >= nlanes) s[i] = 0;
+#pragma unroll
+    for (int i = 0; i < 17; ++i)
+      if (i == nlanes && !odd) s[i] ^= 0x01u;  // bit 0 of the lane after the message
+    if (odd) s[16] ^= 0x80000000u;             // bit 63 of lane 16
+    round(s, 0);
+#pragma unroll 2
+    for (int r = 1; r < 24; ++r) round(s, r);
+  }
+};
+
+// ---- a block's part of a Merkle tree ----------------------------------------
+// A digest in shared memory is eight words (uint2 per state lane: even bits,
+// odd bits); a block keeps the level it just made there, since reading it
+// back from global memory would add an L2 round trip to every level.
+constexpr int kTreeThreads = 256;  // threads of a block that runs tree levels
+constexpr int kTreeWarps = kTreeThreads / 32;
+constexpr int kTreeBlockLog = 9;   // at most 2^9 leaves per block
+struct TreeShared {
+  uint4 a[2 << (kTreeBlockLog - 1)];  // 2^8 digests
+  uint4 b[2 << (kTreeBlockLog - 2)];  // 2^7 digests
+};
+
+// One level: hash t < cnt (a power of two) goes to dst_s (shared, packed) and
+// dst_g (global, digest t at dst_g + 2 t gstride).  A node's message is the
+// digests t and t + cnt of `src` (digest t at src + 2 t stride); a LEAF's is
+// the 32 bytes at src + 2 t stride, interleaved lanes like a digest's.  All
+// threads of a block of kTreeThreads call this; the caller synchronizes around
+// it.  The form per count is the measured fastest (see WarpKeccak and
+// PairKeccak): one warp per hash up to 8, a pair of lanes up to 64, one thread
+// above.
+template <bool LEAF>
+__device__ __forceinline__ void hash_level_block(const WarpKeccak& wk, const uint4* src, size_t stride, uint32_t cnt,
+                                                 uint4* dst_s, uint4* dst_g, size_t gstride) {
+  constexpr int kLanes = LEAF ? 4 : 8;  // message lanes
+  if (cnt <= (uint32_t)kTreeWarps) {
+    const uint32_t t = threadIdx.x >> 5;
+    if (t >= cnt) return;
+    uint2 a = make_uint2(0, 0);
+    if (wk.lane < 4) a = reinterpret_cast<const uint2*>(src + 2 * stride * t)[wk.lane];
+    else if (wk.lane < kLanes) a = reinterpret_cast<const uint2*>(src + 2 * stride * (t + cnt))[wk.lane - 4];
+    if (wk.lane == kLanes) a.x ^= 0x01u;    // pad10*1 after the message
+    if (wk.lane == 16) a.y ^= 0x80000000u;  // last byte of the 136-byte rate
+    a = wk.permute<true>(a);
+    if (wk.lane < 4) {
+      reinterpret_cast<uint2*>(dst_s + 2 * t)[wk.lane] = a;
+      reinterpret_cast<uint2*>(dst_g + 2 * gstride * t)[wk.lane] = a;
+    }
+  } else if (cnt <= 64) {
+    if ((threadIdx.x & ~31u) >= 2 * cnt) return;  // whole warps: cnt is a multiple of 16
+    const PairKeccak pk;
+    const uint32_t t = threadIdx.x >> 1, h = threadIdx.x & 1u;
+    uint32_t s[25];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      s[i] = reinterpret_cast<const uint32_t*>(src + 2 * stride * t)[2 * i + h];
+      if (!LEAF) s[4 + i] = reinterpret_cast<const uint32_t*>(src + 2 * stride * (t + cnt))[2 * i + h];
+    }
+    pk.keccak256(s, kLanes);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      reinterpret_cast<uint32_t*>(dst_s + 2 * t)[2 * i + h] = s[i];
+      reinterpret_cast<uint32_t*>(dst_g + 2 * gstride * t)[2 * i + h] = s[i];
+    }
+  } else {
+    for (uint32_t t = threadIdx.x; t < cnt; t += kTreeThreads) {
+      uint2 s[25];
+      const uint4 l0 = src[2 * stride * t], l1 = src[2 * stride * t + 1];
+      s[0] = make_uint2(l0.x, l0.y);
+      s[1] = make_uint2(l0.z, l0.w);
+      s[2] = make_uint2(l1.x, l1.y);
+      s[3] = make_uint2(l1.z, l1.w);
+      if (!LEAF) {
+        const uint4 r0 = src[2 * stride * (t + cnt)], r1 = src[2 * stride * (t + cnt) + 1];
+        s[4] = make_uint2(r0.x, r0.y);
+        s[5] = make_uint2(r0.z, r0.w);
+        s[6] = make_uint2(r1.x, r1.y);
+        s[7] = make_uint2(r1.z, r1.w);
+      }
+      keccak256_lanes<true>(s, kLanes);
+      const Digest d = digest_from_state(s);
+      dst_s[2 * t] = d.lo;
+      dst_s[2 * t + 1] = d.hi;
+      dst_g[2 * gstride * t] = d.lo;
+      dst_g[2 * gstride * t + 1] = d.hi;
+    }
+  }
+}
+
+// Levels 1 .. k (k <= kTreeBlockLog) above 2^k digests at `src` (digest t at
+// src + 2 t stride), the block's share b of a tree level of n nodes: node t of
+// level j is node b + t (n >> k) of that level, and the levels lie one after
+// another from `out`.  Odd levels pass through o0, even ones through o1
+// (shared; 2^(k-1) and 2^(k-2) digests).  Returns where the level-k digest is
+// (src when k = 0).  All threads of a block of kTreeThreads call this; it ends
+// synchronized.
+__device__ __forceinline__ const uint4* tree_block(const WarpKeccak& wk, uint4* o0, uint4* o1, const uint4* src,
+                                                   size_t stride, uint4* out, size_t n, size_t b, int k) {
+  const size_t nk = n >> k;
+  for (int j = 1; j <= k; ++j) {
+    uint4* o = (j & 1) ? o0 : o1;
+    hash_level_block<false>(wk, src, stride, 1u << (k - j), o, out + 2 * b, nk);
+    __syncthreads();
+    src = o;
+    stride = 1;
+    n >>= 1;
+    out += 2 * n;
+  }
+  return src;
 }
 
 // keccak256 of matrix rows of `words` 32-bit words, one lane per row, the

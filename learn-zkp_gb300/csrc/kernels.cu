@@ -16,6 +16,7 @@
 //    nodes sits at bitrev_h(m).  Then node s of the next level is
 //    H(prev[s] || prev[s + half]) — both children in the two contiguous
 //    halves of the level below — so every level is one coalesced pass.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <atomic>
 #include <algorithm>
@@ -647,26 +648,42 @@ __global__ void __launch_bounds__(128) level_kernel(const uint4* __restrict__ pr
     store_digest(next, s, hash_node(load_digest(prev, s), load_digest(prev, s + n_next)));
 }
 
-// The remaining levels of a small tree, in one block; the root is also
+// The remaining 2^k nodes of a small tree, in one block; the root is also
 // copied to `root_out` when given.
-__global__ void __launch_bounds__(256) tree_top_kernel(uint4* level, size_t n, uint4* root_out) {
+__global__ void __launch_bounds__(kTreeThreads) tree_top_kernel(uint4* level, int k, uint4* root_out) {
+  __shared__ TreeShared sh;
   const WarpKeccak wk;
-  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  uint4* cur = level;
-  while (n > 1) {
-    const size_t h = n >> 1;
-    uint4* nxt = cur + 2 * n;
-    if (h <= (size_t)nwarps) {  // latency-bound: one warp per node
-      for (size_t s = warp; s < h; s += nwarps) warp_hash_node(wk, cur, s, h, nxt);
-    } else {
-      for (size_t s = threadIdx.x; s < h; s += blockDim.x)
-        store_digest(nxt, s, hash_node(load_digest(cur, s), load_digest(cur, s + h)));
-    }
-    __syncthreads();
-    cur = nxt;
-    n = h;
+  const size_t n = (size_t)1 << k;
+  const uint4* root = tree_block(wk, sh.a, sh.b, level, 1, level + 2 * n, n, 0, k);
+  if (root_out && threadIdx.x < 2) root_out[threadIdx.x] = root[threadIdx.x];
+}
+
+// The same for 2^8 .. 2^12 nodes on a cluster of eight blocks: block r takes the
+// subtree under node r of the level of eight nodes, block 0 the three levels
+// above from the eight digests the blocks hand it through distributed shared
+// memory.  Eight SMs run a 512-node top's first levels on pairs of lanes and
+// warps instead of one SM on threads.
+constexpr int kTopCluster = 8, kTopClusterLog = 3;
+__global__ void __cluster_dims__(kTopCluster, 1, 1) __launch_bounds__(kTreeThreads)
+    tree_top_cluster_kernel(uint4* level, int k, uint4* root_out) {
+  namespace cg = cooperative_groups;
+  __shared__ TreeShared sh;
+  __shared__ uint4 roots[2 * kTopCluster];
+  cg::cluster_group cl = cg::this_cluster();
+  const unsigned r = cl.block_rank();
+  const WarpKeccak wk;
+  const size_t n = (size_t)1 << k;
+  cl.sync();  // block 0 is running: its shared memory may be written
+  const uint4* sub =
+      tree_block(wk, sh.a, sh.b, level + 2 * r, kTopCluster, level + 2 * n, n, r, k - kTopClusterLog);
+  uint4* dst = cl.map_shared_rank(roots, 0);
+  if (threadIdx.x < 2) dst[2 * r + threadIdx.x] = sub[threadIdx.x];
+  cl.sync();
+  if (r == 0) {
+    const uint4* root =
+        tree_block(wk, sh.a, sh.b, roots, 1, level + 2 * (2 * n - kTopCluster), kTopCluster, 0, kTopClusterLog);
+    if (root_out && threadIdx.x < 2) root_out[threadIdx.x] = root[threadIdx.x];
   }
-  if (root_out && threadIdx.x == 0) store_digest(root_out, 0, load_digest(cur, 0));
 }
 
 // Leaf of a row of `width` elements: keccak256 of its 16*width bytes
@@ -702,45 +719,42 @@ cudaError_t launch_leaves_pair(const uint4* pi, uint4* leaves, size_t n, cudaStr
 }
 
 // Levels 1..k above `level` (n nodes), stored one after another after it, in
-// one launch.  Block b owns the top nodes [b M, (b+1) M) of level k
-// (n >> k nodes), M = 2^(9-k), and at level k - j the runs s + m (n >> k),
-// m < 2^j, of their subtrees: node i of a level has children i and
-// i + (its level's size) below, so a block only reads what it wrote and
-// __syncthreads separates the levels.  Level 1 has one node per thread.
-constexpr int kSubtreeThreads = 256;
-__global__ void __launch_bounds__(kSubtreeThreads) subtree_kernel(uint4* level, size_t n, int k) {
-  const size_t nk = n >> k;
-  const int log_m = 9 - k;  // M = 2^log_m top nodes per block
-  const size_t a = (size_t)blockIdx.x << log_m;
-  uint4* cur = level;
-  size_t ncur = n;
-  for (int j = 1; j <= k; ++j) {
-    const size_t h = ncur >> 1;
-    uint4* nxt = cur + 2 * ncur;
-    const int per = 1 << (log_m + k - j);  // this block's nodes at level j
-    for (int t = threadIdx.x; t < per; t += blockDim.x) {
-      const size_t s = a + (size_t)(t & ((1 << log_m) - 1)) + (size_t)(t >> log_m) * nk;
-      store_digest(nxt, s, hash_node(load_digest(cur, s), load_digest(cur, s + h)));
-    }
-    __syncthreads();
-    cur = nxt;
-    ncur = h;
-  }
+// one launch.  Block b owns node b of level k (n >> k nodes, one block each)
+// and its subtree: node i of a level has children i and i + (its level's size)
+// below, so its nodes at level j are b + t (n >> k), t < 2^(k-j), a block only
+// reads what it wrote, and __syncthreads separates the levels.  Bound by the
+// chain of permutations.  A whole tree of 2^12 leaves takes 36.9 us on GB300
+// (59.4 with 2^9-leaf blocks, one thread per node and levels in global
+// memory), of 2^16 leaves 57.4 (75.8).
+__global__ void __launch_bounds__(kTreeThreads) subtree_kernel(uint4* level, size_t n, int k) {
+  __shared__ TreeShared sh;
+  const WarpKeccak wk;
+  const size_t b = blockIdx.x;
+  tree_block(wk, sh.a, sh.b, level + 2 * b, n >> k, level + 2 * n, n, b, k);
 }
+
+static int floor_log2(size_t n) {
+  int l = 0;
+  while (n >>= 1) ++l;
+  return l;
+}
+
+// Where the single-block top ends.  Measured on GB300, one tree of n leaves with
+// its launches: 2^8 nodes 22.6 us on the cluster, 26.7 as a subtree launch and
+// a single-block top; 2^9 nodes 26.6 and 28.7 (39.0 on one block of threads);
+// 2^7 nodes 22.1 in one block, 24.6 in two launches.
+constexpr size_t kTopSingle = 128;
 
 cudaError_t launch_tree(uint4* leaves, size_t n, cudaStream_t st, uint4* root_out, const Tune& tune) {
   uint4* cur = leaves;
   const size_t top_nodes = (size_t)tune.top_nodes;
   const size_t subtree_max = (size_t)1 << tune.subtree_log;  // larger levels: one launch each
   while (n > top_nodes) {
-    if (n <= subtree_max && n >= 1024) {  // the latency-bound middle levels in one launch
-      int k = 0;
-      size_t m = n;
-      while (m > top_nodes && k < 9) {
-        m >>= 1;
-        ++k;
-      }
-      subtree_kernel<<<(unsigned)(n >> 9), kSubtreeThreads, 0, st>>>(cur, n, k);
+    if (n <= subtree_max) {
+      // the latency-bound middle levels in one launch: about one block per SM,
+      // of 2^6 leaves (whose levels run on pairs of lanes and warps) to 2^9
+      const int k = std::max(6, std::min(kTreeBlockLog, floor_log2(n) - 7));
+      subtree_kernel<<<(unsigned)(n >> k), kTreeThreads, 0, st>>>(cur, n, k);
       COUNT_LAUNCH();
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
@@ -759,8 +773,11 @@ cudaError_t launch_tree(uint4* leaves, size_t n, cudaStream_t st, uint4* root_ou
     cur = nxt;
     n = h;
   }
-  if (n > 1 || root_out) {
-    tree_top_kernel<<<1, 256, 0, st>>>(cur, n, root_out);
+  if (n > kTopSingle) {
+    tree_top_cluster_kernel<<<kTopCluster, kTreeThreads, 0, st>>>(cur, floor_log2(n), root_out);
+    COUNT_LAUNCH();
+  } else if (n > 1 || root_out) {
+    tree_top_kernel<<<1, kTreeThreads, 0, st>>>(cur, floor_log2(n), root_out);
     COUNT_LAUNCH();
   }
   return cudaGetLastError();

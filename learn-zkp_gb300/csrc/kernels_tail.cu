@@ -228,52 +228,77 @@ __global__ void __launch_bounds__(32) open_round_kernel(OpenState* S, int i, int
   state_store(S, sh);
 }
 
+// The last rounds in one block of eight warps.  Rounds whose fold has at most
+// kTailShared outputs keep the folded codeword, the leaf messages and the tree
+// levels in shared memory (a level read back from global memory costs an L2
+// round trip), hash each level in the form that is fastest for its count
+// (hash_level_block), and multiply by the twiddles, which need no challenge,
+// on warps 1..7 while warp 0 runs the transcript step: after the challenge a
+// fold output is one product.  Bound by the chain of dependent permutations
+// (one per level, leaf and transcript step).  Measured at 2^8 leaves and below,
+// GB300: 195 us for the last eight rounds, 262 us with one thread per
+// leaf, the codeword and the levels in global memory and both products after
+// the challenge.
+constexpr int kTailShared = 512;
+
 __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P) {
+  static_assert(kTailThreads == kTreeThreads, "the tail hashes levels with hash_level_block");
   __shared__ OpenState sh;
-  __shared__ uint4 sh_S, sh_root_lo, sh_root_hi;
-  __shared__ uint4 scratch[32];
+  __shared__ uint4 pi_a[2 * kTailShared], pi_b[kTailShared];  // (lo', hi' - lo') pairs of a fold's input
+  __shared__ uint4 msg[kTailShared];                          // a fold's outputs as interleaved lanes
+  __shared__ TreeShared ts;
+  __shared__ __align__(16) uint32_t sums[2][4];  // the round's reduction and the next one's
   const int d = P.d;
   const size_t c = (size_t)1 << P.log2_c;
   const WarpKeccak wk;
-  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5;
   state_load(sh, P.state);
-  if (threadIdx.x == 0 && P.i0 >= 0) {
-    sh_root_lo = P.root_i0[0];
-    sh_root_hi = P.root_i0[1];
-    sh_S = P.S_i0[0];
-  }
+  if (threadIdx.x == 0 && P.i0 >= 0) *reinterpret_cast<uint4*>(sums[0]) = P.S_i0[0];
+  const uint4* root = P.root_i0;  // the round's tree root
+  const uint4* pi_s = nullptr;    // the round's folded codeword in shared memory, if it is there
   __syncthreads();
   int k = 0;
   for (int i = P.i0; i >= 0; --i, ++k) {
-    // ---- transcript step (warp 0) ----
-    if (warp == 0)
-      round_step(wk, sh, i, d, P.scal, sh_root_lo, sh_root_hi, sh_S, reinterpret_cast<uint4*>(P.result + 64 * (size_t)k));
-    __syncthreads();
-    const uint4 x = sh.x;
-    // ---- fold (+ next leaves) and fix (+ next reduction), whole block ----
     const size_t ni = c << i;
+    const bool small = ni <= (size_t)kTailShared;
     const uint4* pi_in = (i == d - 1) ? P.pi_first : P.pi_fold + c * (((size_t)1 << d) - ((size_t)1 << (i + 2)));
     uint4* pi_out = P.pi_fold + c * (((size_t)1 << d) - ((size_t)1 << (i + 1)));
     const uint4* tlo = P.tw->lo[d - 1 - i];
     const uint4* thi = P.tw->hi[d - 1 - i];
+    uint4* pairs = pi_s == pi_b ? pi_b : pi_a;
+    uint4* next = pairs == pi_a ? pi_b : pi_a;
+    // ---- transcript step (warp 0); meanwhile the other warps interpolate ----
+    if (warp == 0) {
+      round_step(wk, sh, i, d, P.scal, root[0], root[1], *reinterpret_cast<const uint4*>(sums[k & 1]),
+                 reinterpret_cast<uint4*>(P.result + 64 * (size_t)k));
+    } else {
+      if (threadIdx.x == 32) *reinterpret_cast<uint4*>(sums[(k + 1) & 1]) = make_uint4(0, 0, 0, 0);
+      if (small) {
+        const uint4* src = pi_s ? pi_s : pi_in;
+        for (uint32_t t = threadIdx.x - 32; t < ni; t += blockDim.x - 32) {
+          const uint4 tw = gf_add(tlo[t & 4095], thi[t >> 12]);
+          const uint4 lo = src[2 * t], hi = gf_add(src[2 * t + 1], lo);
+          const uint4 l = gf_add(lo, gf_mul(hi, tw));
+          pairs[2 * t] = l;
+          pairs[2 * t + 1] = gf_add(hi, l);
+        }
+      }
+    }
+    __syncthreads();
+    const uint4 x = sh.x;
     uint4* leaves = nullptr;
     if (i > 0)
       leaves = P.pi_trees + 2 * ((c << 1) * (((size_t)1 << (d - 1)) - ((size_t)1 << i)) - (size_t)(d - 1 - i));
-    if (i > 0) {
-      for (size_t s = threadIdx.x; s < ni / 2; s += blockDim.x) {
-        uint4 f[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const size_t t = 2 * s + q;
-          const uint4 tw = gf_add(tlo[t & 4095], thi[t >> 12]);
-          uint4 lo = pi_in[2 * t], hi = pi_in[2 * t + 1];
-          hi = gf_add(hi, lo);
-          lo = gf_add(lo, gf_mul(hi, tw));
-          f[q] = gf_add(lo, gf_mul(gf_add(hi, lo), x));
-          pi_out[t] = f[q];
-        }
-        store_digest(leaves, s, hash_pair(f[0], f[1]));
+    // ---- fold from the first thread up, fix (+ next reduction) from the last down ----
+    if (small) {
+      for (uint32_t t = threadIdx.x; t < ni; t += blockDim.x) {
+        const uint4 f = gf_add(pairs[2 * t], gf_mul(pairs[2 * t + 1], x));
+        pi_out[t] = f;
+        next[t] = f;
+        const uint2 m0 = bi_from_lane(make_uint2(f.x, f.y)), m1 = bi_from_lane(make_uint2(f.z, f.w));
+        msg[t] = make_uint4(m0.x, m0.y, m1.x, m1.y);
       }
+      pi_s = next;
     } else {
       for (size_t t = threadIdx.x; t < ni; t += blockDim.x) {
         const uint4 tw = gf_add(tlo[t & 4095], thi[t >> 12]);
@@ -286,37 +311,38 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
     const uint4* poly_in = (i == d - 1) ? P.poly_first : P.poly;
     const size_t half = (size_t)1 << i, next_half = i > 0 ? half / 2 : 0;
     uint4 part = make_uint4(0, 0, 0, 0);
-    for (size_t b = threadIdx.x; b < half; b += blockDim.x) {
+    for (size_t b = blockDim.x - 1 - threadIdx.x; b < half; b += blockDim.x) {
       const uint4 lo = poly_in[b], hi = poly_in[b + half];
       const uint4 v = gf_add(lo, gf_mul(x, gf_add(hi, lo)));
       P.poly[b] = v;
       if (b < next_half) part = gf_add(part, gf_mul(P.heq[b], v));
     }
-    part = block_xor(part, scratch);
-    if (threadIdx.x == 0) sh_S = part;
+    part = warp_xor(part);
+    if (wk.lane == 0) atomic_xor4(sums[(k + 1) & 1], part);
     __syncthreads();
-    // ---- the next round's Merkle tree, level by level ----
+    // ---- the next round's leaves and Merkle tree ----
     if (i > 0) {
-      uint4* cur = leaves;
       size_t n = ni / 2;
-      while (n > 1) {
-        const size_t h = n >> 1;
-        uint4* nxt = cur + 2 * n;
-        if (h <= (size_t)nwarps) {  // latency-bound: one warp per node
-          for (size_t s = warp; s < h; s += nwarps) warp_hash_node(wk, cur, s, h, nxt);
-        } else {
+      if (small) {
+        hash_level_block<true>(wk, msg, 1, (uint32_t)n, ts.a, leaves, 1);
+        __syncthreads();
+        root = tree_block(wk, ts.b, ts.a, ts.a, 1, leaves + 2 * n, n, 0, P.log2_c + i - 1);
+      } else {
+        for (size_t s = threadIdx.x; s < n; s += blockDim.x)
+          store_digest(leaves, s, hash_pair(pi_out[2 * s], pi_out[2 * s + 1]));
+        __syncthreads();
+        uint4* cur = leaves;
+        int kn = P.log2_c + i - 1;
+        for (; kn > kTreeBlockLog; --kn, n >>= 1) {
+          const size_t h = n >> 1;
+          uint4* nxt = cur + 2 * n;
           for (size_t s = threadIdx.x; s < h; s += blockDim.x)
             store_digest(nxt, s, hash_node(load_digest(cur, s), load_digest(cur, s + h)));
+          __syncthreads();
+          cur = nxt;
         }
-        __syncthreads();
-        cur = nxt;
-        n = h;
+        root = tree_block(wk, ts.a, ts.b, cur, 1, cur + 2 * n, n, 0, kn);
       }
-      if (threadIdx.x == 0) {
-        sh_root_lo = cur[0];
-        sh_root_hi = cur[1];
-      }
-      __syncthreads();
     }
   }
   // ---- final polynomial (basefold.rs:196) ----

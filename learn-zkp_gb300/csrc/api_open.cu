@@ -229,9 +229,10 @@ int ensure_message(bf_open_session* s) {
 namespace bfapi {
 
 // First round run by the single-block kernel: the largest i <= d-1 whose
-// folded codeword has at most 2^(tail_log+1) entries.
+// folded codeword has at most 2^(tail_log+1) entries, and at least round 0,
+// which has no next tree for the per-round kernels to build.
 int tail_first_round(const bf_pcs* p, int d) {
-  const int lim = p->tune.tail_log + 1 - p->log2_c;
+  const int lim = std::max(0, p->tune.tail_log + 1 - p->log2_c);
   return std::min(d - 1, lim);
 }
 

@@ -556,7 +556,8 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
     std::memcpy(t.pend, tr.in.data() + pos, t.pend_len);
     t.out_len = (uint32_t)tr.out.size();
     std::memcpy(t.out, tr.out.data(), t.out_len);
-    t.outer = bbh::to_dev(claim);
+    t.claim = bbh::to_dev(claim);
+    t.delta = bbh::to_dev(E::one());
     bf::BbRoundConsts c{};
     const std::vector<E> cf = es.correcting_factors();
     for (int k = 0; k < nv; ++k) {
@@ -594,13 +595,44 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
     const int base_k = k == 0 && base_round;
     if (k == 0) CU(bf::bb_launch_leaves_pairs(pi, base_k, tree, ni, li, st));  // later rounds: made by the fold
     CU(bf::launch_tree(tree, ni, st, root_dev, bf::Tune()));
+    if (ni <= (size_t)bf::kBbTailMax) {  // this round and the rest in one block
+      CU(cudaEventRecord(p->ev_dot, sa));  // the last fix
+      CU(cudaStreamWaitEvent(st, p->ev_dot, 0));
+      bf::BbTail tp{};
+      tp.i0 = i;
+      tp.lk = lk;
+      tp.log2_n0 = p->log2_n0();
+      tp.pi = pi;
+      tp.pi_base = base_k;
+      tp.poly = poly;
+      tp.poly_base = base_k;
+      tp.heq = heq;
+      tp.tinv = p->tinv.as<uint32_t>();
+      tp.fold_out = folds + 5 * fold_off;
+      tp.poly_out = fixbuf[k & 1];
+      tp.next_tree = tree + 2 * (2 * ni);
+      tp.root = root_dev;
+      tp.t = tdev;
+      tp.c = cdev;
+      tp.rec = rec_dev + 72 * (size_t)k;
+      CU(bf::bb_launch_tail(tp, st));
+      for (int q = k + 1; q < d; ++q) {  // the codewords and trees it makes
+        const size_t nq = p->n_i(d - q);  // round q - 1's fold outputs
+        gp.pi[q] = folds + 5 * fold_off;
+        fold_off += nq;
+        tree_off += 2 * nq;
+        gp.trees[q] = trees + 2 * tree_off;
+      }
+      pi = folds + 5 * fold_off;  // round d - 1's outputs
+      poly = fixbuf[k & 1];
+      break;
+    }
     CU(cudaMemsetAsync(acc, 0, 40, sa));
     CU(bf::bb_launch_dot(heq, poly, base_k, (size_t)1 << ri, acc, sa));
     CU(cudaEventRecord(p->ev_dot, sa));
     CU(cudaStreamWaitEvent(st, p->ev_dot, 0));
     uint32_t* x_k = xs_dev + 5 * (size_t)k;
-    CU(bf::bb_launch_transcript_round(tdev, cdev, k, ri, nv, root_dev, acc, base_k, x_k, rec_dev + 72 * (size_t)k,
-                                      st));
+    CU(bf::bb_launch_transcript_round(tdev, cdev, ri, root_dev, acc, base_k, x_k, rec_dev + 72 * (size_t)k, st));
     CU(cudaEventRecord(p->ev_x, st));
     CU(cudaStreamWaitEvent(sa, p->ev_x, 0));
     const bb::E5 unused{};

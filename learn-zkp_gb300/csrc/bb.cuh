@@ -81,20 +81,36 @@ __host__ __device__ __forceinline__ E5 e_scale(const E5& a, uint32_t f) {
   for (int i = 0; i < 5; ++i) r.c[i] = mul(a.c[i], f);
   return r;
 }
-// (sum_i a_i X^i)(sum_j b_j X^j) with X^5 = 2: coefficient k takes the
-// products with i + j = k and twice those with i + j = k + 5.
+// t R^-1 mod p for t < p 2^32 (the Montgomery reduction of a sum of products).
+__host__ __device__ __forceinline__ uint32_t reduce(uint64_t t) {
+  const uint32_t m = (uint32_t)t * P_INV;
+  const uint32_t d = (uint32_t)(t >> 32) - (uint32_t)(((uint64_t)m * P) >> 32);
+  return umin(d, d + P);
+}
+// (sum_i a_i X^i)(sum_j b_j X^j) with X^5 = 2: coefficient k is the sum of the
+// five products a_j b_(k-j), those that wrap past X^5 with b doubled.  Four
+// products of words below p sum below 2^63.9; the sum is folded to
+// hi (2^32 mod p) + lo (below 2^60) before the fifth, so one reduction of less
+// than p 2^32 per coefficient replaces one per product.
 __host__ __device__ __forceinline__ E5 e_mul(const E5& a, const E5& b) {
-  uint32_t lo[5] = {0, 0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-  for (int i = 0; i < 5; ++i)
-    for (int j = 0; j < 5; ++j) {
-      const uint32_t t = mul(a.c[i], b.c[j]);
-      if (i + j < 5)
-        lo[i + j] = add(lo[i + j], t);
-      else
-        hi[i + j - 5] = add(hi[i + j - 5], t);
-    }
+  uint32_t bd[5];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int j = 1; j < 5; ++j) bd[j] = add(b.c[j], b.c[j]);
   E5 r;
-  for (int k = 0; k < 5; ++k) r.c[k] = k < 4 ? add(lo[k], add(hi[k], hi[k])) : lo[k];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int k = 0; k < 5; ++k) {
+    uint64_t s = 0;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int j = 0; j < 4; ++j) s += (uint64_t)a.c[j] * (j <= k ? b.c[k - j] : bd[k - j + 5]);
+    s = (s >> 32) * MONT_ONE + (uint32_t)s;
+    r.c[k] = reduce(s + (uint64_t)a.c[4] * (k == 4 ? b.c[0] : bd[k + 1]));
+  }
   return r;
 }
 

@@ -88,31 +88,51 @@ cudaError_t bb_launch_fold(const BbFold& p, const bb::E5& x, cudaStream_t st);
 // input blocks absorbed so far plus the pending input bytes — and its output
 // buffer, with the EvalProver subclaims of the folding sumcheck.  Field
 // elements are Montgomery form.
-struct BbTranscript {
+struct alignas(8) BbTranscript {
   uint2 A[25];          // lanes (low word, high word) of the absorbed input blocks
   uint8_t pend[256];    // input bytes not yet absorbed (fewer than 136 between rounds)
-  uint32_t pend_len;
   uint8_t out[32];      // output buffer: bytes out[0 .. out_len), popped from the end
-  uint32_t out_len;
-  bb::E5 outer;         // the open's subclaim (sumcheck/src/lib.rs:18-48)
-  bb::E5 inner;         // EvalImprProver's inner subclaim value
-  bb::E5 xs[kBbMaxRounds];  // challenges in sampling order
-  uint32_t rounds;
+  uint32_t pend_len, out_len;
+  bb::E5 claim;         // the open's claim in the first round, then EvalImprProver's inner subclaim value
+  bb::E5 delta;         // the delta factor eq_eval(r[ri+1 ..], challenges so far) (eval_impr.rs:45-51); 1 at the start
 };
 // Per sumcheck round ri (< num_vars): the point coordinate, its inverse and
 // the correcting factor prod_{k >= ri} (1 - r_k)^-1 (eval_impr.rs:83-90).
 struct BbRoundConsts {
   bb::E5 r[kBbMaxRounds], r_inv[kBbMaxRounds], cf[kBbMaxRounds];
 };
-// One folding-sumcheck round's transcript (k rounds done before it): observe
-// the round's folded-codeword root (interleaved digest at root_dev), compute
-// the round polynomial from the GPU sum (Montgomery sums, or canonical ones
-// when `canonical`), observe its compressed form, sample the challenge into
-// x_out (Montgomery) and record the root and the compressed polynomial (72
-// canonical bytes) at rec.
-cudaError_t bb_launch_transcript_round(BbTranscript* t, const BbRoundConsts* c, int k, int ri, int num_vars,
-                                       const uint4* root_dev, const unsigned long long* sums, int canonical,
-                                       uint32_t* x_out, uint8_t* rec, cudaStream_t st);
+// One folding-sumcheck round's transcript (sumcheck round ri): observe the
+// round's folded-codeword root (interleaved digest at root_dev), compute the
+// round polynomial from the GPU sum (Montgomery sums, or canonical ones when
+// `canonical`), observe its compressed form, sample the challenge into x_out
+// (Montgomery) and record the root and the compressed polynomial (72 canonical
+// bytes) at rec.
+cudaError_t bb_launch_transcript_round(BbTranscript* t, const BbRoundConsts* c, int ri, const uint4* root_dev,
+                                       const unsigned long long* sums, int canonical, uint32_t* x_out, uint8_t* rec,
+                                       cudaStream_t st);
+
+// The last rounds i0 .. 0 of an open in one block: the rounds whose fold has
+// n_i <= kBbTailMax outputs.  The tree of round i0 is built before (its root
+// at `root`); the trees of the later rounds follow it, as the fold outputs do
+// `fold_out`, one after another.
+constexpr int kBbTailMax = 256;
+struct BbTail {
+  int i0, lk, log2_n0;     // n_i = 2^(log2_n0 + i); the sumcheck round of round i is i + lk
+  const uint32_t* pi;      // 2 n_i0 entries: extension, or base-field Montgomery when pi_base
+  int pi_base;
+  const uint32_t* poly;    // 2^(i0 + lk + 1) entries: extension, or canonical base-field data when poly_base
+  int poly_base;
+  const uint32_t* heq;     // half eq table (Montgomery extension)
+  const uint32_t* tinv;    // fold constants, round i at n_0 (2^i - 1)
+  uint32_t* fold_out;      // round i0's n_i0 outputs, then the later rounds'
+  uint32_t* poly_out;      // the 2^lk entries left at the end
+  uint4* next_tree;        // the tree of round i0 - 1
+  const uint4* root;
+  BbTranscript* t;
+  const BbRoundConsts* c;
+  uint8_t* rec;            // round i0's record (72 bytes), then the later rounds'
+};
+cudaError_t bb_launch_tail(const BbTail& p, cudaStream_t st);
 
 // Query openings in the proof's bincode layout, one record per query:
 // u64 w, w canonical words, u64 L, L digests, u64 d, then per round k:

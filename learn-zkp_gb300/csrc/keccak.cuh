@@ -478,24 +478,29 @@ struct TreeShared {
 };
 
 // One level: hash t < cnt (a power of two) goes to dst_s (shared, packed) and
-// dst_g (global, digest t at dst_g + 2 t gstride).  A node's message is the
-// digests t and t + cnt of `src` (digest t at src + 2 t stride); a LEAF's is
-// the 32 bytes at src + 2 t stride, interleaved lanes like a digest's.  All
-// threads of a block of kTreeThreads call this; the caller synchronizes around
-// it.  The form per count is the measured fastest (see WarpKeccak and
-// PairKeccak): one warp per hash up to 8, a pair of lanes up to 64, one thread
-// above.
-template <bool LEAF>
+// dst_g (global, digest t at dst_g + 2 t gstride).  A node's message (LANES 8)
+// is the digests t and t + cnt of `src` (digest t at src + 2 t stride); a
+// leaf's (LANES < 8) is the LANES interleaved lanes at (const uint2*)src +
+// LANES t.  All threads of a block of kTreeThreads call this; the caller
+// synchronizes around it.  The form per count is the measured fastest (see
+// WarpKeccak and PairKeccak): one warp per hash up to 8, a pair of lanes up to
+// 64, one thread above.
+template <int LANES>
 __device__ __forceinline__ void hash_level_block(const WarpKeccak& wk, const uint4* src, size_t stride, uint32_t cnt,
                                                  uint4* dst_s, uint4* dst_g, size_t gstride) {
-  constexpr int kLanes = LEAF ? 4 : 8;  // message lanes
+  constexpr bool NODE = LANES == 8;
+  auto first = [&](uint32_t t) {  // the lanes of the message, or of a node's left child
+    return NODE ? reinterpret_cast<const uint2*>(src + 2 * stride * t)
+                : reinterpret_cast<const uint2*>(src) + LANES * (size_t)t;
+  };
+  auto second = [&](uint32_t t) { return reinterpret_cast<const uint2*>(src + 2 * stride * (t + cnt)); };
   if (cnt <= (uint32_t)kTreeWarps) {
     const uint32_t t = threadIdx.x >> 5;
     if (t >= cnt) return;
     uint2 a = make_uint2(0, 0);
-    if (wk.lane < 4) a = reinterpret_cast<const uint2*>(src + 2 * stride * t)[wk.lane];
-    else if (wk.lane < kLanes) a = reinterpret_cast<const uint2*>(src + 2 * stride * (t + cnt))[wk.lane - 4];
-    if (wk.lane == kLanes) a.x ^= 0x01u;    // pad10*1 after the message
+    if (wk.lane < (NODE ? 4 : LANES)) a = first(t)[wk.lane];
+    else if (NODE && wk.lane < 8) a = second(t)[wk.lane - 4];
+    if (wk.lane == LANES) a.x ^= 0x01u;     // pad10*1 after the message
     if (wk.lane == 16) a.y ^= 0x80000000u;  // last byte of the 136-byte rate
     a = wk.permute<true>(a);
     if (wk.lane < 4) {
@@ -506,13 +511,16 @@ __device__ __forceinline__ void hash_level_block(const WarpKeccak& wk, const uin
     if ((threadIdx.x & ~31u) >= 2 * cnt) return;  // whole warps: cnt is a multiple of 16
     const PairKeccak pk;
     const uint32_t t = threadIdx.x >> 1, h = threadIdx.x & 1u;
+    const uint32_t* l = reinterpret_cast<const uint32_t*>(first(t)) + h;
     uint32_t s[25];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      s[i] = reinterpret_cast<const uint32_t*>(src + 2 * stride * t)[2 * i + h];
-      if (!LEAF) s[4 + i] = reinterpret_cast<const uint32_t*>(src + 2 * stride * (t + cnt))[2 * i + h];
+    for (int i = 0; i < (NODE ? 4 : LANES); ++i) s[i] = l[2 * i];
+    if (NODE) {
+      const uint32_t* r = reinterpret_cast<const uint32_t*>(second(t)) + h;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[4 + i] = r[2 * i];
     }
-    pk.keccak256(s, kLanes);
+    pk.keccak256(s, LANES);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       reinterpret_cast<uint32_t*>(dst_s + 2 * t)[2 * i + h] = s[i];
@@ -521,19 +529,15 @@ __device__ __forceinline__ void hash_level_block(const WarpKeccak& wk, const uin
   } else {
     for (uint32_t t = threadIdx.x; t < cnt; t += kTreeThreads) {
       uint2 s[25];
-      const uint4 l0 = src[2 * stride * t], l1 = src[2 * stride * t + 1];
-      s[0] = make_uint2(l0.x, l0.y);
-      s[1] = make_uint2(l0.z, l0.w);
-      s[2] = make_uint2(l1.x, l1.y);
-      s[3] = make_uint2(l1.z, l1.w);
-      if (!LEAF) {
-        const uint4 r0 = src[2 * stride * (t + cnt)], r1 = src[2 * stride * (t + cnt) + 1];
-        s[4] = make_uint2(r0.x, r0.y);
-        s[5] = make_uint2(r0.z, r0.w);
-        s[6] = make_uint2(r1.x, r1.y);
-        s[7] = make_uint2(r1.z, r1.w);
+      const uint2* l = first(t);
+#pragma unroll
+      for (int i = 0; i < (NODE ? 4 : LANES); ++i) s[i] = l[i];
+      if (NODE) {
+        const uint2* r = second(t);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[4 + i] = r[i];
       }
-      keccak256_lanes<true>(s, kLanes);
+      keccak256_lanes<true>(s, LANES);
       const Digest d = digest_from_state(s);
       dst_s[2 * t] = d.lo;
       dst_s[2 * t + 1] = d.hi;
@@ -555,7 +559,7 @@ __device__ __forceinline__ const uint4* tree_block(const WarpKeccak& wk, uint4* 
   const size_t nk = n >> k;
   for (int j = 1; j <= k; ++j) {
     uint4* o = (j & 1) ? o0 : o1;
-    hash_level_block<false>(wk, src, stride, 1u << (k - j), o, out + 2 * b, nk);
+    hash_level_block<8>(wk, src, stride, 1u << (k - j), o, out + 2 * b, nk);
     __syncthreads();
     src = o;
     stride = 1;

@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
     if (i > 0) {
       size_t n = ni / 2;
       if (small) {
-        hash_level_block<true>(wk, msg, 1, (uint32_t)n, ts.a, leaves, 1);
+        hash_level_block<4>(wk, msg, 1, (uint32_t)n, ts.a, leaves, 1);
         __syncthreads();
         root = tree_block(wk, ts.b, ts.a, ts.a, 1, leaves + 2 * n, n, 0, P.log2_c + i - 1);
       } else {

@@ -64,7 +64,6 @@ int sumcheck_run(cudaStream_t st, DevBuf& scratch, PinnedBuf& pinned, int k, int
     for (int round = n - 1; round >= 0; --round, ++ri) {
       CU(bf::launch_sumcheck_round(S, k, acc, rec + rec_sz * (size_t)ri, st));
       const size_t half = (size_t)1 << round;
-      if (round > 0) CU(cudaMemsetAsync(acc, 0, 48, st));
       const uint4* const* src = (round == n - 1) ? in : const_cast<const uint4* const*>(work);
       CU(bf::launch_prod_fix(work, src, k, half, uint4{}, half / 2, acc, st, &S->x));
     }

@@ -183,8 +183,9 @@ cudaError_t launch_open_round(OpenState* s, int i, int d, const uint4* scal, con
 // 116-127 for k = 2; its k = 3 extension), observe the compressed round
 // polynomial, sample the challenge into s->x, and advance the claim
 // s->outer to the round polynomial at x (lib.rs:95-103).  `rec` receives
-// the compressed polynomial (16 k bytes) and the challenge (16 bytes).
-cudaError_t launch_sumcheck_round(OpenState* s, int k, const uint32_t* acc, uint8_t* rec, cudaStream_t st);
+// the compressed polynomial (16 k bytes) and the challenge (16 bytes); acc
+// (48 bytes) is cleared once read.
+cudaError_t launch_sumcheck_round(OpenState* s, int k, uint32_t* acc, uint8_t* rec, cudaStream_t st);
 
 // ---- the last rounds of open in one block, then the final polynomial
 constexpr int kTailThreads = 256;

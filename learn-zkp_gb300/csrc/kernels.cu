@@ -25,6 +25,7 @@
 #include "bf_internal.h"
 #include "gf128.cuh"
 #include "keccak.cuh"
+#include "launch.cuh"
 
 namespace bf {
 
@@ -644,6 +645,7 @@ __global__ void __launch_bounds__(128) leaves_pair_kernel(const uint4* __restric
 
 __global__ void __launch_bounds__(128) level_kernel(const uint4* __restrict__ prev, uint4* __restrict__ next,
                                                     size_t n_next) {
+  chain_wait();
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_next; s += (size_t)gridDim.x * blockDim.x)
     store_digest(next, s, hash_node(load_digest(prev, s), load_digest(prev, s + n_next)));
 }
@@ -654,6 +656,7 @@ __global__ void __launch_bounds__(kTreeThreads) tree_top_kernel(uint4* level, in
   __shared__ TreeShared sh;
   const WarpKeccak wk;
   const size_t n = (size_t)1 << k;
+  chain_wait();
   const uint4* root = tree_block(wk, sh.a, sh.b, level, 1, level + 2 * n, n, 0, k);
   if (root_out && threadIdx.x < 2) root_out[threadIdx.x] = root[threadIdx.x];
 }
@@ -674,6 +677,7 @@ __global__ void __cluster_dims__(kTopCluster, 1, 1) __launch_bounds__(kTreeThrea
   const WarpKeccak wk;
   const size_t n = (size_t)1 << k;
   cl.sync();  // block 0 is running: its shared memory may be written
+  chain_wait();
   const uint4* sub =
       tree_block(wk, sh.a, sh.b, level + 2 * r, kTopCluster, level + 2 * n, n, r, k - kTopClusterLog);
   uint4* dst = cl.map_shared_rank(roots, 0);
@@ -730,6 +734,7 @@ __global__ void __launch_bounds__(kTreeThreads) subtree_kernel(uint4* level, siz
   __shared__ TreeShared sh;
   const WarpKeccak wk;
   const size_t b = blockIdx.x;
+  chain_wait();
   tree_block(wk, sh.a, sh.b, level + 2 * b, n >> k, level + 2 * n, n, b, k);
 }
 
@@ -754,9 +759,8 @@ cudaError_t launch_tree(uint4* leaves, size_t n, cudaStream_t st, uint4* root_ou
       // the latency-bound middle levels in one launch: about one block per SM,
       // of 2^6 leaves (whose levels run on pairs of lanes and warps) to 2^9
       const int k = std::max(6, std::min(kTreeBlockLog, floor_log2(n) - 7));
-      subtree_kernel<<<(unsigned)(n >> k), kTreeThreads, 0, st>>>(cur, n, k);
+      cudaError_t e = launch_chained(subtree_kernel, (unsigned)(n >> k), kTreeThreads, 0, st, cur, n, k);
       COUNT_LAUNCH();
-      cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       for (int j = 0; j < k; ++j) {
         cur += 2 * n;
@@ -766,21 +770,21 @@ cudaError_t launch_tree(uint4* leaves, size_t n, cudaStream_t st, uint4* root_ou
     }
     const size_t h = n >> 1;
     uint4* nxt = cur + 2 * n;
-    level_kernel<<<grid_short(h, 128), 128, 0, st>>>(cur, nxt, h);
+    cudaError_t e = launch_chained(level_kernel, grid_short(h, 128), 128, 0, st, cur, nxt, h);
     COUNT_LAUNCH();
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     cur = nxt;
     n = h;
   }
+  cudaError_t e = cudaSuccess;
   if (n > kTopSingle) {
-    tree_top_cluster_kernel<<<kTopCluster, kTreeThreads, 0, st>>>(cur, floor_log2(n), root_out);
+    e = launch_chained(tree_top_cluster_kernel, kTopCluster, kTreeThreads, 0, st, cur, floor_log2(n), root_out);
     COUNT_LAUNCH();
   } else if (n > 1 || root_out) {
-    tree_top_kernel<<<1, kTreeThreads, 0, st>>>(cur, floor_log2(n), root_out);
+    e = launch_chained(tree_top_kernel, 1, kTreeThreads, 0, st, cur, floor_log2(n), root_out);
     COUNT_LAUNCH();
   }
-  return cudaGetLastError();
+  return e;
 }
 
 __device__ __forceinline__ uint64_t splitmix64(uint64_t& x) {
@@ -933,6 +937,7 @@ __global__ void __launch_bounds__(256, 3) fix_kernel(const uint4* in, uint4* out
                                                   const uint4* __restrict__ heq, size_t next_half, uint32_t* acc,
                                                   const uint4* xp) {
   __shared__ uint4 scratch[32];
+  chain_wait();
   if (xp) r = *xp;
   uint4 s = make_uint4(0, 0, 0, 0);
   for (size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x; b < half; b += (size_t)gridDim.x * blockDim.x) {
@@ -956,6 +961,7 @@ __global__ void __launch_bounds__(256, 3) fix_kernel(const uint4* in, uint4* out
 // alone at the end of the launch.
 __global__ void __launch_bounds__(128) fold_fix_kernel(FoldFixParams p, uint4 r) {
   __shared__ uint4 scratch[32];
+  chain_wait();
   if (p.xp) r = *p.xp;
   const unsigned S = p.fix_stride, q = blockIdx.x / S;
   const bool fix = blockIdx.x % S == S - 1 && q < p.fix_blocks;
@@ -996,16 +1002,17 @@ cudaError_t launch_fold_fix(const FoldFixParams& p0, uint4 r, cudaStream_t st) {
   p.fold_blocks = grid_short(p.n_leaves, 128);
   p.fix_blocks = grid_for(p.half, 128, 8);  // few blocks: each ends in one atomic
   p.fix_stride = (p.fold_blocks + p.fix_blocks) / p.fix_blocks;  // >= 2 while fold_blocks >= fix_blocks
-  fold_fix_kernel<<<p.fold_blocks + p.fix_blocks, 128, 0, st>>>(p, r);
+  const cudaError_t e = launch_chained(fold_fix_kernel, p.fold_blocks + p.fix_blocks, 128, 0, st, p, r);
   COUNT_LAUNCH();
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_fix(const uint4* in, uint4* out, size_t half, uint4 r, const uint4* heq, size_t next_half,
                        uint32_t* acc, cudaStream_t st, const uint4* xp) {
-  fix_kernel<<<grid_for(half, 256), 256, 0, st>>>(in, out, half, r, heq, next_half, acc, xp);
+  const cudaError_t e = launch_chained(fix_kernel, grid_for(half, 256), 256, 0, st, in, out, half, r, heq, next_half,
+                                       acc, xp);
   COUNT_LAUNCH();
-  return cudaGetLastError();
+  return e;
 }
 
 // First fix_last_var of column `col` of a row-major matrix with `width`
@@ -1028,6 +1035,7 @@ cudaError_t launch_fix_column(const uint4* in, size_t width, size_t col, uint4* 
 }
 
 __global__ void __launch_bounds__(512) eval_tail_kernel(uint4* buf, EvalTail p) {
+  chain_wait();
   for (int k = p.nvars - 1; k >= 0; --k) {
     const uint32_t half = 1u << k;
     const uint4 r = p.rp ? p.rp[k] : p.r[k];
@@ -1043,9 +1051,9 @@ __global__ void __launch_bounds__(512) eval_tail_kernel(uint4* buf, EvalTail p) 
 cudaError_t launch_eval_tail(uint4* buf, const EvalTail& p, cudaStream_t st) {
   if (p.nvars < 0 || p.nvars > kEvalTailMaxVars) return cudaErrorInvalidValue;
   if (p.nvars == 0) return cudaSuccess;
-  eval_tail_kernel<<<1, 512, 0, st>>>(buf, p);
+  const cudaError_t e = launch_chained(eval_tail_kernel, 1, 512, 0, st, buf, p);
   COUNT_LAUNCH();
-  return cudaGetLastError();
+  return e;
 }
 
 // out[row] = sum_c scalars[c] * rows[row * width + c]   (basefold.rs:166-183).
@@ -1276,6 +1284,7 @@ template <int K>
 __global__ void __launch_bounds__(256, 2) prod_fix_kernel(PolyPtrs p, size_t half, uint4 r, uint32_t* acc,
                                                        const uint4* xp) {
   __shared__ uint4 scratch[32];
+  chain_wait();
   if (xp) r = *xp;
   uint4 s0 = make_uint4(0, 0, 0, 0), s2 = s0, s3 = s0;
   const size_t nh = half >> 1;
@@ -1336,14 +1345,11 @@ cudaError_t launch_prod_fix(uint4* const* out, const uint4* const* in, int k, si
     p.out[i] = out[i];
   }
   const size_t work = half > 1 ? half / 2 : 1;
-  if (k == 2)
-    prod_fix_kernel<2><<<grid_for(work, 256), 256, 0, st>>>(p, half, r, acc, xp);
-  else if (k == 3)
-    prod_fix_kernel<3><<<grid_for(work, 256), 256, 0, st>>>(p, half, r, acc, xp);
-  else
-    return cudaErrorInvalidValue;
+  if (k != 2 && k != 3) return cudaErrorInvalidValue;
+  const cudaError_t e = launch_chained(k == 2 ? prod_fix_kernel<2> : prod_fix_kernel<3>, grid_for(work, 256), 256, 0, st,
+                                       p, half, r, acc, xp);
   COUNT_LAUNCH();
-  return cudaGetLastError();
+  return e;
 }
 
 // ---------------------------------------------------------------------------

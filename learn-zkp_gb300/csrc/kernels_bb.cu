@@ -17,6 +17,7 @@
 #include "bb_internal.h"
 #include "bf_internal.h"
 #include "keccak.cuh"
+#include "launch.cuh"
 
 namespace bf {
 
@@ -801,6 +802,7 @@ __device__ __forceinline__ E5 bb_interp(const E5& lo, const E5& hi, uint32_t t, 
   return bb::e_add(l, bb::e_mul(bb::e_sub(h, l), x));
 }
 __global__ void __launch_bounds__(128) bb_fold_kernel(BbFold p, E5 x) {
+  chain_wait();
   if (p.xp) x = ld_e5(p.xp, 0);
   const size_t n = p.n, q = n >> 1;
   const size_t work = q ? q : 1;  // n = 1: the single output, no leaves
@@ -1172,9 +1174,9 @@ cudaError_t bb_launch_fix(const uint32_t* in, int base, uint32_t* out, size_t ha
 
 cudaError_t bb_launch_fold(const BbFold& p, const E5& x, cudaStream_t st) {
   const size_t q = p.n / 2;
-  bb_fold_kernel<<<blocks_for(q ? q : 1, 128), 128, 0, st>>>(p, x);
+  const cudaError_t e = launch_chained(bb_fold_kernel, blocks_for(q ? q : 1, 128), 128, 0, st, p, x);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t bb_launch_gather(const BbGather& p, cudaStream_t st) {

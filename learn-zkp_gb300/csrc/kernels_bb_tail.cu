@@ -15,6 +15,7 @@
 #include "bb_internal.h"
 #include "bf_internal.h"
 #include "keccak.cuh"
+#include "launch.cuh"
 
 namespace bf {
 
@@ -209,6 +210,7 @@ __global__ void __launch_bounds__(32) bb_transcript_round_kernel(BbTranscript* t
                                                                 int canonical, uint32_t* x_out, uint8_t* rec) {
   __shared__ BbStepShared sh;
   const WarpKeccak wk;
+  chain_wait();
   tr_copy(&sh.t, t);
   const uint32_t v = (uint32_t)(sums[threadIdx.x % 5] % bb::P);
   __syncwarp();
@@ -236,6 +238,7 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
   __shared__ unsigned long long sums[2][5];  // this round's sum and the next one's
   const WarpKeccak wk;
   const int warp = threadIdx.x >> 5;
+  chain_wait();
   tr_copy(&sh.t, p.t);
   if (threadIdx.x < 10) sums[threadIdx.x / 5][threadIdx.x % 5] = 0;
   __syncthreads();
@@ -340,16 +343,17 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
 cudaError_t bb_launch_transcript_round(BbTranscript* t, const BbRoundConsts* c, int ri, const uint4* root_dev,
                                        const unsigned long long* sums, int canonical, uint32_t* x_out, uint8_t* rec,
                                        cudaStream_t st) {
-  bb_transcript_round_kernel<<<1, 32, 0, st>>>(t, c, ri, root_dev, sums, canonical, x_out, rec);
+  const cudaError_t e =
+      launch_chained(bb_transcript_round_kernel, 1, 32, 0, st, t, c, ri, root_dev, sums, canonical, x_out, rec);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t bb_launch_tail(const BbTail& p, cudaStream_t st) {
   if (p.i0 < 0 || (1 << (p.log2_n0 + p.i0)) > kBbTailMax) return cudaErrorInvalidValue;
-  bb_tail_kernel<<<1, kTreeThreads, 0, st>>>(p);
+  const cudaError_t e = launch_chained(bb_tail_kernel, 1, kTreeThreads, 0, st, p);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace bf

@@ -24,6 +24,7 @@
 #include "bf_internal.h"
 #include "gf128.cuh"
 #include "keccak.cuh"
+#include "launch.cuh"
 
 namespace bf {
 
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(32) open_round_kernel(OpenState* S, int i, int
                                                         const uint4* root, const uint4* Sred, uint8_t* rec) {
   __shared__ OpenState sh;
   const WarpKeccak wk;
+  chain_wait();
   state_load(sh, S);
   __syncthreads();
   round_step(wk, sh, i, d, scal, root[0], root[1], Sred[0], reinterpret_cast<uint4*>(rec));
@@ -252,6 +254,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
   const size_t c = (size_t)1 << P.log2_c;
   const WarpKeccak wk;
   const int warp = threadIdx.x >> 5;
+  chain_wait();
   state_load(sh, P.state);
   if (threadIdx.x == 0 && P.i0 >= 0) *reinterpret_cast<uint4*>(sums[0]) = P.S_i0[0];
   const uint4* root = P.root_i0;  // the round's tree root
@@ -365,14 +368,18 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
   state_store(P.state, sh);
 }
 
-// Product sumcheck round (warp): c = [c0, c2, c3] from the device sums.
-__global__ void __launch_bounds__(32) sumcheck_round_kernel(OpenState* S, int k, const uint32_t* acc, uint8_t* rec) {
+// Product sumcheck round (warp): c = [c0, c2, c3] from the device sums, which
+// it clears for the fix that accumulates the next round's.
+__global__ void __launch_bounds__(32) sumcheck_round_kernel(OpenState* S, int k, uint32_t* acc, uint8_t* rec) {
   __shared__ OpenState sh;
   const WarpKeccak wk;
+  chain_wait();
   state_load(sh, S);
   __syncthreads();
-  const uint4* a = reinterpret_cast<const uint4*>(acc);
+  uint4* a = reinterpret_cast<uint4*>(acc);
   const uint4 c0 = a[0], c2 = a[1], c3 = a[2];
+  __syncwarp();
+  if (wk.lane < 3) a[wk.lane] = make_uint4(0, 0, 0, 0);
   const uint4 sc = sh.outer;
   // k = 2: compressed [c0, c2] (the pair scalar is ONE, quadratic.rs:118),
   // round polynomial [c0, sc - 2 c0 - c2 = sc + c2, c2]; k = 3: compressed
@@ -410,11 +417,11 @@ __global__ void __launch_bounds__(32) sumcheck_round_kernel(OpenState* S, int k,
   state_store(S, sh);
 }
 
-cudaError_t launch_sumcheck_round(OpenState* s, int k, const uint32_t* acc, uint8_t* rec, cudaStream_t st) {
+cudaError_t launch_sumcheck_round(OpenState* s, int k, uint32_t* acc, uint8_t* rec, cudaStream_t st) {
   if (k != 2 && k != 3) return cudaErrorInvalidValue;
-  sumcheck_round_kernel<<<1, 32, 0, st>>>(s, k, acc, rec);
+  const cudaError_t e = launch_chained(sumcheck_round_kernel, 1, 32, 0, st, s, k, acc, rec);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_open_observe(OpenState* s, const uint4* root, const uint4* value, cudaStream_t st) {
@@ -425,15 +432,15 @@ cudaError_t launch_open_observe(OpenState* s, const uint4* root, const uint4* va
 
 cudaError_t launch_open_round(OpenState* s, int i, int d, const uint4* scal, const uint4* root, const uint4* S,
                               uint8_t* rec, cudaStream_t st) {
-  open_round_kernel<<<1, 32, 0, st>>>(s, i, d, scal, root, S, rec);
+  const cudaError_t e = launch_chained(open_round_kernel, 1, 32, 0, st, s, i, d, scal, root, S, rec);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_open_tail(const TailParams& p, cudaStream_t st) {
-  open_tail_kernel<<<1, kTailThreads, 0, st>>>(p);
+  const cudaError_t e = launch_chained(open_tail_kernel, 1, kTailThreads, 0, st, p);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace bf

@@ -1,0 +1,41 @@
+// Dependent launches.  The kernels of one proof form a chain on a stream, most
+// of them a few microseconds long, so the time between one kernel's end and the
+// next one's first instruction counts.  With programmatic dependent launch the
+// next grid is placed while its predecessor still runs and only its first
+// memory access waits: every kernel launched with launch_chained calls
+// chain_wait() before it touches memory that another kernel writes or reads
+// (which also orders it behind everything before its predecessor, since that
+// waited too), and then lets its own successor be placed.  Measured on GB300:
+// the 41 launches of a product sumcheck at 2^20 529 -> 388 us, a proof at 2^16
+// 1,336 -> 1,273 us.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace bf {
+
+// Returns when the preceding grid of the stream has completed and its writes
+// are visible; then the next one may be placed (it waits here in turn).
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t st,
+                                  A&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = shared;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+}  // namespace bf

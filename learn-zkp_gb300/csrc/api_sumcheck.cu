@@ -43,7 +43,7 @@ int sumcheck_run(cudaStream_t st, DevBuf& scratch, PinnedBuf& pinned, int k, int
     in[j] = polys + j * N;
   }
   ch.observe_elem(sc);  // lib.rs:67
-  const size_t pin_need = std::max(sizeof(bf::OpenState), rec_sz * (size_t)n + 16 * (size_t)k) + 64;
+  const size_t pin_need = sizeof(bf::OpenState) + rec_sz * (size_t)n + 16 * (size_t)k;
   if (ch.in.size() + 16 * (size_t)k <= (size_t)bf::kTrMax && ch.out.size() <= 32 && pinned.ensure(pin_need) == cudaSuccess) {
     // every round with the transcript on the device: sums, transcript step,
     // fix + next sums; one copy back at the end
@@ -60,18 +60,27 @@ int sumcheck_run(cudaStream_t st, DevBuf& scratch, PinnedBuf& pinned, int k, int
     CU(cudaMemcpyAsync(S, pinned.b(), sizeof(img), cudaMemcpyHostToDevice, st));
     CU(cudaMemsetAsync(acc, 0, 48, st));
     CU(bf::launch_prod_round_sums(in, k, half0, acc, st));
-    int ri = 0;
-    for (int round = n - 1; round >= 0; --round, ++ri) {
+    // large rounds one launch per step, the last ones in one block, which also
+    // writes the final evaluations after the records
+    int ri = 0, round = n - 1;
+    const uint4* const* src = in;
+    for (; round >= bf::kSumcheckTailLog; --round, ++ri) {
       CU(bf::launch_sumcheck_round(S, k, acc, rec + rec_sz * (size_t)ri, st));
       const size_t half = (size_t)1 << round;
-      const uint4* const* src = (round == n - 1) ? in : const_cast<const uint4* const*>(work);
       CU(bf::launch_prod_fix(work, src, k, half, uint4{}, half / 2, acc, st, &S->x));
+      src = work;
     }
-    uint8_t* fin = rec + rec_sz * (size_t)n;
-    for (int j = 0; j < k; ++j) CU(cudaMemcpyAsync(fin + 16 * j, work[j], 16, cudaMemcpyDeviceToDevice, st));
+    bf::SumcheckTail tp{};
+    for (int j = 0; j < k; ++j) tp.in[j] = src[j];
+    tp.m = round + 1;
+    tp.acc = acc;
+    tp.state = S;
+    tp.rec = rec + rec_sz * (size_t)ri;
+    CU(bf::launch_sumcheck_tail(tp, k, st));
     // pinned: records and final evaluations, then the state
     const size_t rec_bytes = rec_sz * (size_t)n + 16 * (size_t)k;
     CU(cudaMemcpyAsync(pinned.b(), rec, rec_bytes, cudaMemcpyDeviceToHost, st));
+    CU(cudaMemcpyAsync(pinned.b() + rec_bytes, S, sizeof(img), cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
     const uint8_t* r = pinned.b();
     for (int i = 0; i < n; ++i) {
@@ -79,9 +88,7 @@ int sumcheck_run(cudaStream_t st, DevBuf& scratch, PinnedBuf& pinned, int k, int
       std::memcpy(out + off_r + 16 * (size_t)i, r + rec_sz * (size_t)i + 16 * (size_t)k, 16);
     }
     std::memcpy(out + off_f, r + rec_sz * (size_t)n, 16 * (size_t)k);
-    CU(cudaMemcpyAsync(pinned.b(), S, sizeof(img), cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
-    std::memcpy(&img, pinned.b(), sizeof(img));
+    std::memcpy(&img, r + rec_bytes, sizeof(img));
     if (img.status != 0) return fail(BF_ERR_ARG, "transcript input outgrew the device buffer");
     ch.in.assign(img.tr.in, img.tr.in + img.tr.in_len);
     ch.out.assign(img.tr.out, img.tr.out + img.tr.out_len);

@@ -187,6 +187,20 @@ cudaError_t launch_open_round(OpenState* s, int i, int d, const uint4* scal, con
 // (48 bytes) is cleared once read.
 cudaError_t launch_sumcheck_round(OpenState* s, int k, uint32_t* acc, uint8_t* rec, cudaStream_t st);
 
+// The last m rounds of the product sumcheck in one block, from the first of
+// them's sums (acc, 48 bytes) and its k input polynomials of 2^m elements.
+// `rec` receives the rounds' records (as launch_sumcheck_round's) and then the
+// k final evaluations.
+constexpr int kSumcheckTailLog = 9;
+struct SumcheckTail {
+  const uint4* in[3];
+  int m;
+  const uint32_t* acc;
+  OpenState* state;
+  uint8_t* rec;
+};
+cudaError_t launch_sumcheck_tail(const SumcheckTail& p, int k, cudaStream_t st);
+
 // ---- the last rounds of open in one block, then the final polynomial
 constexpr int kTailThreads = 256;
 constexpr int kTailMaxLeavesLog = 11;    // largest Tune::tail_log

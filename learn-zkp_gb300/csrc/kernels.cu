@@ -422,33 +422,6 @@ __global__ void replicate_kernel(const uint4* __restrict__ m, uint4* __restrict_
   for (size_t i = threadIdx.x; i < c * w; i += blockDim.x) cw[i] = m[i % w];
 }
 
-void init_kernel_attributes() {
-  static std::atomic<uint64_t> done{0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const uint64_t bit = 1ull << (dev & 63);
-  if (done.load() & bit) return;
-  cudaFuncSetAttribute(ntt_pass_kernel<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(uint4) << kNttMaxT));
-  cudaFuncSetAttribute(ntt_pass_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(uint4) << kNttMaxT));
-  cudaFuncSetAttribute(ntt_pass_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(uint4) << kNttMaxT));
-  cudaFuncSetAttribute(ntt_pass_kernel<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(uint4) << kNttMaxT));
-  cudaFuncSetAttribute(ntt_pass_kernel<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(uint4) << kNttMaxT));
-  cudaFuncSetAttribute(ntt_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(uint4) << kNttMaxT));
-  cudaFuncSetAttribute(ntt_reg_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(uint4) << kNttRegMaxT));
-  cudaFuncSetAttribute(ntt_reg_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(uint4) << kNttRegMaxT));
-  cudaFuncSetAttribute(ntt_last_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(2 * sizeof(uint4) << kNttWsMaxT));
-  done.fetch_or(bit);
-}
-
 bool tune_valid(const Tune& t) {
   const bool threads_ok = t.ntt_threads == 128 || t.ntt_threads == 256 || t.ntt_threads == 512;
   const bool top_ok = t.top_nodes >= 64 && t.top_nodes <= 4096 && (t.top_nodes & (t.top_nodes - 1)) == 0;
@@ -1233,29 +1206,48 @@ struct PolyPtrs {
 __device__ __noinline__ uint4 gf_mul_call(uint4 a, uint4 b) { return gf_mul(a, b); }
 
 // Coefficients c0, c2 (and c3) of prod_k (lo_k + b_k X), b_k = hi_k - lo_k,
-// summed into s0, s2, s3.  For K = 3 the cross term lo1 b2 + b1 lo2 is
-// hi1 hi2 + lo1 lo2 + b1 b2 (characteristic 2, lo + b = hi), which reuses two
-// products the term needs anyway: 7 products instead of 8.
+// summed into s[0], s[1], s[2], unreduced (256-bit carry-less sums; the
+// reduction is GF(2)-linear, so one at the end of a thread's terms serves).
+// For K = 3 the cross term lo1 b2 + b1 lo2 is hi1 hi2 + lo1 lo2 + b1 b2
+// (characteristic 2, lo + b = hi), which reuses two products the term needs
+// anyway: 7 products instead of 8.
+struct ProdSums {
+  uint64_t s[3][4];
+  __device__ __forceinline__ uint4 reduced(int i) const { return gf_reduce256(s[i][0], s[i][1], s[i][2], s[i][3]); }
+};
 template <int K>
-__device__ __forceinline__ void prod_terms(const uint4 lo[K], const uint4 hi[K], uint4& s0, uint4& s2, uint4& s3) {
+__device__ __forceinline__ void prod_terms(const uint4 lo[K], const uint4 hi[K], ProdSums& t) {
   if (K == 2) {
-    s0 = gf_add(s0, gf_mul_call(lo[0], lo[1]));
-    s2 = gf_add(s2, gf_mul_call(gf_add(hi[0], lo[0]), gf_add(hi[1], lo[1])));
+    gf_clmul_acc(lo[0], lo[1], t.s[0]);
+    gf_clmul_acc(gf_add(hi[0], lo[0]), gf_add(hi[1], lo[1]), t.s[1]);
   } else {
-    const uint4 b0 = gf_add(hi[0], lo[0]), b1 = gf_add(hi[1], lo[1]), b2 = gf_add(hi[2], lo[2]);
+    const uint4 b0 = gf_add(hi[0], lo[0]), b1 = gf_add(hi[1], lo[1]), b2 = gf_add(hi[K - 1], lo[K - 1]);
     const uint4 b12 = gf_mul_call(b1, b2);
-    const uint4 lo12 = gf_mul_call(lo[1], lo[2]);
-    const uint4 cross = gf_add(gf_add(gf_mul_call(hi[1], hi[2]), lo12), b12);  // lo1 b2 + b1 lo2
-    s0 = gf_add(s0, gf_mul_call(lo[0], lo12));
-    s2 = gf_add(s2, gf_add(gf_mul_call(b0, cross), gf_mul_call(lo[0], b12)));
-    s3 = gf_add(s3, gf_mul_call(b0, b12));
+    const uint4 lo12 = gf_mul_call(lo[1], lo[K - 1]);
+    const uint4 cross = gf_add(gf_add(gf_mul_call(hi[1], hi[K - 1]), lo12), b12);  // lo1 b2 + b1 lo2
+    gf_clmul_acc(lo[0], lo12, t.s[0]);
+    gf_clmul_acc(b0, cross, t.s[1]);
+    gf_clmul_acc(lo[0], b12, t.s[1]);
+    gf_clmul_acc(b0, b12, t.s[2]);
+  }
+}
+
+// The block's sums into acc (c0, c2, c3, four words each); `scratch` holds 32
+// elements, free for every thread.
+template <int K>
+__device__ __forceinline__ void prod_sums_store(const ProdSums& t, uint4* scratch, uint32_t* acc) {
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const uint4 v = block_xor(t.reduced(i), scratch);
+    if (threadIdx.x == 0) atomic_xor4(acc + 4 * i, v);
+    __syncthreads();
   }
 }
 
 template <int K>
-__global__ void __launch_bounds__(256) prod_sums_kernel(PolyPtrs p, size_t half, uint32_t* acc) {
+__global__ void __launch_bounds__(256, 2) prod_sums_kernel(PolyPtrs p, size_t half, uint32_t* acc) {
   __shared__ uint4 scratch[32];
-  uint4 s0 = make_uint4(0, 0, 0, 0), s2 = s0, s3 = s0;
+  ProdSums t = {};
   for (size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x; b < half; b += (size_t)gridDim.x * blockDim.x) {
     uint4 lo[K], hi[K];
 #pragma unroll
@@ -1263,18 +1255,9 @@ __global__ void __launch_bounds__(256) prod_sums_kernel(PolyPtrs p, size_t half,
       lo[k] = p.in[k][b];
       hi[k] = p.in[k][b + half];
     }
-    prod_terms<K>(lo, hi, s0, s2, s3);
+    prod_terms<K>(lo, hi, t);
   }
-  s0 = block_xor(s0, scratch);
-  __syncthreads();
-  s2 = block_xor(s2, scratch);
-  __syncthreads();
-  if (K == 3) s3 = block_xor(s3, scratch);
-  if (threadIdx.x == 0) {
-    atomic_xor4(acc, s0);
-    atomic_xor4(acc + 4, s2);
-    if (K == 3) atomic_xor4(acc + 8, s3);
-  }
+  prod_sums_store<K>(t, scratch, acc);
 }
 
 // Fix the top variable of every polynomial at r and accumulate the next
@@ -1286,7 +1269,6 @@ __global__ void __launch_bounds__(256, 2) prod_fix_kernel(PolyPtrs p, size_t hal
   __shared__ uint4 scratch[32];
   chain_wait();
   if (xp) r = *xp;
-  uint4 s0 = make_uint4(0, 0, 0, 0), s2 = s0, s3 = s0;
   const size_t nh = half >> 1;
   if (nh == 0) {  // last round: one output per polynomial
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1298,6 +1280,7 @@ __global__ void __launch_bounds__(256, 2) prod_fix_kernel(PolyPtrs p, size_t hal
     }
     return;
   }
+  ProdSums t = {};
   for (size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x; b < nh; b += (size_t)gridDim.x * blockDim.x) {
     uint4 lo[K], hi[K];
 #pragma unroll
@@ -1309,18 +1292,52 @@ __global__ void __launch_bounds__(256, 2) prod_fix_kernel(PolyPtrs p, size_t hal
       p.out[k][b] = lo[k];
       p.out[k][b + nh] = hi[k];
     }
-    prod_terms<K>(lo, hi, s0, s2, s3);
+    prod_terms<K>(lo, hi, t);
   }
-  s0 = block_xor(s0, scratch);
+  prod_sums_store<K>(t, scratch, acc);
+}
+
+// The same fix for large rounds: the products by the challenge, 2 K of the 2 K
+// + 2 (K = 2) or + 7 (K = 3) products of an element pair, come from a
+// shared-memory table of r (GfTab), so the wide multiplier, which bounds
+// prod_fix_kernel, is left with the sums' products, and the table's loads run
+// beside it.  One persistent block per SM builds the table (about 3 us) and
+// walks the pairs.  Measured on GB300, clocks per pair and SM: K = 3 67 at 512
+// threads (68 at 384, 77 at 256; 95 without the table); K = 2 22 at 768
+// threads (24 at 512; 44).
+using ProdTab = GfTab<6>;
+constexpr size_t kProdTabShared = ProdTab::kBytes + 128 * sizeof(uint4);
+template <int K>
+constexpr int kProdTabThreads = K == 2 ? 768 : 512;
+template <int K>
+__global__ void __launch_bounds__(kProdTabThreads<K>, 1) prod_fix_tab_kernel(PolyPtrs p, size_t half, uint4 r,
+                                                                            uint32_t* acc, const uint4* xp) {
+  extern __shared__ uint4 sm[];
+  uint4* basis = sm + ProdTab::kBytes / sizeof(uint4);
+  chain_wait();
+  if (xp) r = *xp;
+  gf_basis(basis, r);
   __syncthreads();
-  s2 = block_xor(s2, scratch);
+  ProdTab::build(sm, basis);
   __syncthreads();
-  if (K == 3) s3 = block_xor(s3, scratch);
-  if (threadIdx.x == 0) {
-    atomic_xor4(acc, s0);
-    atomic_xor4(acc + 4, s2);
-    if (K == 3) atomic_xor4(acc + 8, s3);
+  const uint4* tab = sm + (threadIdx.x & 7u);
+  const size_t nh = half >> 1;
+  ProdSums t = {};
+  for (size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x; b < nh; b += (size_t)gridDim.x * blockDim.x) {
+    uint4 lo[K], hi[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const uint4 a0 = p.in[k][b], a1 = p.in[k][b + half];
+      const uint4 c0 = p.in[k][b + nh], c1 = p.in[k][b + nh + half];
+      lo[k] = gf_add(a0, ProdTab::mul(tab, gf_add(a1, a0)));
+      hi[k] = gf_add(c0, ProdTab::mul(tab, gf_add(c1, c0)));
+      p.out[k][b] = lo[k];
+      p.out[k][b + nh] = hi[k];
+    }
+    prod_terms<K>(lo, hi, t);
   }
+  __syncthreads();  // the table's last reads are done: its space serves the reductions
+  prod_sums_store<K>(t, sm, acc);
 }
 
 cudaError_t launch_prod_round_sums(const uint4* const* polys, int k, size_t half, uint32_t* acc, cudaStream_t st) {
@@ -1336,6 +1353,13 @@ cudaError_t launch_prod_round_sums(const uint4* const* polys, int k, size_t half
   return cudaGetLastError();
 }
 
+// Pairs from which a fix uses the table: below, building it (about 6 us more
+// than a small launch) costs more than its products save.  Measured on GB300,
+// without and with the table: k = 2 13.3 and 14.3 us at 2^16 pairs, 25.1 and
+// 23.2 at 2^17, 156 and 80 at 2^20; k = 3 16.1 and 22.3 us at 2^15, 27.1 and
+// 22.4 at 2^16, 325 and 239 at 2^20.
+constexpr size_t prod_tab_min(int k) { return (size_t)1 << (k == 2 ? 17 : 16); }
+
 cudaError_t launch_prod_fix(uint4* const* out, const uint4* const* in, int k, size_t half, uint4 r, size_t next_half,
                             uint32_t* acc, cudaStream_t st, const uint4* xp) {
   (void)next_half;
@@ -1346,6 +1370,14 @@ cudaError_t launch_prod_fix(uint4* const* out, const uint4* const* in, int k, si
   }
   const size_t work = half > 1 ? half / 2 : 1;
   if (k != 2 && k != 3) return cudaErrorInvalidValue;
+  if (work >= prod_tab_min(k)) {
+    init_kernel_attributes();
+    const cudaError_t e = launch_chained(k == 2 ? prod_fix_tab_kernel<2> : prod_fix_tab_kernel<3>, (unsigned)num_sms(),
+                                         k == 2 ? kProdTabThreads<2> : kProdTabThreads<3>, kProdTabShared, st, p, half,
+                                         r, acc, xp);
+    COUNT_LAUNCH();
+    return e;
+  }
   const cudaError_t e = launch_chained(k == 2 ? prod_fix_kernel<2> : prod_fix_kernel<3>, grid_for(work, 256), 256, 0, st,
                                        p, half, r, acc, xp);
   COUNT_LAUNCH();
@@ -1381,6 +1413,35 @@ cudaError_t launch_test_keccak(uint2* states, size_t n, cudaStream_t st) {
   test_keccak_kernel<<<grid_for(n, 128), 128, 0, st>>>(states, n);
   COUNT_LAUNCH();
   return cudaGetLastError();
+}
+
+void init_kernel_attributes() {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const uint64_t bit = 1ull << (dev & 63);
+  if (done.load() & bit) return;
+  cudaFuncSetAttribute(ntt_pass_kernel<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(uint4) << kNttMaxT));
+  cudaFuncSetAttribute(ntt_pass_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(uint4) << kNttMaxT));
+  cudaFuncSetAttribute(ntt_pass_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(uint4) << kNttMaxT));
+  cudaFuncSetAttribute(ntt_pass_kernel<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(uint4) << kNttMaxT));
+  cudaFuncSetAttribute(ntt_pass_kernel<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(uint4) << kNttMaxT));
+  cudaFuncSetAttribute(ntt_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(uint4) << kNttMaxT));
+  cudaFuncSetAttribute(ntt_reg_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(uint4) << kNttRegMaxT));
+  cudaFuncSetAttribute(ntt_reg_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(uint4) << kNttRegMaxT));
+  cudaFuncSetAttribute(ntt_last_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(2 * sizeof(uint4) << kNttWsMaxT));
+  cudaFuncSetAttribute(prod_fix_tab_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdTabShared);
+  cudaFuncSetAttribute(prod_fix_tab_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdTabShared);
+  done.fetch_or(bit);
 }
 
 }  // namespace bf

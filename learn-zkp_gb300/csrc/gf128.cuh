@@ -310,6 +310,7 @@ __device__ __forceinline__ void atomic_xor4(uint32_t* acc, uint4 v) {
 // 3.0 clocks per product and SM with G = 6 (128 KB), against 6.8 for gf_mul,
 // whose 144 IMAD.WIDE hold the multiplier; the two overlap (one gf_mul and two
 // table products 9.7 clocks).
+constexpr int kGfBasis = 132;  // elements a basis takes in shared memory (128, and slack that is read but not used)
 template <int G>
 struct GfTab {
   static_assert(G == 6 || G == 7, "6 groups: 6 6 5 5 5 5 bits; 7 groups: 6 5 5 4 4 4 4 bits");
@@ -326,10 +327,14 @@ struct GfTab {
   static constexpr int kEntries = 4 * kPerWord;
   static constexpr size_t kBytes = (size_t)kEntries * 128;  // eight copies of 16 bytes
 
-  // Fills the table from basis[k] = r x^k (bit k of a), k < 128, in shared
-  // memory; all threads of the block call this, the caller synchronizes.
+  // Fills the table from basis[k] (gf_basis), k < 128, in shared memory, which
+  // has kGfBasis elements; all threads of the block call this, the caller
+  // synchronizes.  An item is half of an entry's copies; the loads of a warp's
+  // entries of one group are broadcasts and unconditional (a bit past the
+  // group's width selects nothing).
   static __device__ __forceinline__ void build(uint4* tab, const uint4* basis) {
-    for (uint32_t e = threadIdx.x; e < (uint32_t)kEntries; e += blockDim.x) {
+    for (uint32_t it = threadIdx.x; it < 2u * kEntries; it += blockDim.x) {
+      const uint32_t h = it >= (uint32_t)kEntries, e = it - h * kEntries;
       const uint32_t w = e / kPerWord, q = e % kPerWord;
       int g = 0;
 #pragma unroll
@@ -339,10 +344,14 @@ struct GfTab {
       const uint4* b = basis + 32 * w + bit(g);
       uint4 s = make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int i = 0; i < 6; ++i)
-        if ((v >> i) & 1u) s = gf_add(s, b[i]);
+      for (int i = 0; i < 6; ++i) {
+        const uint32_t m = 0u - ((v >> i) & 1u);
+        const uint4 t = b[i];
+        s = make_uint4(s.x ^ (t.x & m), s.y ^ (t.y & m), s.z ^ (t.z & m), s.w ^ (t.w & m));
+      }
+      uint4* dst = tab + 8 * e;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) tab[8 * e + ((c + threadIdx.x) & 7u)] = s;
+      for (int c = 0; c < 4; ++c) dst[(4 * h + c + threadIdx.x) & 7u] = s;
     }
   }
 
@@ -364,14 +373,14 @@ struct GfTab {
   }
 };
 
-// basis[k] = r x^k for k < 128 by the block's first 128 threads; the caller
-// synchronizes.
-__device__ __forceinline__ void gf_basis(uint4* basis, uint4 r) {
-  if (threadIdx.x < 128) {
-    const uint32_t k = threadIdx.x, bit = 1u << (k & 31u);
-    basis[k] = gf_mul(r, make_uint4(k < 32 ? bit : 0u, k >= 32 && k < 64 ? bit : 0u, k >= 64 && k < 96 ? bit : 0u,
-                                    k >= 96 ? bit : 0u));
-  }
+// basis[k] = the product of r and the element with only bit k set, k < 128, by
+// the calling threads k = 0 .. 127: the carry-less product is r shifted left by k,
+// so only the reduction is left.  The caller synchronizes.
+__device__ __forceinline__ void gf_basis(uint4* basis, uint4 r, uint32_t k) {
+  const uint64_t r0 = ((uint64_t)r.y << 32) | r.x, r1 = ((uint64_t)r.w << 32) | r.z;
+  const uint32_t b = k & 63u;
+  const uint64_t l = r0 << b, m = (r1 << b) | (b ? r0 >> (64 - b) : 0), h = b ? r1 >> (64 - b) : 0;
+  basis[k] = k < 64 ? gf_reduce256(l, m, h, 0) : gf_reduce256(0, l, m, h);
 }
 
 }  // namespace bf

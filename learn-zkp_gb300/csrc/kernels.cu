@@ -417,6 +417,179 @@ __global__ void __launch_bounds__(kNttWsThreads, 1) ntt_last_ws_kernel(const uin
   }
 }
 
+// ---------------------------------------------------------------------------
+// Two layers at once over columns.  The rows x = hi 2^(s_lo+2) + a 2^s_lo + u,
+// a < 4, of one (coset, hi) meet in layers s_lo + 1 and s_lo whatever u and the
+// matrix column are, so C = width 2^s_lo neighbouring elements share the three
+// twiddles t (upper layer), u0 and u1 (lower layer).  Each thread takes four
+// rows of one column into registers:
+//   r0 = x0 + x2 t, r2 = x2 + r0;   r1 = x1 + x3 t, r3 = x3 + r1;
+//   y0 = r0 + r1 u0, y1 = r1 + y0;  y2 = r2 + r3 u1, y3 = r3 + y2.
+// With many columns per group (ntt_quad_tab_kernel) three of the four products
+// come from shared-memory tables of t and u0 (GfTab, 128 and 96 KB) and one from
+// the multiplier, which they relieve: measured 14.5 clocks per column and SM, against
+// 28 for four multiplied products.  A persistent block walks a run of columns
+// and rebuilds its tables where the group changes.  Bound by the shared-memory
+// and ALU pipes together (76 lookups, about 620 ALU instructions per column).
+// ---------------------------------------------------------------------------
+struct QuadPass {
+  int n, s_lo, first;  // first: read m, bit-reversed rows
+  // A first pass split by input slices (PassParams) runs the columns with
+  // u mod 2^piece_log = piece_u only, `run_cols` of them per group.
+  int piece_log;
+  uint32_t piece_u;
+  uint32_t width;
+  uint64_t cols, run_cols, total;  // C; the columns run per group; groups * run_cols
+};
+
+// Element indices of rows x0 .. x3 of the q-th column run of group g (g = coset
+// 2^(n - s_lo - 2) + hi), and of row 0 in cw.
+struct QuadAddr {
+  uint64_t src[4], dst;
+  __device__ __forceinline__ QuadAddr(const QuadPass& p, uint64_t g, uint64_t q) {
+    if (p.first) {  // row a 2^s_lo + u of the bit-reversed input is row brev(u) 4 + brev(a) of m
+      const uint64_t v = p.width == 1 ? q : q / p.width, col = q - v * p.width;
+      const uint32_t u = ((uint32_t)v << p.piece_log) | p.piece_u;
+      const uint64_t r = (uint64_t)brev_bits(u, p.s_lo) << 2;
+      src[0] = r * p.width + col;
+      src[1] = (r + 2) * p.width + col;
+      src[2] = (r + 1) * p.width + col;
+      src[3] = (r + 3) * p.width + col;
+      dst = (g << 2) * p.cols + (uint64_t)u * p.width + col;
+    } else {
+      dst = (g << 2) * p.cols + q;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) src[a] = dst + a * p.cols;
+    }
+  }
+};
+
+struct QuadTwiddles {
+  uint4 t, u0, u1;
+  bool has_t, has_u0;  // false: zero (index 0), the product is skipped
+  __device__ __forceinline__ QuadTwiddles(const QuadPass& p, uint64_t g, const TwiddleView* __restrict__ tw) {
+    const int hb = p.n - p.s_lo - 2;
+    const uint32_t j = (uint32_t)(g >> hb), hi = (uint32_t)(g & (((uint64_t)1 << hb) - 1));
+    const uint32_t k1 = (j << hb) | hi, k0 = (j << (hb + 1)) | (hi << 1);
+    t = gf_add(tw->lo[p.s_lo + 1][k1 & 4095u], tw->hi[p.s_lo + 1][k1 >> 12]);
+    u0 = gf_add(tw->lo[p.s_lo][k0 & 4095u], tw->hi[p.s_lo][k0 >> 12]);
+    u1 = gf_add(u0, tw->lo[p.s_lo][1]);  // linear in the index
+    has_t = k1 != 0;
+    has_u0 = k0 != 0;
+  }
+};
+
+constexpr int kQuadTabThreads = 512;
+using QuadTabT = GfTab<6>;
+using QuadTabU = GfTab<7>;
+constexpr size_t kQuadTabShared = QuadTabT::kBytes + QuadTabU::kBytes + kGfBasis * sizeof(uint4);
+
+__global__ void __launch_bounds__(kQuadTabThreads, 1) ntt_quad_tab_kernel(const uint4* __restrict__ m, uint4* cw,
+                                                                         QuadPass p,
+                                                                         const TwiddleView* __restrict__ tw) {
+  extern __shared__ uint4 sm[];
+  uint4* tab_t = sm;
+  uint4* tab_u = sm + QuadTabT::kBytes / sizeof(uint4);
+  uint4* basis = tab_u + QuadTabU::kBytes / sizeof(uint4);
+  const uint4* my_t = tab_t + (threadIdx.x & 7u);
+  const uint4* my_u = tab_u + (threadIdx.x & 7u);
+  const uint4* in = p.first ? m : cw;
+  // this block's run of (group, column) pairs
+  const uint64_t per = p.total / gridDim.x, rem = p.total % gridDim.x;
+  uint64_t pos = per * blockIdx.x + (blockIdx.x < rem ? blockIdx.x : rem);
+  const uint64_t end = pos + per + (blockIdx.x < rem ? 1 : 0);
+  while (pos < end) {
+    const uint64_t g = pos / p.run_cols, g0 = g * p.run_cols;
+    const uint64_t q_end = (end < g0 + p.run_cols ? end : g0 + p.run_cols) - g0;
+    uint64_t q = pos - g0 + threadIdx.x;
+    pos = g0 + q_end;
+    const QuadTwiddles w(p, g, tw);
+    uint4 x[4];
+    uint64_t dst = 0;
+    if (q < q_end) {  // in flight while the tables are built
+      const QuadAddr ad(p, g, q);
+      dst = ad.dst;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) x[a] = in[ad.src[a]];
+    }
+    __syncthreads();  // the last group's lookups are done
+    if (w.has_t) {
+      if (threadIdx.x < 128) gf_basis(basis, w.t, threadIdx.x);
+      __syncthreads();
+      QuadTabT::build(tab_t, basis);
+      __syncthreads();
+    }
+    if (w.has_u0) {
+      if (threadIdx.x < 128) gf_basis(basis, w.u0, threadIdx.x);
+      __syncthreads();
+      QuadTabU::build(tab_u, basis);
+      __syncthreads();
+    }
+    while (q < q_end) {
+      const uint64_t qn = q + kQuadTabThreads;
+      uint4 nx[4];
+      uint64_t nd = 0;
+      if (qn < q_end) {
+        const QuadAddr ad(p, g, qn);
+        nd = ad.dst;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) nx[a] = in[ad.src[a]];
+      }
+      if (w.has_t) {
+        x[0] = gf_add(x[0], QuadTabT::mul(my_t, x[2]));
+        x[1] = gf_add(x[1], QuadTabT::mul(my_t, x[3]));
+      }
+      x[2] = gf_add(x[2], x[0]);
+      x[3] = gf_add(x[3], x[1]);
+      if (w.has_u0) x[0] = gf_add(x[0], QuadTabU::mul(my_u, x[1]));
+      x[1] = gf_add(x[1], x[0]);
+      x[2] = gf_add(x[2], gf_mul(x[3], w.u1));
+      x[3] = gf_add(x[3], x[2]);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) cw[dst + a * p.cols] = x[a];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) x[a] = nx[a];
+      q = qn;
+      dst = nd;
+    }
+  }
+}
+
+// The same two layers (or, with ONE, layer s_lo alone) for groups of too few
+// columns for a table: every product multiplied, one thread per column of a group.
+template <bool ONE>
+__global__ void __launch_bounds__(256, 2) ntt_quad_kernel(uint4* cw, QuadPass p, const TwiddleView* __restrict__ tw) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= p.total) return;
+  const uint64_t g = i / p.cols, q = i - g * p.cols;
+  if (ONE) {  // rows hi 2^(s_lo+1) + a 2^s_lo + u, a < 2
+    uint4* io = cw + (g << 1) * p.cols + q;
+    const uint32_t k = (uint32_t)g;  // coset 2^(n-1-s_lo) + hi
+    uint4 x0 = io[0], x1 = io[p.cols];
+    if (k != 0) x0 = gf_add(x0, gf_mul(x1, gf_add(tw->lo[p.s_lo][k & 4095u], tw->hi[p.s_lo][k >> 12])));
+    io[0] = x0;
+    io[p.cols] = gf_add(x1, x0);
+    return;
+  }
+  const QuadTwiddles w(p, g, tw);
+  uint4* io = cw + (g << 2) * p.cols + q;
+  uint4 x[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) x[a] = io[a * p.cols];
+  if (w.has_t) {
+    x[0] = gf_add(x[0], gf_mul(x[2], w.t));
+    x[1] = gf_add(x[1], gf_mul(x[3], w.t));
+  }
+  x[2] = gf_add(x[2], x[0]);
+  x[3] = gf_add(x[3], x[1]);
+  if (w.has_u0) x[0] = gf_add(x[0], gf_mul(x[1], w.u0));
+  x[1] = gf_add(x[1], x[0]);
+  x[2] = gf_add(x[2], gf_mul(x[3], w.u1));
+  x[3] = gf_add(x[3], x[2]);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) io[a * p.cols] = x[a];
+}
+
 // n = 0: every coset is the single row of m.
 __global__ void replicate_kernel(const uint4* __restrict__ m, uint4* __restrict__ cw, size_t c, size_t w) {
   for (size_t i = threadIdx.x; i < c * w; i += blockDim.x) cw[i] = m[i % w];
@@ -429,6 +602,20 @@ bool tune_valid(const Tune& t) {
          t.tail_log <= kTailMaxLeavesLog && t.subtree_log >= 10 && t.subtree_log <= 20 && t.ntt_kind >= 0 &&
          t.ntt_kind <= 3 && t.gf_mix >= 0 && t.gf_mix <= 4 && t.ntt_ws_warps >= 2 && t.ntt_ws_warps <= 14;
 }
+
+// Column passes with tables: elements of the codeword from which they pay, and
+// columns per group (a group's tables cost about 5 us with the pipeline's drain;
+// at 1024 columns a pass of 2^25 elements takes 653 us, 797 multiplied, 385 with
+// 2^14 columns or more).  Measured on GB300, encode without and with them:
+// width 1, blowup 2, 2^19 rows 592 and 657 us, 2^20 1189 and 1142, 2^24 19.41 and
+// 17.43 ms; 2^14 x 16 107 and 125 us, 2^15 x 16 207 and 197, 2^11 x 256 168 and
+// 150, 2^16 x 256 6.50 and 3.90 ms.
+constexpr size_t quad_tab_elems(size_t width) { return (size_t)1 << (width == 1 ? 21 : 20); }
+constexpr size_t kQuadTabCols = 1024;
+// Without tables, for the layers left of a wide matrix: at least kQuadWide columns
+// and at most kQuadRest layers (more layers run faster in shared memory).
+constexpr size_t kQuadWide = 16;
+constexpr int kQuadRest = 6;
 
 static void launch_ntt_nohash(dim3 grid, int threads, size_t smem, cudaStream_t s, const uint4* m, uint4* cw,
                               const PassParams& p, const TwiddleView* tw, int gf_mix) {
@@ -505,19 +692,81 @@ cudaError_t launch_encode(const uint4* m, uint4* cw, int n, int log2_c, size_t w
     return cudaGetLastError();
   }
   init_kernel_attributes();
-  // Fewest passes whose tiles fit 2^ntt_max_T, then more (smaller tiles) while
-  // a pass would have fewer blocks than SMs and tiles stay >= 2^5.
-  int passes = (n + tune.ntt_max_T - 1) / tune.ntt_max_T;
-  while (passes < n) {
-    const int T = (n + passes - 1) / passes;
-    const int T_next = (n + passes) / (passes + 1);
-    if ((c << (n - T)) >= (size_t)num_sms() || T_next < 5) break;
-    ++passes;
-  }
+  // Layers [0, top) in the fewest passes whose tiles fit 2^ntt_max_T, then more
+  // (smaller tiles) while a pass would have fewer blocks than SMs (a matrix,
+  // one column per block: than two per SM) and tiles stay >= 2^5.  Measured for
+  // matrices, blowup 2: 2^13 x 37 112 us in two passes, 336 in the three that
+  // counting one column's blocks gave; 2^12 x 100 137 us in two, 209 in one.
+  const size_t want = (size_t)num_sms() * (width > 1 ? 2 : 1);
+  auto plan_passes = [&](int top) {
+    int passes = (top + tune.ntt_max_T - 1) / tune.ntt_max_T;
+    while (passes < top) {
+      const int T = (top + passes - 1) / passes;
+      const int T_next = (top + passes) / (passes + 1);
+      if ((c << (n - T)) * width >= want || T_next < 5) break;
+      ++passes;
+    }
+    return passes;
+  };
+  int passes = plan_passes(n);
   if (tune.ntt_kind == 3 && passes == 2 && leaves && pair_leaves && slices == 0 && st2 && ev_a && ev_b)
     return encode_pipelined(m, cw, n, log2_c, tw, st, st2, ev_a, ev_b, leaves, pair_leaves, tune, (n + 1) / 2,
                             last_a, last_b);
+  // Pairs of layers over columns (kind 2): with tables while a group has at least
+  // kQuadTabCols columns, when the encode is large enough; the last few layers of
+  // a wide matrix without.
   int top = n;
+  auto quad_pass = [&](bool tab, bool one, int piece_log, int piece) {
+    QuadPass q{};
+    q.n = n;
+    q.s_lo = top - (one ? 1 : 2);
+    q.first = top == n;
+    q.piece_log = piece_log;
+    q.piece_u = 0;
+    for (int b = 0; b < piece_log; ++b) q.piece_u |= (uint32_t)((piece >> b) & 1) << (piece_log - 1 - b);
+    q.width = (uint32_t)width;
+    q.cols = (uint64_t)width << q.s_lo;
+    q.run_cols = q.cols >> piece_log;
+    q.total = (((uint64_t)c << n) * width) >> ((one ? 1 : 2) + piece_log);
+    const unsigned blocks = (unsigned)((q.total + 255) / 256);
+    if (tab)
+      ntt_quad_tab_kernel<<<(unsigned)num_sms(), kQuadTabThreads, kQuadTabShared, st>>>(m, cw, q, tw);
+    else if (one)
+      ntt_quad_kernel<true><<<blocks, 256, 0, st>>>(cw, q, tw);
+    else
+      ntt_quad_kernel<false><<<blocks, 256, 0, st>>>(cw, q, tw);
+    COUNT_LAUNCH();
+    return cudaGetLastError();
+  };
+  if (tune.ntt_kind == 2 && tune.gf_mix == 0 && (c << n) * width >= quad_tab_elems(width)) {
+    while (top >= 2 && (width << (top - 2)) >= kQuadTabCols) {
+      int piece_log = 0;  // the first pass may start on each slice of the input as it arrives
+      if (top == n && slices > 0) {
+        while ((1 << piece_log) < slices) ++piece_log;
+        if ((1 << piece_log) != slices || piece_log > n - 2) {
+          piece_log = 0;
+          const cudaError_t e = cudaStreamWaitEvent(st, slice_ready[slices - 1], 0);  // copies are in order
+          if (e != cudaSuccess) return e;
+        }
+      }
+      for (int piece = 0; piece < (1 << piece_log); ++piece) {
+        cudaError_t e = piece_log ? cudaStreamWaitEvent(st, slice_ready[piece], 0) : cudaSuccess;
+        if (e == cudaSuccess) e = quad_pass(true, false, piece_log, piece);
+        if (e != cudaSuccess) return e;
+      }
+      top -= 2;
+    }
+    if (top < n && width >= kQuadWide && top <= kQuadRest) {  // the rest of a wide matrix
+      cudaError_t e = last_a ? cudaEventRecord(last_a, st) : cudaSuccess;
+      while (e == cudaSuccess && top > 0) {
+        e = quad_pass(false, top == 1, 0, 0);
+        top -= top == 1 ? 1 : 2;
+      }
+      if (e == cudaSuccess && last_b) e = cudaEventRecord(last_b, st);
+      return e;
+    }
+    if (top < n) passes = plan_passes(top);
+  }
   for (int pidx = 0; pidx < passes; ++pidx) {
     const int remaining = passes - pidx;
     const int T = (top + remaining - 1) / remaining;  // balanced split, largest first
@@ -525,7 +774,7 @@ cudaError_t launch_encode(const uint4* m, uint4* cw, int n, int log2_c, size_t w
     p.n = n;
     p.T = T;
     p.s_lo = top - T;
-    p.first = (pidx == 0);
+    p.first = (top == n);
     p.width = (int)width;
     const bool last = (pidx == passes - 1);
     p.leaves = last ? leaves : nullptr;
@@ -1306,7 +1555,7 @@ __global__ void __launch_bounds__(256, 2) prod_fix_kernel(PolyPtrs p, size_t hal
 // threads (68 at 384, 77 at 256; 95 without the table); K = 2 22 at 768
 // threads (24 at 512; 44).
 using ProdTab = GfTab<6>;
-constexpr size_t kProdTabShared = ProdTab::kBytes + 128 * sizeof(uint4);
+constexpr size_t kProdTabShared = ProdTab::kBytes + kGfBasis * sizeof(uint4);
 template <int K>
 constexpr int kProdTabThreads = K == 2 ? 768 : 512;
 template <int K>
@@ -1316,7 +1565,7 @@ __global__ void __launch_bounds__(kProdTabThreads<K>, 1) prod_fix_tab_kernel(Pol
   uint4* basis = sm + ProdTab::kBytes / sizeof(uint4);
   chain_wait();
   if (xp) r = *xp;
-  gf_basis(basis, r);
+  if (threadIdx.x < 128) gf_basis(basis, r, threadIdx.x);
   __syncthreads();
   ProdTab::build(sm, basis);
   __syncthreads();
@@ -1441,6 +1690,7 @@ void init_kernel_attributes() {
                        (int)(2 * sizeof(uint4) << kNttWsMaxT));
   cudaFuncSetAttribute(prod_fix_tab_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdTabShared);
   cudaFuncSetAttribute(prod_fix_tab_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdTabShared);
+  cudaFuncSetAttribute(ntt_quad_tab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQuadTabShared);
   done.fetch_or(bit);
 }
 

@@ -113,6 +113,37 @@ struct PassParams {
   int coset0;      // the launch covers cosets coset0, coset0 + 1, ... (grid / tiles per coset of them)
 };
 
+// The leaf hashes of a tile of 2^T codeword elements at buf (position q0 of the
+// codeword), by threads t, t + nthr, ..: per pair the two codeword leaves
+// H(cw[q]) and the folded-codeword leaf H(cw[2s] || cw[2s+1]).  A tile with fewer
+// pairs than threads takes its hashes one by one instead, so that all threads
+// hash at once: a thread per pair runs three permutations of 4.1 us one after
+// another (GB300, encode with leaves at 2^10 20.7 us, 28.9 per pair; at 2^15 67.6
+// and 84.2).  With pairs for every thread the pair order is the faster (2^24
+// 17.41 ms, 17.49 one by one).
+__device__ __forceinline__ void hash_tile(const PassParams& p, const uint4* buf, uint32_t tsize, size_t q0, uint32_t t,
+                                          uint32_t nthr) {
+  const uint32_t pairs = tsize >> 1;
+  if (pairs >= nthr) {
+    for (uint32_t k = t; k < pairs; k += nthr) {
+      const uint4 e0 = buf[2 * k], e1 = buf[2 * k + 1];
+      const size_t q = q0 + 2 * k;
+      store_digest(p.leaves, q, hash_elem(e0));
+      store_digest(p.leaves, q + 1, hash_elem(e1));
+      store_digest(p.pair_leaves, q >> 1, hash_pair(e0, e1));
+    }
+    return;
+  }
+  for (uint32_t i = t; i < tsize + pairs; i += nthr) {
+    if (i < tsize) {
+      store_digest(p.leaves, q0 + i, hash_elem(buf[i]));
+    } else {
+      const uint32_t k = i - tsize;
+      store_digest(p.pair_leaves, (q0 >> 1) + k, hash_pair(buf[2 * k], buf[2 * k + 1]));
+    }
+  }
+}
+
 // H: field products take H of their nine 32 x 32 products from the 16-bit
 // form (gf_mul_mix), moving multiplier work of the passes without hashing,
 // which are bound by the wide multiplies, onto the ALU pipe.
@@ -175,14 +206,7 @@ __global__ void __launch_bounds__(512) ntt_pass_kernel(const uint4* __restrict__
   }
   if (HASH) {
     // last pass: s_lo = 0, the tile is the contiguous run [coset_base + hi 2^T, +2^T)
-    const size_t q0 = coset_base + ((size_t)hi << T);
-    for (uint32_t k = threadIdx.x; k < (tsize >> 1); k += blockDim.x) {
-      const uint4 e0 = sm[2 * k], e1 = sm[2 * k + 1];
-      const size_t q = q0 + 2 * k;
-      store_digest(p.leaves, q, hash_elem(e0));
-      store_digest(p.leaves, q + 1, hash_elem(e1));
-      store_digest(p.pair_leaves, q >> 1, hash_pair(e0, e1));
-    }
+    hash_tile(p, sm, tsize, coset_base + ((size_t)hi << T), threadIdx.x, blockDim.x);
   }
 }
 
@@ -405,13 +429,7 @@ __global__ void __launch_bounds__(kNttWsThreads, 1) ntt_last_ws_kernel(const uin
       const size_t q0 = ((size_t)j << n) + ((size_t)hi << T);
       const uint4* buf = sm + ((k & 1u) << T);
       named_sync(2 + (int)(k & 1u), kNttWsThreads);
-      for (uint32_t kk = t; kk < (tsize >> 1); kk += hthr) {
-        const uint4 e0 = buf[2 * kk], e1 = buf[2 * kk + 1];
-        const size_t q = q0 + 2 * kk;
-        store_digest(p.leaves, q, hash_elem(e0));
-        store_digest(p.leaves, q + 1, hash_elem(e1));
-        store_digest(p.pair_leaves, q >> 1, hash_pair(e0, e1));
-      }
+      hash_tile(p, buf, tsize, q0, t, hthr);
       if (k + 2 < K) named_arrive(4 + (int)(k & 1u), kNttWsThreads);  // the butterfly warps may refill it
     }
   }
@@ -783,7 +801,8 @@ cudaError_t launch_encode(const uint4* m, uint4* cw, int n, int log2_c, size_t w
     p.ntt_warps = tune.ntt_ws_warps;
     p.coset0 = 0;
     // one butterfly per thread and layer at most: 2^(T-1) threads, >= one warp
-    const int threads = std::max(32, std::min(tune.ntt_threads, 1 << (T - 1)));
+    // (a tile that is hashed: one leaf per thread)
+    const int threads = std::max(32, std::min(tune.ntt_threads, p.leaves ? (3 << (T - 1)) + 31 & ~31 : 1 << (T - 1)));
     const uint32_t tiles = 1u << (n - T);
     // the first pass may start on each slice of the input as it arrives
     // (slices a power of two, at most the tiles per coset)
@@ -1219,8 +1238,71 @@ __global__ void __launch_bounds__(128) fold_fix_kernel(FoldFixParams p, uint4 r)
   if (threadIdx.x == 0) atomic_xor4(p.acc, acc);
 }
 
+// The same for smaller rounds, whose time is one thread's chain of four products
+// and a permutation: a block takes 64 leaves, one thread per fold output (two
+// products), then a pair of lanes per leaf hash (PairKeccak).  Blocks past
+// fold_blocks fix.
+constexpr int kFoldSmallLeaves = 64;
+__global__ void __launch_bounds__(2 * kFoldSmallLeaves) fold_fix_small_kernel(FoldFixParams p, uint4 r) {
+  __shared__ uint4 scratch[32];
+  __shared__ uint4 msg[2 * kFoldSmallLeaves];  // the outputs as interleaved lanes
+  chain_wait();
+  if (p.xp) r = *p.xp;
+  if (blockIdx.x < p.fold_blocks) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 2 * p.n_leaves) {
+      const uint4 tw = gf_add(p.tlo[t & 4095], p.thi[t >> 12]);
+      uint4 lo = p.pi[2 * t], hi = p.pi[2 * t + 1];
+      hi = gf_add(hi, lo);
+      lo = gf_add(lo, gf_mul(hi, tw));
+      const uint4 f = gf_add(lo, gf_mul(gf_add(hi, lo), r));
+      p.pi_out[t] = f;
+      const uint2 m0 = bi_from_lane(make_uint2(f.x, f.y)), m1 = bi_from_lane(make_uint2(f.z, f.w));
+      msg[threadIdx.x] = make_uint4(m0.x, m0.y, m1.x, m1.y);
+    }
+    __syncthreads();
+    const size_t s = (size_t)blockIdx.x * kFoldSmallLeaves + (threadIdx.x >> 1);
+    const uint32_t h = threadIdx.x & 1u;
+    const PairKeccak pk;
+    uint32_t st[25];
+    const uint32_t* l = reinterpret_cast<const uint32_t*>(msg + 2 * (threadIdx.x >> 1)) + h;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) st[i] = l[2 * i];
+    pk.keccak256(st, 4);
+    if (s < p.n_leaves) {
+      uint32_t* d = reinterpret_cast<uint32_t*>(p.leaves + 2 * s) + h;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d[2 * i] = st[i];
+    }
+    return;
+  }
+  uint4 acc = make_uint4(0, 0, 0, 0);
+  for (size_t b = (size_t)(blockIdx.x - p.fold_blocks) * blockDim.x + threadIdx.x; b < p.half;
+       b += (size_t)p.fix_blocks * blockDim.x) {
+    const uint4 lo = p.poly_in[b], hi = p.poly_in[b + p.half];
+    const uint4 v = gf_add(lo, gf_mul(r, gf_add(hi, lo)));
+    p.poly_out[b] = v;
+    if (b < p.next_half) acc = gf_add(acc, gf_mul(p.heq[b], v));
+  }
+  acc = block_xor(acc, scratch);
+  if (threadIdx.x == 0) atomic_xor4(p.acc, acc);
+}
+
+// Leaves up to which the small form runs.  Measured on GB300, one thread per leaf
+// and small form: 2^10 leaves 8.4 and 5.5 us, 2^15 24.8 and 15.2, 2^17 56 and 50,
+// 2^18 93 and 97 (the pairs' shuffles cost once the ALUs are full).
+constexpr size_t kFoldSmallMax = (size_t)1 << 17;
+
 cudaError_t launch_fold_fix(const FoldFixParams& p0, uint4 r, cudaStream_t st) {
   FoldFixParams p = p0;
+  if (p.n_leaves <= kFoldSmallMax) {
+    p.fold_blocks = (unsigned)((p.n_leaves + kFoldSmallLeaves - 1) / kFoldSmallLeaves);
+    p.fix_blocks = grid_for(p.half, 2 * kFoldSmallLeaves, 8);  // few blocks: each ends in one atomic
+    const cudaError_t e = launch_chained(fold_fix_small_kernel, p.fold_blocks + p.fix_blocks, 2 * kFoldSmallLeaves, 0, st,
+                                         p, r);
+    COUNT_LAUNCH();
+    return e;
+  }
   p.fold_blocks = grid_short(p.n_leaves, 128);
   p.fix_blocks = grid_for(p.half, 128, 8);  // few blocks: each ends in one atomic
   p.fix_stride = (p.fold_blocks + p.fix_blocks) / p.fix_blocks;  // >= 2 while fold_blocks >= fix_blocks

@@ -820,6 +820,43 @@ __global__ void __launch_bounds__(128) bb_fold_kernel(BbFold p, E5 x) {
   }
 }
 
+// The same for smaller rounds, whose time is one thread's two outputs and a
+// permutation one after another: a block takes 64 leaves, one thread per output
+// (threads 0 .. 63 out[s], 64 .. 127 out[s + n/2]), then a pair of lanes per leaf
+// hash (PairKeccak).
+constexpr int kBbFoldLeaves = 64;
+__global__ void __launch_bounds__(2 * kBbFoldLeaves) bb_fold_small_kernel(BbFold p, E5 x) {
+  __shared__ uint32_t w[kBbFoldLeaves][10];  // canonical words of out[s], out[s + n/2]
+  chain_wait();
+  if (p.xp) x = ld_e5(p.xp, 0);
+  const size_t n = p.n, q = n >> 1, s0 = (size_t)blockIdx.x * kBbFoldLeaves;
+  const int k = threadIdx.x / kBbFoldLeaves, i = threadIdx.x % kBbFoldLeaves;
+  if (s0 + i < q) {
+    const size_t j = s0 + i + (k ? q : 0);
+    const E5 lo = p.base ? bb::e_from(p.w[j]) : ld_e5(p.w, j);
+    const E5 hi = p.base ? bb::e_from(p.w[j + n]) : ld_e5(p.w, j + n);
+    const E5 f = bb_interp(lo, hi, p.tinv[j], x);
+    st_e5(p.out, j, f);
+#pragma unroll
+    for (int e = 0; e < 5; ++e) w[i][5 * k + e] = bb::from_mont(f.c[e]);
+  }
+  __syncthreads();
+  const int t = threadIdx.x >> 1;
+  const PairKeccak pk;
+  uint32_t st[25];
+#pragma unroll
+  for (int e = 0; e < 5; ++e) {
+    const uint2 l = bi_from_lane(make_uint2(w[t][2 * e], w[t][2 * e + 1]));
+    st[e] = pk.odd ? l.y : l.x;
+  }
+  pk.keccak256(st, 5);
+  if (s0 + t < q) {
+    uint32_t* d = reinterpret_cast<uint32_t*>(p.leaves + 2 * (size_t)brev_bits(s0 + t, p.leaf_bits)) + (pk.odd ? 1 : 0);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) d[2 * e] = st[e];
+  }
+}
+
 // ---- query openings (basefold.rs:200-222) ---------------------------------------
 // One block per query; every field of the record sits on a 4-byte boundary.
 __device__ __forceinline__ void put64w(uint32_t* o, size_t wo, uint64_t v) {
@@ -1172,8 +1209,19 @@ cudaError_t bb_launch_fix(const uint32_t* in, int base, uint32_t* out, size_t ha
   return cudaGetLastError();
 }
 
+// Leaves up to which the small fold runs.  Measured on GB300, one thread per leaf
+// and small form: 2^10 leaves 6.9 and 5.1 us, 2^13 7.2 and 5.2, 2^14 7.2 and 7.5,
+// 2^20 243 and 284.
+constexpr size_t kBbFoldSmallMax = (size_t)1 << 13;
+
 cudaError_t bb_launch_fold(const BbFold& p, const E5& x, cudaStream_t st) {
   const size_t q = p.n / 2;
+  if (p.leaves && q && q <= kBbFoldSmallMax) {
+    const cudaError_t e = launch_chained(bb_fold_small_kernel, (unsigned)((q + kBbFoldLeaves - 1) / kBbFoldLeaves),
+                                         2 * kBbFoldLeaves, 0, st, p, x);
+    count_launch();
+    return e;
+  }
   const cudaError_t e = launch_chained(bb_fold_kernel, blocks_for(q ? q : 1, 128), 128, 0, st, p, x);
   count_launch();
   return e;

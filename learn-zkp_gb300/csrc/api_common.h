@@ -244,6 +244,7 @@ struct bf_pcs {
   bfapi::Profiler prof;
   bf::Tune tune;  // launch shapes and thresholds (bf_pcs_autotune / bf_pcs_set_tune)
   // bf_verify_batch staging (grow-only): proofs and query records in, flags out
+  bool reads_host = false;  // the device reads pageable host memory through the host's page tables
   bfapi::PinnedBuf verify_pin;
   bfapi::DevBuf verify_dev;
   std::mutex verify_mu;

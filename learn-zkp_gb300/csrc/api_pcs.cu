@@ -469,6 +469,12 @@ int bf_pcs_setup(int device, int lambda, int log2_c, int num_vars, void* stream,
   CU(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
   CU(cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming));
   for (cudaEvent_t& e : p->slice_ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  {
+    int pageable = 0, tables = 0;
+    CU(cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device));
+    CU(cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device));
+    p->reads_host = pageable != 0 && tables != 0;
+  }
   TRY(build_twiddles(p.get()));
   bf::init_kernel_attributes();
   CU(p->pinned.ensure(4096));

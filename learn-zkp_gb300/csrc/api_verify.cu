@@ -1,6 +1,8 @@
 // libbasefold_gpu.so: the Basefold verifier on the host.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -270,6 +272,7 @@ bool parse_layout(const uint8_t* b, size_t n, Layout& lay) {
       if (!r.skip(32 * m)) return false;
       lay.ext.push_back(x);
     }
+    if (&o == &lay.open.front() && k) lay.ext.reserve(std::min<uint64_t>(k * a, n / 24));  // alike openings, 24 bytes a round
   }
   return r.ok && r.off == n;
 }
@@ -282,7 +285,11 @@ struct VJob {
   std::vector<uint64_t> idx;   // query positions
   size_t nq_dev = 0;
   int after = BF_VERIFY_OK;  // status of query nq_dev, decided by its structure (or OK: none left)
-  uint64_t elems = 0, proof = 0;  // device image offsets
+  uint64_t elems = 0;  // device image offset
+  // where the kernels read the proof: the caller's bytes in place, or (staged)
+  // their copy at this device image offset
+  uint64_t proof = 0;
+  bool staged = false;
 };
 
 // The transcript part of bf_verify for one job: the same observations,
@@ -363,19 +370,22 @@ void verify_host_part(const bf_pcs* p, const bf_verify_job& jb, VJob& v) {
   if (v.nq_dev == 0) v.status = v.after;
 }
 
+// f(0) .. f(count - 1) on up to 16 threads, the calling one among them; a thread
+// takes the next job as it finishes one.
 template <class F>
 void parallel_jobs(size_t count, F&& f) {
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
   const size_t nt = std::min<size_t>({(size_t)hw, (size_t)16, (count + 3) / 4});
-  if (nt <= 1) {
-    for (size_t i = 0; i < count; ++i) f(i);
-    return;
-  }
+  std::atomic<size_t> next{0};
+  auto work = [&] {
+    for (size_t i; (i = next.fetch_add(1, std::memory_order_relaxed)) < count;) f(i);
+  };
   std::vector<std::thread> th;
-  for (size_t t = 0; t < nt; ++t)
-    th.emplace_back([&, t] {
-      for (size_t i = t; i < count; i += nt) f(i);
-    });
+  try {
+    for (size_t t = 1; t < nt; ++t) th.emplace_back(work);
+  } catch (const std::system_error&) {  // fewer threads
+  }
+  work();
   for (auto& x : th) x.join();
 }
 
@@ -398,10 +408,15 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
   DeviceGuard g(p->device);
   const int d = p->d;
   const uint64_t Q = p->Q;
-  // Device image: [jobs | queries | rounds | elements | proofs], then scratch
-  // and flags.  Every job owns Q query slots and fixed element and proof
-  // ranges, so one pass over the jobs fills it; slots a job does not use
-  // (queries decided on the host) are marked inactive.
+  // Device image: [jobs | queries | rounds | elements | staged proofs], then
+  // scratch and flags.  Every job owns Q query slots and a fixed element range,
+  // so one pass over the jobs fills it; slots a job does not use (queries decided
+  // on the host) are marked inactive.  A device that shares the host's page
+  // tables reads the proofs where the caller has them (8-byte aligned; every
+  // field of a proof then is): each byte crosses once, as the paths are hashed,
+  // instead of being copied to pinned memory and from there to the device
+  // (64 proofs of 2^14, 83 MB, GB300: 3.5 -> 2.9 ms a batch, 7.2 -> 3.5 ms the
+  // first one of a pcs, which no longer pins 83 MB).
   const uint64_t nq = count * Q;
   if (nq > 0xffffffffull / (uint64_t)(d + 2)) return fail(BF_ERR_ARG, "too many queries in one batch");
   std::vector<VJob> v(count);
@@ -416,6 +431,8 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
   const uint64_t header = align16(cur);  // what the kernels read besides the proofs
   cur = header;
   for (size_t j = 0; j < count; ++j) {
+    v[j].staged = !p->reads_host || (reinterpret_cast<uintptr_t>(jobs[j].proof) & 7) != 0;
+    if (!v[j].staged) continue;
     v[j].proof = cur;
     cur = align16(cur + jobs[j].proof_len);
   }
@@ -429,6 +446,7 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
   }
   uint8_t* h = p->verify_pin.b();
   uint8_t* dv = reinterpret_cast<uint8_t*>(p->verify_dev.p);
+  const uint64_t dev = reinterpret_cast<uint64_t>(dv);  // the records hold device addresses
   cudaStream_t st = p->stream;
   std::vector<cudaError_t> copy_err(count, cudaSuccess);
   parallel_jobs(count, [&](size_t j) {
@@ -438,19 +456,21 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
     if (Q == 0) return;
     const Layout& lay = x.lay;
     const size_t active = x.status < 0 ? x.nq_dev : 0;
+    const uint64_t proof = x.staged ? dev + x.proof : reinterpret_cast<uint64_t>(jb.proof);
     bf::VerifyJob rec{};
-    rec.root = x.elems;
-    rec.challenges = x.elems + 32;
-    rec.scalars = x.elems + 32 + 16 * (uint64_t)d;
-    rec.pi_comms = x.proof + (active ? lay.pi_off : 0);
-    rec.final_poly = x.proof + (active ? lay.final_off : 0);
+    rec.root = dev + x.elems;
+    rec.challenges = dev + x.elems + 32;
+    rec.scalars = dev + x.elems + 32 + 16 * (uint64_t)d;
+    rec.pi_comms = proof + (active ? lay.pi_off : 0);
+    rec.final_poly = proof + (active ? lay.final_off : 0);
     rec.width = (uint32_t)jb.width;
     std::memcpy(h + off_jobs + sizeof(rec) * j, &rec, sizeof(rec));
     if (active) {
-      std::memcpy(h + x.elems, jb.root, 32);
-      for (int k = 0; k < d; ++k) bfh::store(h + x.elems + 32 + 16 * k, x.rounds_x[k]);
+      uint8_t* e = h + x.elems;
+      std::memcpy(e, jb.root, 32);
+      for (int k = 0; k < d; ++k) bfh::store(e + 32 + 16 * k, x.rounds_x[k]);
       if (jb.width > 1)
-        for (size_t w = 0; w < jb.width; ++w) bfh::store(h + rec.scalars + 16 * w, x.scalars[w]);
+        for (size_t w = 0; w < jb.width; ++w) bfh::store(e + 32 + 16 * (size_t)d + 16 * w, x.scalars[w]);
     }
     for (uint64_t q = 0; q < Q; ++q) {
       bf::VerifyQuery vq{};
@@ -459,17 +479,17 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
       if (q < active) {
         const Layout::Open& o = lay.open[q];
         vq.idx = x.idx[q];
-        vq.leaves = x.proof + o.leaves;
-        vq.path = x.proof + o.path;
+        vq.leaves = proof + o.leaves;
+        vq.path = proof + o.path;
         for (int k = 0; k < d; ++k) {
           const Layout::Ext& e = lay.ext[o.ext0 + k];
-          bf::VerifyRound vr{x.proof + e.sib, x.proof + e.path};
+          bf::VerifyRound vr{proof + e.sib, proof + e.path};
           std::memcpy(h + off_rounds + sizeof(vr) * (gq * d + k), &vr, sizeof(vr));
         }
       }
       std::memcpy(h + off_queries + sizeof(vq) * gq, &vq, sizeof(vq));
     }
-    if (active && jb.proof_len) {  // stage the proof and start its copy while other jobs are prepared
+    if (active && x.staged && jb.proof_len) {  // start the proof's copy while other jobs are prepared
       std::memcpy(h + x.proof, jb.proof, jb.proof_len);
       copy_err[j] = cudaSetDevice(p->device);  // worker threads start on device 0
       if (copy_err[j] == cudaSuccess)
@@ -480,7 +500,6 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
   if (nq > 0) {
     CU(cudaMemcpyAsync(dv, h, header, cudaMemcpyHostToDevice, st));
     bf::VerifyParams vp{};
-    vp.blob = dv;
     vp.jobs = reinterpret_cast<const bf::VerifyJob*>(dv + off_jobs);
     vp.queries = reinterpret_cast<const bf::VerifyQuery*>(dv + off_queries);
     vp.rounds = reinterpret_cast<const bf::VerifyRound*>(dv + off_rounds);

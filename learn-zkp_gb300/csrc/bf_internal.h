@@ -222,8 +222,9 @@ struct TailParams {
 cudaError_t launch_open_tail(const TailParams& p, cudaStream_t st);
 
 // ---- Basefold::verify of many proofs (basefold.rs:284-320) on the device.
-// Offsets are byte offsets into `blob`, multiples of 8.  All proofs share one
-// pcs (num_vars d, blowup 2^log2_c) and are checked query by query.
+// Fields are addresses the device can read, multiples of 8 (device memory, or the
+// caller's host memory where the device shares the host's page tables).  All
+// proofs share one pcs (num_vars d, blowup 2^log2_c) and are checked query by query.
 struct VerifyJob {
   uint64_t root;        // 32-byte commitment
   uint64_t pi_comms;    // the proof's d folded-codeword roots, 32 bytes apart
@@ -246,7 +247,6 @@ struct VerifyRound {
   uint64_t path;     // its log2 n_i sibling digests
 };
 struct VerifyParams {
-  const uint8_t* blob;
   const VerifyJob* jobs;
   const VerifyQuery* queries;  // nq
   const VerifyRound* rounds;   // nq * d, query-major

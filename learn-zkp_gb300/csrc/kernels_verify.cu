@@ -31,21 +31,28 @@ namespace bf {
 
 namespace {
 
-__device__ __forceinline__ uint4 load_elem8(const uint8_t* blob, uint64_t off) {
-  const uint2* p = reinterpret_cast<const uint2*>(blob + off);
+__device__ __forceinline__ uint4 load_elem8(uint64_t at) {
+  const uint2* p = reinterpret_cast<const uint2*>(at);
   const uint2 a = p[0], b = p[1];
   return make_uint4(a.x, a.y, b.x, b.y);
 }
 
-// A digest stored as bytes, in the interleaved lane form the tree hashes use.
-__device__ __forceinline__ Digest load_digest_bytes(const uint8_t* blob, uint64_t off) {
-  const uint2* p = reinterpret_cast<const uint2*>(blob + off);
-  Digest d;
-  const uint2 l0 = p[0], l1 = p[1], l2 = p[2], l3 = p[3];
-  d.lo = make_uint4(l0.x, l0.y, l1.x, l1.y);
-  d.hi = make_uint4(l2.x, l2.y, l3.x, l3.y);
-  return digest_interleaved(d);
+// A digest stored as bytes: its four lanes as they are, and interleaved as the
+// tree hashes use them.
+struct RawDigest {
+  uint2 l[4];
+  __device__ __forceinline__ Digest interleaved() const {
+    Digest d;
+    d.lo = make_uint4(l[0].x, l[0].y, l[1].x, l[1].y);
+    d.hi = make_uint4(l[2].x, l[2].y, l[3].x, l[3].y);
+    return digest_interleaved(d);
+  }
+};
+__device__ __forceinline__ RawDigest load_digest_raw(uint64_t at) {
+  const uint2* p = reinterpret_cast<const uint2*>(at);
+  return RawDigest{{p[0], p[1], p[2], p[3]}};
 }
+__device__ __forceinline__ Digest load_digest_bytes(uint64_t at) { return load_digest_raw(at).interleaved(); }
 
 __device__ __forceinline__ bool digest_eq(const Digest& a, const Digest& b) {
   return a.lo.x == b.lo.x && a.lo.y == b.lo.y && a.lo.z == b.lo.z && a.lo.w == b.lo.w && a.hi.x == b.hi.x &&
@@ -57,11 +64,11 @@ __device__ __forceinline__ bool elem_eq(uint4 a, uint4 b) { return a.x == b.x &&
 // Leaf of a row of `width` > 1 elements: keccak256 of its 16*width bytes,
 // any number of 136-byte (17-lane) blocks; lanes are indexed statically so
 // the state stays in registers.
-__device__ __forceinline__ Digest hash_row(const uint8_t* blob, uint64_t off, uint32_t width) {
+__device__ __forceinline__ Digest hash_row(uint64_t at, uint32_t width) {
   uint2 s[25];
 #pragma unroll
   for (int k = 0; k < 25; ++k) s[k] = make_uint2(0, 0);
-  const uint2* row = reinterpret_cast<const uint2*>(blob + off);
+  const uint2* row = reinterpret_cast<const uint2*>(at);
   const uint64_t lanes = 2ull * width;
   for (uint64_t k = 0;; k += 17) {
     const uint64_t left = lanes - k;  // message lanes from this block on
@@ -89,14 +96,13 @@ __global__ void __launch_bounds__(128) verify_fold_kernel(VerifyParams P) {
     return;
   }
   const VerifyJob J = P.jobs[Q.job];
-  const uint8_t* blob = P.blob;
   uint4 folded;
   if (J.width == 1) {
-    folded = load_elem8(blob, Q.leaves);  // scalars = [ONE] (basefold.rs:253-254)
+    folded = load_elem8(Q.leaves);  // scalars = [ONE] (basefold.rs:253-254)
   } else {
     folded = make_uint4(0, 0, 0, 0);
     for (uint32_t w = 0; w < J.width; ++w)
-      folded = gf_add(folded, gf_mul(load_elem8(blob, J.scalars + 16ull * w), load_elem8(blob, Q.leaves + 16ull * w)));
+      folded = gf_add(folded, gf_mul(load_elem8(J.scalars + 16ull * w), load_elem8(Q.leaves + 16ull * w)));
   }
   const int d = P.d;
   for (int k = 0; k < d; ++k) {
@@ -105,7 +111,7 @@ __global__ void __launch_bounds__(128) verify_fold_kernel(VerifyParams P) {
     const uint64_t ii = Q.idx & ((1ull << bits) - 1);
     const bool sib_left = ((Q.idx >> bits) & 1) != 0;  // the sibling is values[0]
     const VerifyRound R = P.rounds[(size_t)q * d + k];
-    const uint4 s = load_elem8(blob, R.sibling);
+    const uint4 s = load_elem8(R.sibling);
     uint4 v0 = sib_left ? s : folded, v1 = sib_left ? folded : s;
     P.pairs[2 * ((size_t)q * d + k)] = v0;
     P.pairs[2 * ((size_t)q * d + k) + 1] = v1;
@@ -114,9 +120,9 @@ __global__ void __launch_bounds__(128) verify_fold_kernel(VerifyParams P) {
     const uint4 t = gf_add(P.tw->lo[k][K & ((1u << kTwLoBits) - 1)], P.tw->hi[k][K >> kTwLoBits]);
     v1 = gf_add(v1, v0);
     v0 = gf_add(v0, gf_mul(v1, t));
-    folded = gf_add(v0, gf_mul(gf_add(v1, v0), load_elem8(blob, J.challenges + 16ull * k)));
+    folded = gf_add(v0, gf_mul(gf_add(v1, v0), load_elem8(J.challenges + 16ull * k)));
   }
-  P.final_bad[q] = elem_eq(folded, load_elem8(blob, J.final_poly)) ? 0 : 1;
+  P.final_bad[q] = elem_eq(folded, load_elem8(J.final_poly)) ? 0 : 1;
 }
 
 __global__ void __launch_bounds__(128) verify_path_kernel(VerifyParams P) {
@@ -130,7 +136,6 @@ __global__ void __launch_bounds__(128) verify_path_kernel(VerifyParams P) {
     return;
   }
   const VerifyJob J = P.jobs[Q.job];
-  const uint8_t* blob = P.blob;
   Digest cur, root;
   int log_h;
   uint64_t index, path;
@@ -138,19 +143,23 @@ __global__ void __launch_bounds__(128) verify_path_kernel(VerifyParams P) {
     log_h = P.d + P.log2_c;
     index = Q.idx;
     path = Q.path;
-    root = load_digest_bytes(blob, J.root);
-    cur = J.width == 1 ? hash_elem(load_elem8(blob, Q.leaves)) : hash_row(blob, Q.leaves, J.width);
+    root = load_digest_bytes(J.root);
+    cur = J.width == 1 ? hash_elem(load_elem8(Q.leaves)) : hash_row(Q.leaves, J.width);
   } else {  // folded codeword of round k: leaf = keccak256(values[0] || values[1])
     const int k = (int)level - 1;
     log_h = P.log2_c + P.d - 1 - k;
     index = Q.idx & ((1ull << log_h) - 1);
     path = P.rounds[(size_t)q * P.d + k].path;
-    root = load_digest_bytes(blob, J.pi_comms + 32ull * k);
+    root = load_digest_bytes(J.pi_comms + 32ull * k);
     const size_t pr = 2 * ((size_t)q * P.d + k);
     cur = hash_pair(P.pairs[pr], P.pairs[pr + 1]);
   }
+  // The next sibling is loaded while this one is hashed: it may come from host
+  // memory, some two microseconds away.
+  RawDigest next = log_h > 0 ? load_digest_raw(path) : RawDigest{};
   for (int b = 0; b < log_h; ++b) {
-    const Digest sib = load_digest_bytes(blob, path + 32ull * b);
+    const Digest sib = next.interleaved();
+    if (b + 1 < log_h) next = load_digest_raw(path + 32ull * (b + 1));
     // the side is picked by selects, not a branch: threads of a warp differ in it
     const bool right = ((index >> b) & 1) != 0;
     Digest l, r;

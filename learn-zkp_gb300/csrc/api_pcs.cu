@@ -357,6 +357,15 @@ int eval_enqueue(bf_pcs* p, const bf_commitment* cm, const uint8_t* point, uint4
     CU(cudaMemcpyAsync(value_pin, data, 16 * w, cudaMemcpyDeviceToHost, st));
     return BF_OK;
   }
+  if (w == 1 && d >= bf::kEvalSplitMin && d <= bf::kEvalSplitMax) {
+    // one sum against the eq table in two factors, in the scratch's tail
+    uint4* value = scratch + ((size_t)1 << (d - 1)) - 1;
+    ProfScope ps(p->prof, st, P_FIX);
+    CU(bf::launch_eval_split(data, d, point_dev ? nullptr : point, point_dev, scratch, value, st));
+    if (value_dev) *value_dev = value;
+    CU(cudaMemcpyAsync(value_pin, value, 16, cudaMemcpyDeviceToHost, st));
+    return BF_OK;
+  }
   auto coord = [&](int k) {
     uint4 r{};
     if (!point_dev) std::memcpy(&r, point + 16 * k, 16);

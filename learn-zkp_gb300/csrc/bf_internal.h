@@ -66,6 +66,26 @@ cudaError_t launch_tree(uint4* leaves, size_t n, cudaStream_t st, uint4* root_ou
 cudaError_t launch_fill_random(uint4* out, size_t n, uint64_t seed, cudaStream_t st);
 
 cudaError_t launch_eq_table(const uint4* r, int nvars, uint4* out, uint4* tmp_lo, uint4* tmp_hi, cudaStream_t st);
+// Up to two eq tables of at most 16 variables each in one launch: job j's table
+// is over coordinates first .. first + nv - 1 of the point, which is rp in device
+// memory or, when rp is null, r.  `zero`, when given, receives a zero element.
+struct EqTables {
+  struct Job {
+    uint4* out;  // null: no table
+    int first, nv;
+    unsigned blocks;  // set by the launcher
+  } job[2];
+  uint4 r[32];
+  const uint4* rp;
+  uint4* zero;
+};
+cudaError_t launch_eq_tables(EqTables p, cudaStream_t st);
+// The value of the multilinear extension of 2^n elements (kEvalSplitMin <= n <=
+// kEvalSplitMax) at the point r (16 n host bytes) or rp (device memory), into
+// *value (device).  `scratch` holds 2^((n+1)/2) + 2^(n/2) elements.
+constexpr int kEvalSplitMin = 5, kEvalSplitMax = 30;
+cudaError_t launch_eval_split(const uint4* data, int n, const uint8_t* r, const uint4* rp, uint4* scratch, uint4* value,
+                              cudaStream_t st);
 cudaError_t launch_dot_xor(const uint4* x, const uint4* y, size_t n, uint32_t* acc, cudaStream_t st);
 // The fold and fix challenge is `r`, or *xp when xp is not null (a challenge
 // sampled on the device).

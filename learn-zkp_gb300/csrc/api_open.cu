@@ -185,6 +185,28 @@ int session_alloc(bf_open_session* s) {
   return BF_OK;
 }
 
+// Round i >= 1 on the device: fold (binary_reed_solomon.rs:88-96, the stage d-1-i
+// twiddles) with the next round's leaves, and fix_last_var
+// (multilinear.rs:183-198) with the next round's reduction.
+bf::FoldFixParams fold_round(const bf_open_session* s, int i) {
+  const bf_pcs* p = s->p;
+  const int d = s->d;
+  bf::FoldFixParams fp{};
+  fp.pi = (i == d - 1) ? s->first_pi() : s->pi_fold_out(i + 1);
+  fp.pi_out = s->pi_fold_out(i);
+  fp.leaves = s->pi_tree(i - 1);
+  fp.n_leaves = p->n_i(i) / 2;
+  fp.tlo = p->tw_host.lo[d - 1 - i];
+  fp.thi = p->tw_host.hi[d - 1 - i];
+  fp.poly_in = (i == d - 1) ? s->first_poly() : s->w_poly;
+  fp.poly_out = s->w_poly;
+  fp.half = (size_t)1 << i;
+  fp.heq = s->w_heq;
+  fp.next_half = (size_t)1 << (i - 1);
+  fp.acc = reinterpret_cast<uint32_t*>(s->stage(i - 1) + 32);
+  return fp;
+}
+
 // Reads the result of the enqueued work and computes the host-side message of
 // the current round: EvalImprProver::compute_round_poly + decompress
 // (eval_impr.rs:116-127,187-197) lifted by EvalProver (eval.rs:89-106).
@@ -294,19 +316,7 @@ int open_resident_enqueue_device(bf_open_session* s, const uint4* root_dev, cons
       // fold (binary_reed_solomon.rs:88-96) + next leaves, and fix_last_var
       // (multilinear.rs:183-198) + next reduction, in one launch
       ProfScope ps(p->prof, st, P_FOLD);
-      bf::FoldFixParams fp{};
-      fp.pi = (i == d - 1) ? s->first_pi() : s->pi_fold_out(i + 1);
-      fp.pi_out = s->pi_fold_out(i);
-      fp.leaves = s->pi_tree(i - 1);
-      fp.n_leaves = p->n_i(i) / 2;
-      fp.tlo = p->tw_host.lo[d - 1 - i];
-      fp.thi = p->tw_host.hi[d - 1 - i];
-      fp.poly_in = (i == d - 1) ? s->first_poly() : s->w_poly;
-      fp.poly_out = s->w_poly;
-      fp.half = (size_t)1 << i;
-      fp.heq = s->w_heq;
-      fp.next_half = (size_t)1 << (i - 1);
-      fp.acc = reinterpret_cast<uint32_t*>(s->stage(i - 1) + 32);
+      bf::FoldFixParams fp = fold_round(s, i);
       fp.xp = xp;
       CU(bf::launch_fold_fix(fp, uint4{}, st));
     }
@@ -671,25 +681,17 @@ int bf_open_challenge(bf_open_session* s, const uint8_t r_i[16]) {
   s->delta_prod = bfh::mul(s->delta_prod, ONE ^ s->r[i] ^ x);
   const uint4 xr = to_uint4(x);
   cudaStream_t st = s->st;
-  // fold (binary_reed_solomon.rs:88-96) with the stage d-1-i twiddles,
-  // fused with the leaves of the next round's tree
-  const size_t ni = p->n_i(i);
-  const uint4* pi_in = (i == d - 1) ? s->first_pi() : s->pi_fold_out(i + 1);
-  const uint4* tlo = p->tw_host.lo[d - 1 - i];
-  const uint4* thi = p->tw_host.hi[d - 1 - i];
-  {
+  if (i > 0) {
     ProfScope ps(p->prof, st, P_FOLD);
-    if (i > 0)
-      CU(bf::launch_fold_leaves(pi_in, s->pi_fold_out(i), s->pi_tree(i - 1), ni / 2, tlo, thi, xr, st));
-    else
-      CU(bf::launch_fold(pi_in, s->pi_fold_out(i), ni, tlo, thi, xr, st));
-  }
-  // fix_last_var (multilinear.rs:183-198) + next round's reduction
-  const uint4* poly_in = (i == d - 1) ? s->first_poly() : s->w_poly;
-  {
+    CU(bf::launch_fold_fix(fold_round(s, i), xr, st));
+  } else {  // the last fold and fix: no next round
+    {
+      ProfScope ps(p->prof, st, P_FOLD);
+      CU(bf::launch_fold((i == d - 1) ? s->first_pi() : s->pi_fold_out(1), s->pi_fold_out(0), p->n_i(0),
+                         p->tw_host.lo[d - 1], p->tw_host.hi[d - 1], xr, st));
+    }
     ProfScope ps(p->prof, st, P_FIX);
-    CU(bf::launch_fix(poly_in, s->w_poly, (size_t)1 << i, xr, s->w_heq, i > 0 ? ((size_t)1 << (i - 1)) : 0,
-                      i > 0 ? reinterpret_cast<uint32_t*>(s->stage(i - 1) + 32) : nullptr, st));
+    CU(bf::launch_fix((i == d - 1) ? s->first_poly() : s->w_poly, s->w_poly, 1, xr, s->w_heq, 0, nullptr, st));
   }
   uint8_t* pin = s->pin->b();
   if (i > 0) {

@@ -91,14 +91,12 @@ cudaError_t launch_dot_xor(const uint4* x, const uint4* y, size_t n, uint32_t* a
 // sampled on the device).
 cudaError_t launch_fold(const uint4* pi, uint4* out, size_t n_out, const uint4* tw_lo, const uint4* tw_hi, uint4 r,
                         cudaStream_t st, const uint4* xp = nullptr);
-cudaError_t launch_fold_leaves(const uint4* pi, uint4* out, uint4* leaves, size_t n_leaves, const uint4* tw_lo,
-                               const uint4* tw_hi, uint4 r, cudaStream_t st, const uint4* xp = nullptr);
 cudaError_t launch_fix(const uint4* in, uint4* out, size_t half, uint4 r, const uint4* heq, size_t next_half,
                        uint32_t* acc, cudaStream_t st, const uint4* xp = nullptr);
 cudaError_t launch_fix_column(const uint4* in, size_t width, size_t col, uint4* out, size_t half, uint4 r,
                               cudaStream_t st, const uint4* xp = nullptr);
 // A round of open (i >= 1) in one launch: the fold of `pi` into `pi_out`
-// with the next round's leaves (launch_fold_leaves) and the fix of
+// with the next round's leaves and the fix of
 // `poly_in` into `poly_out` with the next round's reduction into `acc`
 // (launch_fix).  The challenge is *xp when xp is set, else r.
 struct FoldFixParams {

@@ -1207,38 +1207,6 @@ __global__ void __launch_bounds__(256) fold_kernel(const uint4* __restrict__ pi,
   }
 }
 
-// Fold fused with the next round's leaf hashing: thread s folds the four
-// entries pi[4s..4s+3] into out[2s], out[2s+1] and hashes that pair, which is
-// leaf s of the next round's folded-codeword tree.
-__global__ void __launch_bounds__(128) fold_leaves_kernel(const uint4* __restrict__ pi, uint4* __restrict__ out,
-                                                          uint4* __restrict__ leaves, size_t n_leaves,
-                                                          const uint4* __restrict__ tlo,
-                                                          const uint4* __restrict__ thi, uint4 r,
-                                                          const uint4* xp) {
-  if (xp) r = *xp;
-  for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_leaves; s += (size_t)gridDim.x * blockDim.x) {
-    uint4 f[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const size_t t = 2 * s + k;
-      const uint4 tw = gf_add(tlo[t & 4095], thi[t >> 12]);
-      uint4 lo = pi[2 * t], hi = pi[2 * t + 1];
-      hi = gf_add(hi, lo);
-      lo = gf_add(lo, gf_mul(hi, tw));
-      f[k] = gf_add(lo, gf_mul(gf_add(hi, lo), r));
-      out[t] = f[k];
-    }
-    store_digest(leaves, s, hash_pair(f[0], f[1]));
-  }
-}
-
-cudaError_t launch_fold_leaves(const uint4* pi, uint4* out, uint4* leaves, size_t n_leaves, const uint4* tw_lo,
-                               const uint4* tw_hi, uint4 r, cudaStream_t st, const uint4* xp) {
-  fold_leaves_kernel<<<grid_short(n_leaves, 128), 128, 0, st>>>(pi, out, leaves, n_leaves, tw_lo, tw_hi, r, xp);
-  COUNT_LAUNCH();
-  return cudaGetLastError();
-}
-
 cudaError_t launch_fold(const uint4* pi, uint4* out, size_t n_out, const uint4* tw_lo, const uint4* tw_hi, uint4 r,
                         cudaStream_t st, const uint4* xp) {
   fold_kernel<<<grid_for(n_out, 256), 256, 0, st>>>(pi, out, n_out, tw_lo, tw_hi, r, xp);
@@ -1267,9 +1235,10 @@ __global__ void __launch_bounds__(256, 3) fix_kernel(const uint4* in, uint4* out
   }
 }
 
-// One round of open in one launch: fold_blocks blocks fold the codeword and
-// hash the next round's leaves (as fold_leaves_kernel), fix_blocks blocks fix
-// the sumcheck polynomial and reduce for the next round (as fix_kernel).
+// One round of open in one launch: fold_blocks blocks fold the codeword (thread
+// s folds the four entries pi[4s..4s+3] into out[2s], out[2s+1]) and hash the next
+// round's leaves (that pair), fix_blocks blocks fix the sumcheck polynomial and
+// reduce for the next round (as fix_kernel).
 // Both read the round's challenge.  The fix blocks are spread through the
 // grid (block S q + S - 1 is fix block q, S = grid / fix_blocks), so their
 // multiplier-bound work runs beside the ALU-bound fold blocks instead of

@@ -313,17 +313,17 @@ __device__ __forceinline__ void atomic_xor4(uint32_t* acc, uint4 v) {
 constexpr int kGfBasis = 132;  // elements a basis takes in shared memory (128, and slack that is read but not used)
 template <int G>
 struct GfTab {
-  static_assert(G == 6 || G == 7, "6 groups: 6 6 5 5 5 5 bits; 7 groups: 6 5 5 4 4 4 4 bits");
+  static_assert(G >= 6 && G <= 8, "6 groups: 6 6 5 5 5 5 bits; 7 groups: 6 5 5 4 4 4 4 bits; 8 groups of 4 bits");
   static __host__ __device__ constexpr int bits(int g) {
-    return G == 6 ? (g < 2 ? 6 : 5) : (g == 0 ? 6 : g < 3 ? 5 : 4);
+    return G == 8 ? 4 : G == 6 ? (g < 2 ? 6 : 5) : (g == 0 ? 6 : g < 3 ? 5 : 4);
   }
   static __host__ __device__ constexpr int bit(int g) {  // first bit of group g
-    return G == 6 ? (g < 2 ? 6 * g : 12 + 5 * (g - 2)) : (g == 0 ? 0 : g < 3 ? 6 + 5 * (g - 1) : 16 + 4 * (g - 3));
+    return G == 8 ? 4 * g : G == 6 ? (g < 2 ? 6 * g : 12 + 5 * (g - 2)) : (g == 0 ? 0 : g < 3 ? 6 + 5 * (g - 1) : 16 + 4 * (g - 3));
   }
   static __host__ __device__ constexpr int entry(int g) {  // its first entry within the word's
-    return G == 6 ? (g < 2 ? 64 * g : 128 + 32 * (g - 2)) : (g == 0 ? 0 : g < 3 ? 64 + 32 * (g - 1) : 128 + 16 * (g - 3));
+    return G == 8 ? 16 * g : G == 6 ? (g < 2 ? 64 * g : 128 + 32 * (g - 2)) : (g == 0 ? 0 : g < 3 ? 64 + 32 * (g - 1) : 128 + 16 * (g - 3));
   }
-  static constexpr int kPerWord = G == 6 ? 256 : 192;
+  static constexpr int kPerWord = G == 8 ? 128 : G == 6 ? 256 : 192;
   static constexpr int kEntries = 4 * kPerWord;
   static constexpr size_t kBytes = (size_t)kEntries * 128;  // eight copies of 16 bytes
 
@@ -344,7 +344,7 @@ struct GfTab {
       const uint4* b = basis + 32 * w + bit(g);
       uint4 s = make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int i = 0; i < 6; ++i) {
+      for (int i = 0; i < bits(0); ++i) {
         const uint32_t m = 0u - ((v >> i) & 1u);
         const uint4 t = b[i];
         s = make_uint4(s.x ^ (t.x & m), s.y ^ (t.y & m), s.z ^ (t.z & m), s.w ^ (t.w & m));

@@ -501,7 +501,7 @@ struct QuadTwiddles {
 constexpr int kQuadTabThreads = 512;
 using QuadTabT = GfTab<6>;
 using QuadTabU = GfTab<7>;
-constexpr size_t kQuadTabShared = QuadTabT::kBytes + QuadTabU::kBytes + kGfBasis * sizeof(uint4);
+constexpr size_t kQuadTabShared = QuadTabT::kBytes + QuadTabU::kBytes + kGfBasis * sizeof(uint4) + 64;
 
 __global__ void __launch_bounds__(kQuadTabThreads, 1) ntt_quad_tab_kernel(const uint4* __restrict__ m, uint4* cw,
                                                                          QuadPass p,
@@ -510,6 +510,7 @@ __global__ void __launch_bounds__(kQuadTabThreads, 1) ntt_quad_tab_kernel(const 
   uint4* tab_t = sm;
   uint4* tab_u = sm + QuadTabT::kBytes / sizeof(uint4);
   uint4* basis = tab_u + QuadTabU::kBytes / sizeof(uint4);
+  uint4* next_w = basis + kGfBasis;  // t, u0, u1 of the group to come and whether t and u0 are not zero
   const uint4* my_t = tab_t + (threadIdx.x & 7u);
   const uint4* my_u = tab_u + (threadIdx.x & 7u);
   const uint4* in = p.first ? m : cw;
@@ -517,12 +518,19 @@ __global__ void __launch_bounds__(kQuadTabThreads, 1) ntt_quad_tab_kernel(const 
   const uint64_t per = p.total / gridDim.x, rem = p.total % gridDim.x;
   uint64_t pos = per * blockIdx.x + (blockIdx.x < rem ? blockIdx.x : rem);
   const uint64_t end = pos + per + (blockIdx.x < rem ? 1 : 0);
+  auto load_w = [&](uint64_t g) {
+    const QuadTwiddles w(p, g, tw);
+    next_w[0] = w.t;
+    next_w[1] = w.u0;
+    next_w[2] = w.u1;
+    next_w[3] = make_uint4(w.has_t, w.has_u0, 0, 0);
+  };
+  if (threadIdx.x == 0 && pos < end) load_w(pos / p.run_cols);
   while (pos < end) {
     const uint64_t g = pos / p.run_cols, g0 = g * p.run_cols;
     const uint64_t q_end = (end < g0 + p.run_cols ? end : g0 + p.run_cols) - g0;
     uint64_t q = pos - g0 + threadIdx.x;
     pos = g0 + q_end;
-    const QuadTwiddles w(p, g, tw);
     uint4 x[4];
     uint64_t dst = 0;
     if (q < q_end) {  // in flight while the tables are built
@@ -532,18 +540,19 @@ __global__ void __launch_bounds__(kQuadTabThreads, 1) ntt_quad_tab_kernel(const 
       for (int a = 0; a < 4; ++a) x[a] = in[ad.src[a]];
     }
     __syncthreads();  // the last group's lookups are done
-    if (w.has_t) {
-      if (threadIdx.x < 128) gf_basis(basis, w.t, threadIdx.x);
-      __syncthreads();
-      QuadTabT::build(tab_t, basis);
-      __syncthreads();
+    const uint4 u1 = next_w[2];
+    const bool has_t = next_w[3].x, has_u0 = next_w[3].y;
+    // both bases at once: t's in the space of u0's table, which is built last
+    if (threadIdx.x < 256) {
+      const bool u = threadIdx.x >= 128;
+      gf_basis(u ? basis : tab_u, next_w[u], threadIdx.x & 127u);
     }
-    if (w.has_u0) {
-      if (threadIdx.x < 128) gf_basis(basis, w.u0, threadIdx.x);
-      __syncthreads();
-      QuadTabU::build(tab_u, basis);
-      __syncthreads();
-    }
+    __syncthreads();
+    if (has_t) QuadTabT::build(tab_t, tab_u);
+    __syncthreads();
+    if (has_u0) QuadTabU::build(tab_u, basis);
+    __syncthreads();
+    if (threadIdx.x == 0 && pos < end) load_w(g + 1);
     while (q < q_end) {
       const uint64_t qn = q + kQuadTabThreads;
       uint4 nx[4];
@@ -554,15 +563,15 @@ __global__ void __launch_bounds__(kQuadTabThreads, 1) ntt_quad_tab_kernel(const 
 #pragma unroll
         for (int a = 0; a < 4; ++a) nx[a] = in[ad.src[a]];
       }
-      if (w.has_t) {
+      if (has_t) {
         x[0] = gf_add(x[0], QuadTabT::mul(my_t, x[2]));
         x[1] = gf_add(x[1], QuadTabT::mul(my_t, x[3]));
       }
       x[2] = gf_add(x[2], x[0]);
       x[3] = gf_add(x[3], x[1]);
-      if (w.has_u0) x[0] = gf_add(x[0], QuadTabU::mul(my_u, x[1]));
+      if (has_u0) x[0] = gf_add(x[0], QuadTabU::mul(my_u, x[1]));
       x[1] = gf_add(x[1], x[0]);
-      x[2] = gf_add(x[2], gf_mul(x[3], w.u1));
+      x[2] = gf_add(x[2], gf_mul(x[3], u1));
       x[3] = gf_add(x[3], x[2]);
 #pragma unroll
       for (int a = 0; a < 4; ++a) cw[dst + a * p.cols] = x[a];
@@ -571,6 +580,69 @@ __global__ void __launch_bounds__(kQuadTabThreads, 1) ntt_quad_tab_kernel(const 
       q = qn;
       dst = nd;
     }
+  }
+}
+
+// The same two layers for groups of a few hundred columns, whose table builds
+// ntt_quad_tab_kernel cannot hide: one block per group and three per SM, so that
+// one block's build runs beside the others' products.  The two products by t come
+// from a small table (64 KB, 4-bit groups), the two others from the multiplier with
+// their factors split beforehand (gf_prepare; 80 registers a thread, 670 us below
+// against 809 with the factors in registers and spills, 762 at two blocks).  Bound
+// by the ALU pipe.  Measured on GB300, a pass of 2^25 elements with 256 columns
+// per group: 670 us, 800 multiplied; with 1024: 460, 525 with the large tables.
+constexpr int kQuadMixThreads = 256, kQuadMixBlocks = 3;
+using QuadTabM = GfTab<8>;
+constexpr size_t kQuadMixShared = QuadTabM::kBytes + kGfBasis * sizeof(uint4) + 2 * sizeof(GfPrep);
+
+__global__ void __launch_bounds__(kQuadMixThreads, kQuadMixBlocks)
+    ntt_quad_mix_kernel(uint4* cw, QuadPass p, const TwiddleView* __restrict__ tw) {
+  extern __shared__ uint4 sm[];
+  uint4* basis = sm + QuadTabM::kBytes / sizeof(uint4);
+  uint4* prep = basis + kGfBasis;  // u0, u1
+  const uint4* my_t = sm + (threadIdx.x & 7u);
+  const uint64_t g = blockIdx.x;
+  uint4* io = cw + (g << 2) * p.cols;
+  uint64_t q = threadIdx.x;
+  uint4 x[4];
+  auto load = [&] {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) x[a] = io[a * p.cols + q];
+  };
+  if (q < p.cols) load();
+  bool has_t, has_u0;
+  {
+    const QuadTwiddles w(p, g, tw);
+    has_t = w.has_t;
+    has_u0 = w.has_u0;
+    if (threadIdx.x < 128) gf_basis(basis, w.t, threadIdx.x);
+    if ((threadIdx.x & 127u) == 127u) gf_prepare(threadIdx.x < 128 ? w.u0 : w.u1, reinterpret_cast<uint32_t*>(prep + (threadIdx.x < 128 ? 0 : 9)));
+  }
+  __syncthreads();
+  if (has_t) QuadTabM::build(sm, basis);
+  __syncthreads();
+  auto mul_u = [&](uint4 a, int i) {
+    uint64_t c[4] = {0, 0, 0, 0};
+    gf_clmul_acc(a, prep + 9 * i, c);
+    return gf_reduce256(c[0], c[1], c[2], c[3]);
+  };
+  while (q < p.cols) {
+    if (has_t) {
+      x[0] = gf_add(x[0], QuadTabM::mul(my_t, x[2]));
+      x[1] = gf_add(x[1], QuadTabM::mul(my_t, x[3]));
+    }
+    x[2] = gf_add(x[2], x[0]);
+    x[3] = gf_add(x[3], x[1]);
+    if (has_u0) x[0] = gf_add(x[0], mul_u(x[1], 0));
+    x[1] = gf_add(x[1], x[0]);
+    io[q] = x[0];
+    io[q + p.cols] = x[1];
+    x[2] = gf_add(x[2], mul_u(x[3], 1));
+    x[3] = gf_add(x[3], x[2]);
+    io[q + 2 * p.cols] = x[2];
+    io[q + 3 * p.cols] = x[3];
+    q += kQuadMixThreads;
+    if (q < p.cols) load();
   }
 }
 
@@ -623,14 +695,21 @@ bool tune_valid(const Tune& t) {
 }
 
 // Column passes with tables: elements of the codeword from which they pay, and
-// columns per group (a group's tables cost about 5 us with the pipeline's drain;
-// at 1024 columns a pass of 2^25 elements takes 653 us, 797 multiplied, 385 with
-// 2^14 columns or more).  Measured on GB300, encode without and with them:
-// width 1, blowup 2, 2^19 rows 592 and 657 us, 2^20 1189 and 1142, 2^24 19.41 and
-// 17.43 ms; 2^14 x 16 107 and 125 us, 2^15 x 16 207 and 197, 2^11 x 256 168 and
-// 150, 2^16 x 256 6.50 and 3.90 ms.
+// columns per group.  The large tables (ntt_quad_tab_kernel) cost about 2.5 us a
+// group with the pipeline's drain: a pass of 2^25 elements takes 385 us with 2^14
+// columns per group or more, 410 with 4096, 525 with 1024.  Measured on GB300,
+// encode without and with them: width 1, blowup 2, 2^19 rows 592 and 657 us, 2^20
+// 1189 and 1142, 2^24 19.41 and 17.43 ms; 2^14 x 16 107 and 125 us, 2^15 x 16 207
+// and 197, 2^11 x 256 168 and 150, 2^16 x 256 6.50 and 3.53 ms.
 constexpr size_t quad_tab_elems(size_t width) { return (size_t)1 << (width == 1 ? 21 : 20); }
 constexpr size_t kQuadTabCols = 1024;
+// Columns per group for the small table (ntt_quad_mix_kernel), given three blocks
+// per SM.  Measured on GB300, encodes with the passes of 1024 columns on the large
+// tables and on the small one: 2^16 x 256 3615 and 3532 us, 2^20 x 16 5217 and
+// 5132; those of 2368 or 3200 columns: 2^16 x 37 712 and 725, 2^17 x 100 3366 and
+// 3399.  Passes of 256 columns multiplied and on the small table: 2^16 x 256 3792
+// and 3658; of 148: 2^16 x 37 731 and 743.
+constexpr size_t kQuadMixCols = 256, kQuadMixEnd = 2048;
 // Without tables, for the layers left of a wide matrix: at least kQuadWide columns
 // and at most kQuadRest layers (more layers run faster in shared memory).
 constexpr size_t kQuadWide = 16;
@@ -748,7 +827,12 @@ cudaError_t launch_encode(const uint4* m, uint4* cw, int n, int log2_c, size_t w
     q.run_cols = q.cols >> piece_log;
     q.total = (((uint64_t)c << n) * width) >> ((one ? 1 : 2) + piece_log);
     const unsigned blocks = (unsigned)((q.total + 255) / 256);
-    if (tab)
+    const uint64_t groups = q.total / q.run_cols;  // of all columns after the first pass
+    const bool mix = !one && !q.first && q.cols >= kQuadMixCols && q.cols < kQuadMixEnd &&
+                     groups >= (uint64_t)kQuadMixBlocks * num_sms();
+    if (mix)
+      ntt_quad_mix_kernel<<<(unsigned)groups, kQuadMixThreads, kQuadMixShared, st>>>(cw, q, tw);
+    else if (tab)
       ntt_quad_tab_kernel<<<(unsigned)num_sms(), kQuadTabThreads, kQuadTabShared, st>>>(m, cw, q, tw);
     else if (one)
       ntt_quad_kernel<true><<<blocks, 256, 0, st>>>(cw, q, tw);
@@ -1816,6 +1900,7 @@ void init_kernel_attributes() {
   cudaFuncSetAttribute(prod_fix_tab_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdTabShared);
   cudaFuncSetAttribute(prod_fix_tab_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdTabShared);
   cudaFuncSetAttribute(ntt_quad_tab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQuadTabShared);
+  cudaFuncSetAttribute(ntt_quad_mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQuadMixShared);
   done.fetch_or(bit);
 }
 

@@ -1,5 +1,6 @@
 """The encode's column passes: pairs of layers with shared-memory tables of the
-twiddles, and the few layers left of a wide matrix without.  Widths that fill,
+twiddles (large for many columns per group, small for a few hundred), and the few
+layers left of a wide matrix without.  Widths that fill,
 straddle and miss the blocks, odd and even layer counts, every blowup, host
 input in slices, and inputs whose bit groups are all zero or all one.  Roots
 against the oracle (a root binds every codeword entry)."""
@@ -20,7 +21,7 @@ def _matrix(n, w, seed):
 
 
 @pytest.mark.parametrize("n,log2_c,w", [(9, 1, 1024), (10, 1, 513), (12, 1, 129), (13, 2, 33), (16, 1, 8), (18, 1, 2),
-                                        (17, 1, 5), (11, 1, 300), (16, 4, 3)])
+                                        (17, 1, 5), (11, 1, 300), (16, 4, 3), (12, 1, 256), (14, 1, 255)])
 def test_matrix_commits_match_the_oracle(built_lib, n, log2_c, w):
     bg = built_lib
     data = _matrix(n, w, 4000 + n + w)

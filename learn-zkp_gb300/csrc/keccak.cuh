@@ -569,59 +569,96 @@ __device__ __forceinline__ const uint4* tree_block(const WarpKeccak& wk, uint4* 
   return src;
 }
 
-// keccak256 of matrix rows of `words` 32-bit words, one lane per row, the
-// 32 rows [r0, r0 + 32) per warp.  The 136-byte rate is 34 words, so every
-// block of every row starts on a word: the warp stages the current block of
-// its rows in shared memory (`st`: 32 x kStagePitch words) with loads whose
-// 32 lanes read one 128-byte row run (8 in flight per lane), then each lane
-// absorbs its row.  word_at(row, i) returns word i of a row (rows < `rows`,
-// i < `words`); the 0x01 pad word follows the message and 0x80 ends the
-// last block.  The row is absorbed and permuted on plain lanes (interleaving
-// 17 message lanes per block would cost more than the interleaved rounds
-// save); only the four digest lanes are interleaved, the trees' form.
-constexpr int kRateWords = 34;
-constexpr int kStagePitch = 35;  // odd pitch: lane r reads word r * 35 + i without bank conflicts
-template <class WordAt>
-__device__ __forceinline__ Digest keccak_rows_warp(uint32_t* st, size_t r0, size_t rows, uint32_t words,
-                                                   const WordAt& word_at) {
+// keccak256 of matrix rows of `words` 32-bit words (`base`, row after row), one
+// lane per row, the 32 rows [r0, r0 + 32) per warp.  The 136-byte rate is 34
+// words, so every block of every row starts on a word: the warp copies a block of
+// its rows into shared memory (`st`: two stages of kStageWords words, 16-byte
+// aligned) while it permutes the block before, with asynchronous copies whose lanes
+// read whole row runs, 8 bytes each where rows are an even number of words; then each lane
+// absorbs its row, conv applied to every word.  The 0x01 pad word follows the
+// message and 0x80 ends the last block.  The row is absorbed and permuted on
+// plain lanes (interleaving 17 message lanes per block would cost more than the
+// interleaved rounds save); only the four digest lanes are interleaved, the
+// trees' form.  Bound by the ALU pipe: the permutations alone
+// take 85 to 95% of the time.  Measured on GB300 before, with loads through
+// registers, padding computed for every word and no copy ahead of its use: 2^20
+// rows of 256 words 2122 us and now 1901, 2^17 rows of 1024 words 1047 and 941,
+// 2^15 rows of 2048 words 684 and 541.
+constexpr int kRateWords = 34;  // a stage's row pitch too: lane r's 8-byte words at 34 r meet no bank twice
+constexpr int kStageWords = 32 * kRateWords;
+__device__ __forceinline__ void copy_async8(uint32_t* dst, const uint32_t* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async4(uint32_t* dst, const uint32_t* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+// The words [34 blk, 34 blk + 34) of the warp's rows, as far as they exist.
+__device__ __forceinline__ void stage_rows(uint32_t* st, const uint32_t* __restrict__ base, size_t r0, size_t rows,
+                                           uint32_t words, uint32_t blk) {
+  const uint32_t lane = threadIdx.x & 31u, c0 = blk * kRateWords;
+  const uint32_t n = words - c0 < (uint32_t)kRateWords ? words - c0 : (uint32_t)kRateWords;
+  const uint32_t in = rows - r0 < 32 ? (uint32_t)(rows - r0) : 32u;  // rows there are
+  const uint32_t* tile = base + r0 * words + c0;
+  if ((words & 1u) == 0) {  // 16 lanes a row, then the last 8 bytes with a lane per row
+    const uint32_t h = lane >> 4, c = 2 * (lane & 15u);
+    const uint32_t* src = tile + (size_t)h * words + c;
+    uint32_t* dst = st + h * kRateWords + c;
+    const uint32_t have = c < n && h < in ? (in - h + 1) / 2 : 0;  // this lane's rows
+    if (have == 16) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k, src += 2 * (size_t)words) copy_async8(dst + 2 * k * kRateWords, src);
+    } else {
+      for (uint32_t k = 0; k < have; ++k) copy_async8(dst + 2 * k * kRateWords, src + 2 * (size_t)k * words);
+    }
+    if (n > 32 && lane < in) copy_async8(st + lane * kRateWords + 32, tile + (size_t)lane * words + 32);
+  } else {  // a row per instruction, then the last two words with a lane per row
+    if (lane < n)
+      for (uint32_t k = 0; k < in; ++k) copy_async4(st + k * kRateWords + lane, tile + (size_t)k * words + lane);
+    for (uint32_t i = 32; i < n; ++i)
+      if (lane < in) copy_async4(st + lane * kRateWords + i, tile + (size_t)lane * words + i);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <class Conv>
+__device__ __forceinline__ Digest keccak_rows_warp(uint32_t* st, const uint32_t* __restrict__ base, size_t r0,
+                                                   size_t rows, uint32_t words, const Conv& conv) {
   const uint32_t lane = threadIdx.x & 31u;
   uint2 s[25];
 #pragma unroll
   for (int i = 0; i < 25; ++i) s[i] = make_uint2(0, 0);
-  const uint32_t nblk = words / kRateWords + 1;
-  for (uint32_t blk = 0; blk < nblk; ++blk) {
-    auto pad = [&](uint32_t i, uint32_t v) {
-      const uint32_t col = blk * kRateWords + i;
-      uint32_t o = col < words ? v : (col == words ? 0x01u : 0u);
-      if (blk == nblk - 1 && i == kRateWords - 1) o |= 0x80000000u;
-      return o;
-    };
-    const uint32_t col = blk * kRateWords + lane;  // words 0..31 of the block: lane = word
-#pragma unroll 1
-    for (int h = 0; h < 32; h += 8) {
-      uint32_t raw[8];
+  const uint32_t last = words / kRateWords;
+  stage_rows(st, base, r0, rows, words, 0);
+  for (uint32_t blk = 0;; ++blk) {
+    const uint2* row = reinterpret_cast<const uint2*>(st + (blk & 1u) * kStageWords + lane * kRateWords);
+    if (blk < last) {
+      stage_rows(st + (~blk & 1u) * kStageWords, base, r0, rows, words, blk + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();
 #pragma unroll
-      for (int k = 0; k < 8; ++k) raw[k] = (col < words && r0 + h + k < rows) ? word_at(r0 + h + k, col) : 0u;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) st[(h + k) * kStagePitch + lane] = pad(lane, raw[k]);
-    }
-#pragma unroll
-    for (int i = 32; i < kRateWords; ++i) {  // words 32, 33: lane = row
-      const uint32_t c2 = blk * kRateWords + i;
-      const uint32_t v = (c2 < words && r0 + lane < rows) ? word_at(r0 + lane, c2) : 0u;
-      st[lane * kStagePitch + i] = pad(i, v);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 17; ++k) {
-      s[k].x ^= st[lane * kStagePitch + 2 * k];
-      s[k].y ^= st[lane * kStagePitch + 2 * k + 1];
-    }
-    __syncwarp();
-    if (blk + 1 < nblk)
+      for (int k = 0; k < 17; ++k) {
+        const uint2 v = row[k];
+        s[k].x ^= conv(v.x);
+        s[k].y ^= conv(v.y);
+      }
+      __syncwarp();  // the stage may be refilled
       keccak_f1600<false>(s);
-    else
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      const int n = (int)(words - last * kRateWords);
+      auto pad = [&](int i, uint32_t v) { return (i < n ? conv(v) : i == n ? 0x01u : 0u) ^ (i == 33 ? 0x80000000u : 0u); };
+#pragma unroll
+      for (int k = 0; k < 17; ++k) {
+        const uint2 v = row[k];
+        s[k].x ^= pad(2 * k, v.x);
+        s[k].y ^= pad(2 * k + 1, v.y);
+      }
+      __syncwarp();
       keccak_f1600_digest<false>(s);
+      break;
+    }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) s[i] = bi_from_lane(s[i]);

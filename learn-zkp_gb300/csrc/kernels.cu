@@ -616,7 +616,9 @@ __global__ void __launch_bounds__(kQuadMixThreads, kQuadMixBlocks)
     has_t = w.has_t;
     has_u0 = w.has_u0;
     if (threadIdx.x < 128) gf_basis(basis, w.t, threadIdx.x);
-    if ((threadIdx.x & 127u) == 127u) gf_prepare(threadIdx.x < 128 ? w.u0 : w.u1, reinterpret_cast<uint32_t*>(prep + (threadIdx.x < 128 ? 0 : 9)));
+    // one thread of two other warps for u0 and u1, beside the basis
+    if (threadIdx.x == kQuadMixThreads - 33) gf_prepare(w.u0, reinterpret_cast<uint32_t*>(prep));
+    if (threadIdx.x == kQuadMixThreads - 1) gf_prepare(w.u1, reinterpret_cast<uint32_t*>(prep + 9));
   }
   __syncthreads();
   if (has_t) QuadTabM::build(sm, basis);
@@ -1018,17 +1020,15 @@ __global__ void __cluster_dims__(kTopCluster, 1, 1) __launch_bounds__(kTreeThrea
 
 // Leaf of a row of `width` elements: keccak256 of its 16*width bytes
 // (GenericHasher over the row's bincode, p3/src/symmetric.rs:16-25), any
-// number of 136-byte blocks; a warp stages the blocks of 32 rows through
-// shared memory (keccak_rows_warp) so that its loads read whole row runs.
-__global__ void __launch_bounds__(128) leaves_rows_kernel(const uint4* __restrict__ cw, uint4* __restrict__ leaves,
+// number of 136-byte blocks (keccak_rows_warp).  Five blocks per SM (96
+// registers) measured 541 us for 2^15 rows of 8 KB, four 543, six 593.
+__global__ void __launch_bounds__(128, 5) leaves_rows_kernel(const uint4* __restrict__ cw, uint4* __restrict__ leaves,
                                                           size_t n, size_t width) {
-  __shared__ uint32_t stage[4][32 * kStagePitch];
+  __shared__ __align__(16) uint32_t stage[4][2 * kStageWords];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t* words = reinterpret_cast<const uint32_t*>(cw);
-  const size_t row_words = 4 * width;
-  auto word_at = [&](size_t row, uint32_t i) { return words[row * row_words + i]; };
   for (size_t r0 = ((size_t)blockIdx.x * 4 + warp) * 32; r0 < n; r0 += (size_t)gridDim.x * 128) {
-    const Digest dg = keccak_rows_warp(stage[warp], r0, n, (uint32_t)row_words, word_at);
+    const Digest dg = keccak_rows_warp(stage[warp], reinterpret_cast<const uint32_t*>(cw), r0, n, (uint32_t)(4 * width),
+                                       [](uint32_t v) { return v; });
     if (r0 + lane < n) store_digest(leaves, r0 + lane, dg);
   }
 }

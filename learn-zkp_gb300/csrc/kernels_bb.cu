@@ -567,17 +567,16 @@ __global__ void __launch_bounds__(128) bb_leaves_one_kernel(const uint32_t* __re
 }
 
 // Any width: keccak256 of the row's 4w bytes (GenericHasher over the row's
-// bincode, p3/src/symmetric.rs:11-25): canonical words staged by a warp per
-// 32 rows (keccak_rows_warp).  Five blocks per SM (96 registers, a few spilled
-// words) measured about 1% faster than four at 128 registers.
+// bincode, p3/src/symmetric.rs:11-25): the words made canonical as they are absorbed
+// (keccak_rows_warp).  Five blocks per SM (96 registers) measured the same as four,
+// six 2% slower.
 __global__ void __launch_bounds__(128, 5) bb_leaves_rows_kernel(const uint32_t* __restrict__ cw,
                                                             uint4* __restrict__ leaves, size_t rows, uint32_t w,
                                                             int bits) {
-  __shared__ uint32_t stage[4][32 * kStagePitch];
+  __shared__ __align__(16) uint32_t stage[4][2 * kStageWords];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto word_at = [&](size_t row, uint32_t i) { return bb::from_mont(cw[row * w + i]); };
   for (size_t r0 = ((size_t)blockIdx.x * 4 + warp) * 32; r0 < rows; r0 += (size_t)gridDim.x * 128) {
-    const Digest dg = keccak_rows_warp(stage[warp], r0, rows, w, word_at);
+    const Digest dg = keccak_rows_warp(stage[warp], cw, r0, rows, w, [](uint32_t v) { return bb::from_mont(v); });
     if (r0 + lane < rows) store_digest(leaves, brev_bits(r0 + lane, bits), dg);
   }
 }

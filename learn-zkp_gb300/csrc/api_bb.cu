@@ -569,9 +569,10 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
     std::memcpy(p->pin.b() + sizeof(t), &c, sizeof(c));
     CU(cudaMemcpyAsync(tdev, p->pin.p, tsz, cudaMemcpyHostToDevice, st));
   }
-  // A round's sums need only the previous fix and its fix only the round's
+  // A large round's sums need only the previous fix and its fix only the round's
   // challenge, so both run on `aux` beside the round's tree and fold: the
-  // main stream's chain per round is tree, transcript step, fold.
+  // main stream's chain per round is tree, transcript step, fold.  Small rounds
+  // (bb_fold_takes_fix) fix in the fold's launch.
   struct AuxJoin {  // joins `aux` back into the main stream on every exit
     bf_bb_pcs* p;
     cudaStream_t st;
@@ -585,6 +586,7 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
   CU(cudaStreamWaitEvent(sa, p->ev_fork, 0));
   join.active = true;
   size_t fold_off = 0, tree_off = 0;
+  bool fixed_here = false;  // the round before ran its fix and this round's sums on `st`
   for (int k = 0; k < d; ++k) {
     const int i = d - 1 - k, li = p->log2_n0() + i;
     const int ri = i + lk;  // the sumcheck round (basefold.rs:356-361)
@@ -596,8 +598,10 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
     if (k == 0) CU(bf::bb_launch_leaves_pairs(pi, base_k, tree, ni, li, st));  // later rounds: made by the fold
     CU(bf::launch_tree(tree, ni, st, root_dev, bf::Tune()));
     if (ni <= (size_t)bf::kBbTailMax) {  // this round and the rest in one block
-      CU(cudaEventRecord(p->ev_dot, sa));  // the last fix
-      CU(cudaStreamWaitEvent(st, p->ev_dot, 0));
+      if (!fixed_here) {
+        CU(cudaEventRecord(p->ev_dot, sa));  // the last fix
+        CU(cudaStreamWaitEvent(st, p->ev_dot, 0));
+      }
       bf::BbTail tp{};
       tp.i0 = i;
       tp.lk = lk;
@@ -627,19 +631,18 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
       poly = fixbuf[k & 1];
       break;
     }
-    CU(cudaMemsetAsync(acc, 0, 40, sa));
-    CU(bf::bb_launch_dot(heq, poly, base_k, (size_t)1 << ri, acc, sa));
-    CU(cudaEventRecord(p->ev_dot, sa));
-    CU(cudaStreamWaitEvent(st, p->ev_dot, 0));
+    if (!fixed_here) {
+      CU(cudaMemsetAsync(acc, 0, 40, sa));
+      CU(bf::bb_launch_dot(heq, poly, base_k, (size_t)1 << ri, acc, sa));
+      CU(cudaEventRecord(p->ev_dot, sa));
+      CU(cudaStreamWaitEvent(st, p->ev_dot, 0));
+    }
     uint32_t* x_k = xs_dev + 5 * (size_t)k;
     CU(bf::bb_launch_transcript_round(tdev, cdev, ri, root_dev, acc, base_k, x_k, rec_dev + 72 * (size_t)k, st));
-    CU(cudaEventRecord(p->ev_x, st));
-    CU(cudaStreamWaitEvent(sa, p->ev_x, 0));
     const bb::E5 unused{};
     uint32_t* fixed = fixbuf[k & 1];  // the fix two rounds back and the sums since have read it (stream order)
-    CU(bf::bb_launch_fix(poly, base_k, fixed, (size_t)1 << ri, unused, sa, x_k));
-    poly = fixed;
-    bf::BbFold fp;
+    fixed_here = i > 0 && bf::bb_fold_takes_fix(ni);
+    bf::BbFold fp{};
     fp.w = pi;
     fp.base = base_k;
     fp.out = folds + 5 * fold_off;
@@ -648,7 +651,22 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
     fp.leaves = i > 0 ? tree + 2 * (2 * ni) : nullptr;  // the next round's tree follows this one
     fp.leaf_bits = li - 1;
     fp.xp = x_k;
-    CU(bf::bb_launch_fold(fp, unused, st));
+    if (fixed_here) {  // small rounds: the fix and the next round's sums in the fold's launch
+      fp.poly = poly;
+      fp.poly_base = base_k;
+      fp.poly_out = fixed;
+      fp.half = (size_t)1 << ri;
+      fp.next_half = p->n_i(i - 1) <= (size_t)bf::kBbTailMax ? 0 : fp.half / 2;  // the tail makes its own
+      fp.heq = heq;
+      fp.sums = acc;
+      CU(bf::bb_launch_fold_fix(fp, st));
+    } else {
+      CU(cudaEventRecord(p->ev_x, st));
+      CU(cudaStreamWaitEvent(sa, p->ev_x, 0));
+      CU(bf::bb_launch_fix(poly, base_k, fixed, (size_t)1 << ri, unused, sa, x_k));
+      CU(bf::bb_launch_fold(fp, unused, st));
+    }
+    poly = fixed;
     pi = fp.out;
     fold_off += ni;
     tree_off += 2 * ni;

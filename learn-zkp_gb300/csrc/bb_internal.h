@@ -80,8 +80,21 @@ struct BbFold {
   uint4* leaves;          // n/2 leaves of the next round, or null
   int leaf_bits;          // log2(n/2)
   const uint32_t* xp;     // the challenge in device memory (Montgomery), or null: the x argument
+  // bb_launch_fold_fix only: the fix of the round's polynomial (2 half entries;
+  // canonical base-field when poly_base) and, when next_half > 0, the next round's
+  // sums over that many entries, added to sums
+  const uint32_t* poly;
+  int poly_base;
+  uint32_t* poly_out;
+  size_t half, next_half;
+  const uint32_t* heq;
+  unsigned long long* sums;
 };
 cudaError_t bb_launch_fold(const BbFold& p, const bb::E5& x, cudaStream_t st);
+// Whether a fold of n outputs with next-round leaves also takes the round's fix
+// and sums along (bb_launch_fold_fix), and that launch.
+bool bb_fold_takes_fix(size_t n);
+cudaError_t bb_launch_fold_fix(const BbFold& p, cudaStream_t st);
 
 // The open's Fiat–Shamir transcript on the device: HashChallenger<u8,
 // Keccak256Hash, 32> (p3/src/challenger.rs) as a sponge — the lanes of the
@@ -108,7 +121,7 @@ struct BbRoundConsts {
 // (Montgomery) and record the root and the compressed polynomial (72 canonical
 // bytes) at rec.
 cudaError_t bb_launch_transcript_round(BbTranscript* t, const BbRoundConsts* c, int ri, const uint4* root_dev,
-                                       const unsigned long long* sums, int canonical, uint32_t* x_out, uint8_t* rec,
+                                       unsigned long long* sums, int canonical, uint32_t* x_out, uint8_t* rec,
                                        cudaStream_t st);
 
 // The last rounds i0 .. 0 of an open in one block: the rounds whose fold has

@@ -206,7 +206,7 @@ __device__ __forceinline__ void st_e5(uint32_t* p, size_t i, const E5& e) {
 }  // namespace
 
 __global__ void __launch_bounds__(32) bb_transcript_round_kernel(BbTranscript* t, const BbRoundConsts* c, int ri,
-                                                                const uint4* root_dev, const unsigned long long* sums,
+                                                                const uint4* root_dev, unsigned long long* sums,
                                                                 int canonical, uint32_t* x_out, uint8_t* rec) {
   __shared__ BbStepShared sh;
   const WarpKeccak wk;
@@ -214,6 +214,7 @@ __global__ void __launch_bounds__(32) bb_transcript_round_kernel(BbTranscript* t
   tr_copy(&sh.t, t);
   const uint32_t v = (uint32_t)(sums[threadIdx.x % 5] % bb::P);
   __syncwarp();
+  if (threadIdx.x < 5) sums[threadIdx.x] = 0;  // for the fix that adds up the next round's
   bb_round_step(wk, sh, c, ri, root_dev, canonical ? bb::to_mont(v) : v, rec);
   if (threadIdx.x < 5) x_out[threadIdx.x] = sh.x[threadIdx.x];
   tr_copy(t, &sh.t);
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
 }
 
 cudaError_t bb_launch_transcript_round(BbTranscript* t, const BbRoundConsts* c, int ri, const uint4* root_dev,
-                                       const unsigned long long* sums, int canonical, uint32_t* x_out, uint8_t* rec,
+                                       unsigned long long* sums, int canonical, uint32_t* x_out, uint8_t* rec,
                                        cudaStream_t st) {
   const cudaError_t e =
       launch_chained(bb_transcript_round_kernel, 1, 32, 0, st, t, c, ri, root_dev, sums, canonical, x_out, rec);

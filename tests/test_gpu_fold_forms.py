@@ -40,3 +40,23 @@ def test_prime_folds(built_lib, n, log2_c, w):
     assert comm.root == root
     proof = pcs.open(comm, [prime.PrimePolyEvals(values, point)], GenericChallenger.from_state(blob))
     assert proof == O.bb_open(n, log2_c, flat, point, values, blob)
+
+
+@pytest.mark.parametrize("n,log2_c,lk,w", [(11, 0, 9, 1), (12, 1, 9, 2), (14, 0, 10, 1)])
+def test_prime_folds_without_a_tail(built_lib, n, log2_c, lk, w):
+    """Base codes of more than 2^8 rows: the last round's fix is a launch of its
+    own after rounds that fix in the fold's."""
+    from basefold_gpu import BasefoldConfig, GenericChallenger, prime
+
+    rng = np.random.default_rng(9970 + n + w)
+    data = rng.integers(0, O.BB_P, (1 << n, w), dtype=np.uint32)
+    point = rng.integers(0, O.BB_P, (n, 5), dtype=np.uint32)
+    flat = data if w > 1 else data.reshape(-1)
+    kw = dict(log2_k0=lk, ts=O.bb_random_ts(n, log2_c, lk, 5))
+    code = prime.GenericRandomFoldableCode(128, log2_c, lk, n - lk, kw["ts"])
+    pcs = prime.BabyBearBasefold.setup(BasefoldConfig(code), device=0)
+    comm = pcs.commit(data)
+    root, values, blob = O.bb_harness_prepare(n, log2_c, flat, point, **kw)
+    assert comm.root == root
+    proof = pcs.open(comm, [prime.PrimePolyEvals(values, point)], GenericChallenger.from_state(blob))
+    assert proof == O.bb_open(n, log2_c, flat, point, values, blob, **kw)

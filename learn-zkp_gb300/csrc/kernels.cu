@@ -1718,47 +1718,68 @@ __global__ void __launch_bounds__(256, 2) prod_sums_kernel(PolyPtrs p, size_t ha
   prod_sums_store<K>(t, scratch, acc);
 }
 
-// Fix the top variable of every polynomial at r and accumulate the next
-// round's sums.  Each thread produces the pair (b, b + half/2) of the fixed
-// polynomials, which is exactly what the next round's sums need.
+// Fix the top variable of every polynomial at r and accumulate the next round's
+// sums.  Outputs b and b + half/2 are the pair that the next round's sums need; a
+// block takes 32 pairs, a warp per output of the fix and then a warp per product
+// of the sums: one thread per pair runs its 6 (K = 2) or 13 (K = 3) products of
+// 0.65 us one after another.  Bound by that chain and the launch below about 2^13
+// pairs, by the wide multiplier above.  Measured on GB300 against a thread per
+// pair: K = 2, 2^9 to 2^13 pairs 7.4 to 8.3 us (12), 2^14 10.2 (12.4), 2^15 13.7
+// (12.6), 2^16 18.4 (17.9); K = 3, 2^9 to 2^12 pairs 8.3 to 9.1 us (20), 2^14 14.4
+// (20.8), 2^15 19.7 (23.2).
 template <int K>
-__global__ void __launch_bounds__(256, 2) prod_fix_kernel(PolyPtrs p, size_t half, uint4 r, uint32_t* acc,
-                                                       const uint4* xp) {
-  __shared__ uint4 scratch[32];
+__global__ void __launch_bounds__(64 * K) prod_fix_kernel(PolyPtrs p, size_t half, uint4 r, uint32_t* acc,
+                                                                const uint4* xp) {
+  __shared__ uint4 f[2 * K][32];  // lo, then hi of every polynomial
+  __shared__ uint4 m[K == 3 ? 3 : 1][32];  // K = 3: b1 b2, lo1 lo2, hi1 hi2
   chain_wait();
   if (xp) r = *xp;
   const size_t nh = half >> 1;
-  if (nh == 0) {  // last round: one output per polynomial
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const uint4 lo = p.in[k][0], hi = p.in[k][1];
-        p.out[k][0] = gf_add(lo, gf_mul(r, gf_add(hi, lo)));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = warp % K, s = warp / K;
+  uint4 sum = make_uint4(0, 0, 0, 0);
+  for (size_t b0 = (size_t)blockIdx.x * 32; b0 < (nh ? nh : 1); b0 += (size_t)gridDim.x * 32) {
+    const size_t b = b0 + lane + (s ? nh : 0);
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (nh ? b0 + lane < nh : threadIdx.x < 32 * K && lane == 0) {
+      const uint4 a0 = p.in[j][b], a1 = p.in[j][b + half];
+      v = gf_add(a0, gf_mul(r, gf_add(a1, a0)));
+      p.out[j][b] = v;
+    }
+    if (nh == 0) return;  // the last round has one output per polynomial and no sums
+    f[warp][lane] = v;
+    __syncthreads();
+    if (K == 2) {
+      if (warp < 2) {  // c0 = lo0 lo1, c2 = b0 b1
+        const uint4 l0 = f[0][lane], l1 = f[1][lane];
+        const uint4 u = warp ? gf_add(l0, f[K][lane]) : l0, w = warp ? gf_add(l1, f[K + 1][lane]) : l1;
+        sum = gf_add(sum, gf_mul(u, w));
+      }
+    } else {
+      if (warp < 3) {
+        const uint4 l1 = f[1][lane], h1 = f[K + 1][lane], l2 = f[K - 1][lane], h2 = f[2 * K - 1][lane];
+        m[K == 3 ? warp : 0][lane] = gf_mul(warp == 0 ? gf_add(l1, h1) : warp == 1 ? l1 : h1,
+                                            warp == 0 ? gf_add(l2, h2) : warp == 1 ? l2 : h2);
+      }
+      __syncthreads();
+      if (warp < 4) {  // c0 = lo0 lo12; c2 = b0 cross + lo0 b12, cross = hi12 + lo12 + b12; c3 = b0 b12
+        const uint4 b12 = m[0][lane], lo12 = m[K == 3 ? 1 : 0][lane], hi12 = m[K == 3 ? 2 : 0][lane];
+        const uint4 l0 = f[0][lane], e0 = gf_add(l0, f[K][lane]);
+        sum = gf_add(sum, gf_mul(warp == 0 || warp == 2 ? l0 : e0,
+                                 warp == 0 ? lo12 : warp == 1 ? gf_add(gf_add(hi12, lo12), b12) : b12));
       }
     }
-    return;
+    __syncthreads();  // f and m are read
   }
-  ProdSums t = {};
-  for (size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x; b < nh; b += (size_t)gridDim.x * blockDim.x) {
-    uint4 lo[K], hi[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const uint4 a0 = p.in[k][b], a1 = p.in[k][b + half];
-      const uint4 c0 = p.in[k][b + nh], c1 = p.in[k][b + nh + half];
-      lo[k] = gf_add(a0, gf_mul_call(r, gf_add(a1, a0)));
-      hi[k] = gf_add(c0, gf_mul_call(r, gf_add(c1, c0)));
-      p.out[k][b] = lo[k];
-      p.out[k][b + nh] = hi[k];
-    }
-    prod_terms<K>(lo, hi, t);
+  if (warp < (K == 2 ? 2 : 4)) {
+    sum = warp_xor(sum);
+    if (lane == 0) atomic_xor4(acc + 4 * (K == 2 ? warp : warp == 0 ? 0 : warp == 3 ? 2 : 1), sum);
   }
-  prod_sums_store<K>(t, scratch, acc);
 }
 
 // The same fix for large rounds: the products by the challenge, 2 K of the 2 K
 // + 2 (K = 2) or + 7 (K = 3) products of an element pair, come from a
 // shared-memory table of r (GfTab), so the wide multiplier, which bounds
-// prod_fix_kernel, is left with the sums' products, and the table's loads run
+// prod_fix_kernel in large rounds, is left with the sums' products, and the table's loads run
 // beside it.  One persistent block per SM builds the table (about 3 us) and
 // walks the pairs.  Measured on GB300, clocks per pair and SM: K = 3 67 at 512
 // threads (68 at 384, 77 at 256; 95 without the table); K = 2 22 at 768
@@ -1811,12 +1832,11 @@ cudaError_t launch_prod_round_sums(const uint4* const* polys, int k, size_t half
   return cudaGetLastError();
 }
 
-// Pairs from which a fix uses the table: below, building it (about 6 us more
-// than a small launch) costs more than its products save.  Measured on GB300,
-// without and with the table: k = 2 13.3 and 14.3 us at 2^16 pairs, 25.1 and
-// 23.2 at 2^17, 156 and 80 at 2^20; k = 3 16.1 and 22.3 us at 2^15, 27.1 and
-// 22.4 at 2^16, 325 and 239 at 2^20.
-constexpr size_t prod_tab_min(int k) { return (size_t)1 << (k == 2 ? 17 : 16); }
+// Pairs from which a fix uses the table, whose build takes a launch of few pairs to
+// 18 us (k = 2) or 26 us (k = 3).  Measured on GB300, without and with the table: k =
+// 2 18.1 and 18.2 us at 2^16 pairs, 26.9 and 27.2 at 2^17, 47.3 and 35.8 at 2^18; k = 3
+// 19.9 and 26.3 us at 2^15, 30.2 and 26.4 at 2^16, 56.1 and 43.2 at 2^17.
+constexpr size_t prod_tab_min(int k) { return (size_t)1 << (k == 2 ? 18 : 16); }
 
 cudaError_t launch_prod_fix(uint4* const* out, const uint4* const* in, int k, size_t half, uint4 r, size_t next_half,
                             uint32_t* acc, cudaStream_t st, const uint4* xp) {
@@ -1836,8 +1856,8 @@ cudaError_t launch_prod_fix(uint4* const* out, const uint4* const* in, int k, si
     COUNT_LAUNCH();
     return e;
   }
-  const cudaError_t e = launch_chained(k == 2 ? prod_fix_kernel<2> : prod_fix_kernel<3>, grid_for(work, 256), 256, 0, st,
-                                       p, half, r, acc, xp);
+  const cudaError_t e = launch_chained(k == 2 ? prod_fix_kernel<2> : prod_fix_kernel<3>,
+                                       grid_for(work, 32), 64 * k, 0, st, p, half, r, acc, xp);
   COUNT_LAUNCH();
   return e;
 }

@@ -468,8 +468,8 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
                         Q * rec,
                         128,
                         w > 1 ? 20 * rows : 0,
-                        sizeof(bf::BbTranscript) + sizeof(bf::BbRoundConsts),
-                        (20 + 72) * (size_t)(d > 0 ? d : 1),
+                        sizeof(bf::BbRoundConsts) + sizeof(bf::BbTranscript) + 72 * (size_t)d + 20 * k0,
+                        20 * (size_t)d,
                         w > 1 ? 20 * w : 0};
   constexpr int kSlots = sizeof(wsz) / sizeof(wsz[0]);
   size_t off[kSlots + 1] = {0};
@@ -487,15 +487,22 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
   unsigned long long* acc = reinterpret_cast<unsigned long long*>(base + off[9]);
   uint4* root_dev = reinterpret_cast<uint4*>(base + off[9] + 64);  // after the five sums
   uint32_t* poly_canon = reinterpret_cast<uint32_t*>(base + off[10]);  // width > 1: the combined poly, canonical
-  // the device transcript, the round constants, each round's challenge (20 bytes) and record (72)
-  bf::BbTranscript* tdev = reinterpret_cast<bf::BbTranscript*>(base + off[11]);
-  bf::BbRoundConsts* cdev = reinterpret_cast<bf::BbRoundConsts*>(base + off[11] + sizeof(bf::BbTranscript));
+  // the round constants and the device transcript (copied in), each round's record (72
+  // bytes) and the final polynomial when the tail makes it (copied out with the
+  // transcript); each round's challenge (20 bytes)
+  static_assert(sizeof(bf::BbRoundConsts) % 8 == 0, "the transcript follows the constants");
+  bf::BbRoundConsts* cdev = reinterpret_cast<bf::BbRoundConsts*>(base + off[11]);
+  bf::BbTranscript* tdev = reinterpret_cast<bf::BbTranscript*>(base + off[11] + sizeof(bf::BbRoundConsts));
+  uint8_t* rec_dev = reinterpret_cast<uint8_t*>(tdev + 1);
+  uint32_t* fin_dev = reinterpret_cast<uint32_t*>(rec_dev + 72 * (size_t)d);
   uint32_t* xs_dev = reinterpret_cast<uint32_t*>(base + off[12]);
-  uint8_t* rec_dev = base + off[12] + 20 * (size_t)(d > 0 ? d : 1);
   uint32_t* scal_dev = reinterpret_cast<uint32_t*>(base + off[13]);  // width > 1: the batching scalars
-  CU(p->pin.ensure(std::max<size_t>(8 * Q + 20 * k0 + 20 * 64 + 256 + sizeof(bf::BbTranscript) +
-                                         sizeof(bf::BbRoundConsts) + 72 * (size_t)d,
-                                     20 * w)));
+  // staging: the round constants and the transcript, then the batching scalars; later
+  // the results (transcript, records, final polynomial, the check's entries) and
+  // the query indices
+  const size_t tsz = sizeof(bf::BbRoundConsts) + sizeof(bf::BbTranscript), scal_off = (tsz + 255) & ~(size_t)255;
+  CU(p->pin.ensure(std::max<size_t>(8 * Q + 20 * k0 + 20 * 64 + 256 + sizeof(bf::BbTranscript) + 72 * (size_t)d,
+                                     scal_off + 20 * w)));
 
   // The polynomial and codeword the folding sumcheck runs on (basefold.rs:154-177).
   E claim;
@@ -508,7 +515,7 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
     const std::vector<E> s = bbh::scalars_by_eq(w, tr);
     for (size_t c = 0; c < w; ++c) claim = bbh::eadd(claim, bbh::emul(s[c], vals[c]));
     // s R^2 against the canonical evaluations
-    bb::E5* sd = reinterpret_cast<bb::E5*>(p->pin.p);
+    bb::E5* sd = reinterpret_cast<bb::E5*>(p->pin.b() + scal_off);
     for (size_t c = 0; c < w; ++c) sd[c] = bbh::to_dev2(s[c]);
     CU(cudaMemcpyAsync(scal_dev, sd, 20 * w, cudaMemcpyHostToDevice, st));
     CU(bf::bb_launch_combine(cm->data.as<uint32_t>(), rows, w, scal_dev, polyE, st));
@@ -517,11 +524,8 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
     // combined polynomial, coefficient by coefficient: a 5-column encode of
     // 2^num_vars rows instead of w products per codeword row, the same values.
     CU(bf::bb_launch_from_mont(polyE, poly_canon, 5 * rows, st));
-    uint32_t* flag = p->small.as<uint32_t>();
-    CU(cudaMemsetAsync(flag, 0, 4, st));
-    CU(bf::bb_launch_encode(poly_canon, piE, p->d, p->log2_c, p->log2_k0, p->generic, 5, p->tw.as<uint2>(), flag,
-                            st));
-    CU(cudaStreamSynchronize(st));  // the staging of the scalars is reused below
+    CU(bf::bb_launch_encode(poly_canon, piE, p->d, p->log2_c, p->log2_k0, p->generic, 5, p->tw.as<uint2>(),
+                            p->small.as<uint32_t>(), st));  // the flag is not read: the input is canonical
     poly = polyE;
     pi = piE;
     base_round = 0;
@@ -536,7 +540,6 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
   std::vector<std::array<uint8_t, 32>> roots;
   bf::BbGather gp{};
   gp.pi0_base = w == 1;
-  const size_t tsz = sizeof(bf::BbTranscript) + sizeof(bf::BbRoundConsts);
   if (d > 0) {
     // the caller's transcript as a sponge: whole 136-byte blocks of its input
     // absorbed here, the rest pending
@@ -565,9 +568,9 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
       c.r_inv[k] = bbh::to_dev(es.r_inv[k]);
       c.cf[k] = bbh::to_dev(cf[k]);
     }
-    std::memcpy(p->pin.p, &t, sizeof(t));
-    std::memcpy(p->pin.b() + sizeof(t), &c, sizeof(c));
-    CU(cudaMemcpyAsync(tdev, p->pin.p, tsz, cudaMemcpyHostToDevice, st));
+    std::memcpy(p->pin.p, &c, sizeof(c));
+    std::memcpy(p->pin.b() + sizeof(c), &t, sizeof(t));
+    CU(cudaMemcpyAsync(cdev, p->pin.p, tsz, cudaMemcpyHostToDevice, st));
   }
   // A large round's sums need only the previous fix and its fix only the round's
   // challenge, so both run on `aux` beside the round's tree and fold: the
@@ -613,7 +616,7 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
       tp.heq = heq;
       tp.tinv = p->tinv.as<uint32_t>();
       tp.fold_out = folds + 5 * fold_off;
-      tp.poly_out = fixbuf[k & 1];
+      tp.poly_out = fin_dev;
       tp.next_tree = tree + 2 * (2 * ni);
       tp.root = root_dev;
       tp.t = tdev;
@@ -628,7 +631,7 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
         gp.trees[q] = trees + 2 * tree_off;
       }
       pi = folds + 5 * fold_off;  // round d - 1's outputs
-      poly = fixbuf[k & 1];
+      poly = fin_dev;
       break;
     }
     if (!fixed_here) {
@@ -678,26 +681,25 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
   std::vector<E> fin(k0);
   {
     const int fin_base = d == 0 && base_round;  // still the caller's base-field data
-    CU(cudaMemcpyAsync(p->pin.p, poly, (fin_base ? 4 : 20) * k0, cudaMemcpyDeviceToHost, st));
-    const size_t chk_off = 20 * k0 + 64;
-    const size_t t_off = chk_off + 20 * 64;  // then the transcript, then the round records
+    const size_t rec_off = sizeof(bf::BbTranscript), fin_off = rec_off + 72 * (size_t)d, chk_off = fin_off + 20 * k0;
     size_t nchk = 0;
+    const bool one_copy = poly == fin_dev;  // behind the transcript and the records
+    if (d > 0) CU(cudaMemcpyAsync(p->pin.p, tdev, one_copy ? chk_off : fin_off, cudaMemcpyDeviceToHost, st));
+    if (!one_copy)
+      CU(cudaMemcpyAsync(p->pin.b() + fin_off, poly, (fin_base ? 4 : 20) * k0, cudaMemcpyDeviceToHost, st));
     if (d > 0) {  // debug_assert_eq!(encode0(final_poly), pi) (basefold.rs:189), up to 64 entries
       nchk = p->n0() < 64 ? p->n0() : 64;
       CU(cudaMemcpyAsync(p->pin.b() + chk_off, pi, 20 * nchk, cudaMemcpyDeviceToHost, st));
-      CU(cudaMemcpyAsync(p->pin.b() + t_off, tdev, sizeof(bf::BbTranscript), cudaMemcpyDeviceToHost, st));
-      CU(cudaMemcpyAsync(p->pin.b() + t_off + sizeof(bf::BbTranscript), rec_dev, 72 * (size_t)d,
-                         cudaMemcpyDeviceToHost, st));
     }
     CU(cudaStreamSynchronize(st));
     for (size_t t = 0; t < k0; ++t) {
       if (fin_base) {
         uint32_t v;
-        std::memcpy(&v, p->pin.b() + 4 * t, 4);
+        std::memcpy(&v, p->pin.b() + fin_off + 4 * t, 4);
         fin[t] = E::from(v);
       } else {
         uint32_t m[5];
-        std::memcpy(m, p->pin.b() + 20 * t, 20);
+        std::memcpy(m, p->pin.b() + fin_off + 20 * t, 20);
         for (int q = 0; q < 5; ++q) fin[t].c[q] = bb::from_mont(m[q]);
       }
     }
@@ -713,12 +715,12 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
       // the caller's transcript continues from the device's: after a sample the
       // sponge holds no absorbed block, only pending input bytes
       bf::BbTranscript t;
-      std::memcpy(&t, p->pin.b() + t_off, sizeof(t));
+      std::memcpy(&t, p->pin.p, sizeof(t));
       for (int l = 0; l < 25; ++l)
         if (t.A[l].x | t.A[l].y) return fail(BF_ERR_CHECK, "device transcript left an absorbed block");
       tr.in.assign(t.pend, t.pend + t.pend_len);
       tr.out.assign(t.out, t.out + t.out_len);
-      const uint8_t* rb = p->pin.b() + t_off + sizeof(bf::BbTranscript);
+      const uint8_t* rb = p->pin.b() + rec_off;
       for (int k = 0; k < d; ++k) {
         std::array<uint8_t, 32> root;
         std::memcpy(root.data(), rb + 72 * k, 32);

@@ -179,12 +179,12 @@ int eval_enqueue(bf_pcs* p, const bf_commitment* cm, const uint8_t* point, uint4
 struct bf_open_session;
 namespace bfapi {
 int open_start_impl(bf_pcs* p, const bf_commitment* cm, const uint8_t* point, const uint8_t* values,
-                    const uint8_t* scalars, void* stream, bf_open_session** out);
+                    const uint8_t* scalars, void* stream, bf_open_session** out, const bfh::Challenger* resident);
 // The pieces of open_start_impl / open_resident_enqueue, for graph capture:
 // host-side preparation (pinned staging) apart from the device work.
 int open_session_create(bf_pcs* p, const bf_commitment* cm, void* stream, bf_open_session** out);
 int open_session_prepare(bf_open_session* s, const uint8_t* point, const uint8_t* values, const uint8_t* scalars);
-int open_session_enqueue_start(bf_open_session* s);
+int open_session_enqueue_start(bf_open_session* s, bool resident);
 const uint4* open_session_point_dev(const bf_open_session* s);
 void open_session_mark_launched(bf_open_session* s);  // the resident open was launched by a graph
 cudaStream_t open_session_stream(const bf_open_session* s);
@@ -194,8 +194,7 @@ void open_session_set_stream(bf_open_session* s, cudaStream_t st);
 cudaEvent_t open_session_event(const bf_open_session* s);
 int open_resident_prepare(bf_open_session* s, const bfh::Challenger& ch);
 int open_resident_enqueue_device(bf_open_session* s, const uint4* root_dev, const uint4* value_dev);
-int open_resident_enqueue(bf_open_session* s, const bfh::Challenger& ch, const uint4* root_dev,
-                          const uint4* value_dev);
+int open_resident_enqueue(bf_open_session* s, const uint4* root_dev, const uint4* value_dev);
 int open_resident_complete(bf_open_session* s, bfh::Challenger& ch);
 int open_finish_enqueue(bf_open_session* s, const uint64_t* indices, size_t nq);
 int open_finish_complete(bf_open_session* s, uint8_t* proof, size_t cap, size_t* proof_len);

@@ -211,11 +211,11 @@ int admit(bf_engine* e, Job* j) {
   CU(j->eval_ws.alloc_async(16 * half, p->pool, j->st));
   const uint4* value_dev = nullptr;
   TRY(eval_enqueue(p, j->cm.get(), pj->point, j->eval_ws.as<uint4>(), j->st, pin + 64, &value_dev));
-  TRY(open_start_impl(p, j->cm.get(), pj->point, nullptr, nullptr, j->st, &j->sess));
   const size_t nd = p->n_d();
   const uint4* root_dev = j->cm->tree.as<uint4>() + 2 * (2 * nd - 2);
   j->ch = bfh::Challenger();  // GenericChallenger::keccak256()
-  TRY(open_resident_enqueue(j->sess, j->ch, root_dev, value_dev));
+  TRY(open_start_impl(p, j->cm.get(), pj->point, nullptr, nullptr, j->st, &j->sess, &j->ch));
+  TRY(open_resident_enqueue(j->sess, root_dev, value_dev));
   j->state = J_OPEN;
   return BF_OK;
 }
@@ -226,7 +226,7 @@ int capture_job(bf_engine* e, int slot, Plan* pl) {
   bf_commitment* cm = pl->cm.get();
   cudaStream_t st = e->streams[slot];
   uint8_t* pin = slot_pin(e, slot);
-  TRY(open_session_enqueue_start(pl->sess));  // copies the point first: the evaluation reads it
+  TRY(open_session_enqueue_start(pl->sess, true));  // copies the point first: the evaluation reads it
   TRY(commit_enqueue(p, cm, cm->data.as<uint4>(), st, pin));
   const uint4* value_dev = nullptr;
   TRY(eval_enqueue(p, cm, nullptr, pl->eval_ws.as<uint4>(), st, pin + 64, &value_dev,

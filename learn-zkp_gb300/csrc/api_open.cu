@@ -61,7 +61,7 @@ struct bf_open_session {
   uint4* w_pi_first_tree = nullptr;
   uint4* w_poly_first = nullptr;
   // device transcript: per-round scalars, the OpenState, the round records
-  uint8_t* w_tail = nullptr;
+  uint8_t* w_in = nullptr;  // the inputs, see point_off()
   bf::OpenState* w_state = nullptr;
   uint8_t* w_rec = nullptr;
   bool resident_pending = false;   // a device-transcript open is in flight
@@ -82,10 +82,18 @@ struct bf_open_session {
   const uint4* first_pi() const { return w == 1 ? cm->cw.as<uint4>() : w_pi_first; }
   const uint4* first_poly() const { return w == 1 ? cm->data.as<uint4>() : w_poly_first; }
   const uint4* first_tree() const { return w == 1 ? cm->pi_tree.as<uint4>() : w_pi_first_tree; }
-  // Pinned offset of the device-transcript inputs: past the staging, the eq
-  // scalars and the point, whose host-to-device copies may still be queued
-  // when the resident open is enqueued.
-  size_t tail_in_off() const { return 64 + 16 * ((size_t)(d > 0 ? d : 1) + w); }
+  // The session's inputs lie one after another, in the pinned staging from byte
+  // 64 on and on the device, so that one copy takes them: the eq scalars (width
+  // > 1), the point, zeros for the rounds' stages, and for a device-transcript
+  // open the rounds' scalars (three per round: r_i, r_i^-1, correcting factor)
+  // and the OpenState image.
+  size_t n_point() const { return d > 0 ? d : 1; }
+  size_t point_off() const { return w > 1 ? 16 * w : 0; }
+  size_t stage_off() const { return point_off() + 16 * n_point(); }
+  size_t scal_off() const { return stage_off() + 48 * n_point(); }
+  size_t state_off() const { return scal_off() + 48 * n_point(); }
+  size_t inputs_end() const { return state_off() + sizeof(bf::OpenState); }
+  uint8_t* inputs_pin() const { return pin->b() + 64; }
   // Root of round d-1's tree on the device: the commitment's pair tree for
   // width 1, the combined rows' tree otherwise.
   const uint4* first_root_dev() const {
@@ -109,13 +117,10 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
-// Device-transcript workspace: per round 3 scalars (r_i, r_i^-1, correcting
-// factor), the OpenState, then 64 bytes per round (root, c0, c2) and the
-// final polynomial.
-size_t state_off(int d) { return align256(48 * (size_t)(d > 0 ? d : 1)); }
-size_t rec_off(int d) { return state_off(d) + align256(sizeof(bf::OpenState)); }
+// Device-transcript results, behind the OpenState: 64 bytes per round (root, c0,
+// c2) and the final polynomial.
+static_assert(sizeof(bf::OpenState) % 16 == 0, "records follow the state on 16-byte boundaries");
 size_t rec_bytes(int d) { return 64 * (size_t)d + 16; }
-size_t tail_bytes(int d) { return rec_off(d) + rec_bytes(d); }
 
 int session_alloc(bf_open_session* s) {
   bf_pcs* p = s->p;
@@ -132,15 +137,13 @@ int session_alloc(bf_open_session* s) {
     off += align256(bytes);
     return o;
   };
-  const size_t o_point = take(16 * n_point), o_fold = take(16 * n_fold), o_tree = take(32 * n_tree);
+  const size_t o_in = take(s->inputs_end() + rec_bytes(d)), o_fold = take(16 * n_fold), o_tree = take(32 * n_tree);
   const size_t o_poly = take(16 * half), o_heq = take(16 * half), o_lo = take(16 * 4096);
-  const size_t o_hi = take(16 * ((size_t)1 << hi_vars)), o_stage = take(48 * n_point);
+  const size_t o_hi = take(16 * ((size_t)1 << hi_vars));
   const size_t bb = p->block_bytes(s->w);
   const size_t o_idx = take(8 * (p->Q + 1)), o_open = take(bb * (p->Q + 1));
-  const size_t o_tail = take(tail_bytes(d));
-  size_t o_sc = 0, o_pif = 0, o_pift = 0, o_polyf = 0;
+  size_t o_pif = 0, o_pift = 0, o_polyf = 0;
   if (s->w > 1) {
-    o_sc = take(16 * s->w);
     o_pif = take(16 * p->n_d());
     o_pift = take(32 * p->n_d());
     o_polyf = take(16 * ((size_t)1 << d));
@@ -148,28 +151,27 @@ int session_alloc(bf_open_session* s) {
   CU(s->ws.alloc_async(off, p->pool, s->st));
   uint8_t* b = s->ws.as<uint8_t>();
   if (s->w > 1) {
-    s->w_scalars = reinterpret_cast<uint4*>(b + o_sc);
+    s->w_scalars = reinterpret_cast<uint4*>(b + o_in);
     s->w_pi_first = reinterpret_cast<uint4*>(b + o_pif);
     s->w_pi_first_tree = reinterpret_cast<uint4*>(b + o_pift);
     s->w_poly_first = reinterpret_cast<uint4*>(b + o_polyf);
   }
-  s->w_tail = b + o_tail;
-  s->w_state = reinterpret_cast<bf::OpenState*>(b + o_tail + state_off(d));
-  s->w_rec = b + o_tail + rec_off(d);
-  s->w_point = reinterpret_cast<uint4*>(b + o_point);
+  s->w_in = b + o_in;
+  s->w_point = reinterpret_cast<uint4*>(s->w_in + s->point_off());
+  s->w_stage = s->w_in + s->stage_off();
+  s->w_state = reinterpret_cast<bf::OpenState*>(s->w_in + s->state_off());
+  s->w_rec = s->w_in + s->inputs_end();
   s->w_pi_fold = reinterpret_cast<uint4*>(b + o_fold);
   s->w_pi_trees = reinterpret_cast<uint4*>(b + o_tree);
   s->w_poly = reinterpret_cast<uint4*>(b + o_poly);
   s->w_heq = reinterpret_cast<uint4*>(b + o_heq);
   s->w_eq_lo = reinterpret_cast<uint4*>(b + o_lo);
   s->w_eq_hi = reinterpret_cast<uint4*>(b + o_hi);
-  s->w_stage = b + o_stage;
   s->w_idx = reinterpret_cast<uint64_t*>(b + o_idx);
   s->w_open = b + o_open;
   const size_t res_off = align16(64 + 16 * (n_point + s->w) + 8 * (p->Q + 1) + bb * (p->Q + 1));
   const size_t pin_bytes =
-      std::max(res_off + align16(rec_bytes(d)) + sizeof(bf::OpenState),
-               s->tail_in_off() + 48 * n_point + sizeof(bf::OpenState));
+      std::max(res_off + sizeof(bf::OpenState) + rec_bytes(d), 64 + s->inputs_end());
   {
     std::lock_guard<std::mutex> lk(p->pinned_mu);
     if (!p->pinned_cache.empty()) {
@@ -267,10 +269,7 @@ int open_resident_prepare(bf_open_session* s, const bfh::Challenger& ch) {
     return fail(BF_ERR_ARG, "a device-transcript open starts before the first round");
   if (ch.in.size() > (size_t)bf::kTrMax || ch.out.size() > 32)
     return fail(BF_ERR_ARG, "transcript state too large for the device (%zu input bytes)", ch.in.size());
-  const size_t n_point = d > 0 ? d : 1;
-  // Inputs go where no copy still in flight reads (the start's scalar and
-  // point copies): scalars per round, then the OpenState image.
-  uint8_t* in = s->pin->b() + s->tail_in_off();
+  uint8_t* in = s->inputs_pin() + s->scal_off();
   for (int i = 0; i < d; ++i) {
     bfh::store(in + 48 * i, s->r[i]);
     bfh::store(in + 48 * i + 16, s->r_inv[i]);
@@ -284,7 +283,7 @@ int open_resident_prepare(bf_open_session* s, const bfh::Challenger& ch) {
   img.tr.out_len = (int)ch.out.size();
   img.outer = to_uint4(s->outer_val);
   img.delta = to_uint4(bfh::one());
-  std::memcpy(in + 48 * n_point, &img, sizeof(img));
+  std::memcpy(s->inputs_pin() + s->state_off(), &img, sizeof(img));
   return BF_OK;
 }
 
@@ -296,13 +295,9 @@ int open_resident_prepare(bf_open_session* s, const bfh::Challenger& ch) {
 int open_resident_enqueue_device(bf_open_session* s, const uint4* root_dev, const uint4* value_dev) {
   bf_pcs* p = s->p;
   const int d = s->d;
-  const size_t n_point = d > 0 ? d : 1;
-  const uint8_t* in = s->pin->b() + s->tail_in_off();
   cudaStream_t st = s->st;
-  if (d > 0) CU(cudaMemcpyAsync(s->w_tail, in, 48 * (size_t)d, cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(s->w_state, in + 48 * n_point, sizeof(bf::OpenState), cudaMemcpyHostToDevice, st));
   if (root_dev || value_dev) CU(bf::launch_open_observe(s->w_state, root_dev, value_dev, st));
-  const uint4* scal = reinterpret_cast<const uint4*>(s->w_tail);
+  const uint4* scal = reinterpret_cast<const uint4*>(s->w_in + s->scal_off());
   const uint4* xp = &s->w_state->x;
   const int i_tail = d > 0 ? tail_first_round(p, d) : -1;
   for (int i = d - 1; i > i_tail; --i) {  // large rounds: one kernel per step
@@ -348,19 +343,14 @@ int open_resident_enqueue_device(bf_open_session* s, const uint4* root_dev, cons
     ProfScope ps(p->prof, st, P_TAIL);
     CU(bf::launch_open_tail(tp, st));
   }
-  CU(cudaMemcpyAsync(s->res_pin, s->w_rec, rec_bytes(d), cudaMemcpyDeviceToHost, st));
-  CU(cudaMemcpyAsync(s->res_pin + align16(rec_bytes(d)), s->w_state, sizeof(bf::OpenState), cudaMemcpyDeviceToHost,
-                     st));
+  CU(cudaMemcpyAsync(s->res_pin, s->w_state, sizeof(bf::OpenState) + rec_bytes(d), cudaMemcpyDeviceToHost, st));
   return BF_OK;
 }
 
-// Enqueues every round of `s`, and the final polynomial, with the transcript
-// on the device, starting from `ch` (see open_resident_prepare /
-// open_resident_enqueue_device); nothing is read back until
-// open_resident_complete.
-int open_resident_enqueue(bf_open_session* s, const bfh::Challenger& ch, const uint4* root_dev,
-                          const uint4* value_dev) {
-  TRY(open_resident_prepare(s, ch));
+// Enqueues every round of a session started with its transcript
+// (open_start_impl), and the final polynomial, with the transcript on the device;
+// nothing is read back until open_resident_complete.
+int open_resident_enqueue(bf_open_session* s, const uint4* root_dev, const uint4* value_dev) {
   TRY(open_resident_enqueue_device(s, root_dev, value_dev));
   CU(cudaEventRecord(s->ev, s->st));
   s->pending = true;
@@ -378,9 +368,9 @@ int open_resident_complete(bf_open_session* s, bfh::Challenger& ch) {
   s->pending = false;
   s->resident_pending = false;
   const int d = s->d;
-  const uint8_t* res = s->res_pin;
+  const uint8_t* res = s->res_pin + sizeof(bf::OpenState);
   bf::OpenState img;
-  std::memcpy(&img, res + align16(rec_bytes(d)), sizeof(img));
+  std::memcpy(&img, s->res_pin, sizeof(img));
   if (img.status & 1) return fail(BF_ERR_ARG, "transcript input outgrew the device buffer");
   if (img.status & 2)
     return fail(BF_ERR_CHECK, "self-check failed: the last folded codeword is not encode0(final polynomial)");
@@ -481,7 +471,7 @@ extern "C" {
 int bf_open_start(bf_pcs* p, const bf_commitment* cm, const uint8_t* point, const uint8_t* values,
                   const uint8_t* scalars, void* stream, bf_open_session** out) {
   if (!values) return fail(BF_ERR_ARG, "null argument");
-  return open_start_impl(p, cm, point, values, scalars, stream, out);
+  return open_start_impl(p, cm, point, values, scalars, stream, out, nullptr);
 }
 
 }  // extern "C"
@@ -547,24 +537,26 @@ int open_session_prepare(bf_open_session* s, const uint8_t* point, const uint8_t
   s->roots.clear();
   put_u64(s->rounds, (uint64_t)d);
   put_u64(s->roots, (uint64_t)d);
-  uint8_t* pin = s->pin->b();
-  if (w > 1) std::memcpy(pin + 64, scalars, 16 * w);
-  if (d > 0) std::memcpy(pin + 64 + 16 * w, point, 16 * (size_t)d);
+  uint8_t* in = s->inputs_pin();
+  if (w > 1) std::memcpy(in, scalars, 16 * w);
+  if (d > 0) std::memcpy(in + s->point_off(), point, 16 * (size_t)d);
+  std::memset(in + s->stage_off(), 0, 48 * s->n_point());
   return BF_OK;
 }
 
-// Device side of the start, from the staging: row combination and the first
-// round's tree (width > 1), the point, the half-eq table and the first
-// round's reduction.  No event is recorded.
-int open_session_enqueue_start(bf_open_session* s) {
+// Device side of the start, from the staging: the inputs, row combination and the
+// first round's tree (width > 1), the half-eq table and the first round's
+// reduction, which is copied back unless the transcript's inputs are in the
+// staging too (resident).  No event is recorded.
+int open_session_enqueue_start(bf_open_session* s, bool resident) {
   bf_pcs* p = s->p;
   const bf_commitment* cm = s->cm;
   const int d = s->d;
   const size_t w = s->w;
   uint8_t* pin = s->pin->b();
   cudaStream_t st = s->st;
+  CU(cudaMemcpyAsync(s->w_in, s->inputs_pin(), resident ? s->inputs_end() : s->scal_off(), cudaMemcpyHostToDevice, st));
   if (w > 1) {  // combine rows with the eq scalars (basefold.rs:166-183)
-    CU(cudaMemcpyAsync(s->w_scalars, pin + 64, 16 * w, cudaMemcpyHostToDevice, st));
     {
       ProfScope ps(p->prof, st, P_FIX);
       CU(bf::launch_combine_rows(cm->data.as<uint4>(), (size_t)1 << d, w, s->w_scalars, s->w_poly_first, st));
@@ -579,7 +571,7 @@ int open_session_enqueue_start(bf_open_session* s) {
     if (e != cudaSuccess) return fail(BF_ERR_CUDA, "encode of the combined polynomial: %s", cudaGetErrorString(e));
   }
   if (d == 0) {
-    CU(cudaMemcpyAsync(pin, s->first_poly(), 16, cudaMemcpyDeviceToHost, st));
+    if (!resident) CU(cudaMemcpyAsync(pin, s->first_poly(), 16, cudaMemcpyDeviceToHost, st));
     return BF_OK;
   }
   if (w > 1) {  // the first round's tree over the combined codeword pairs
@@ -588,9 +580,6 @@ int open_session_enqueue_start(bf_open_session* s) {
     CU(bf::launch_leaves_pair(s->w_pi_first, s->w_pi_first_tree, n1, st));
     CU(bf::launch_tree(s->w_pi_first_tree, n1, st, reinterpret_cast<uint4*>(s->stage(d - 1)), p->tune));
   }
-  CU(cudaMemcpyAsync(s->w_point, pin + 64 + 16 * w, 16 * (size_t)d, cudaMemcpyHostToDevice, st));
-  CU(cudaMemsetAsync(s->stage(d - 1) + 32, 0, 16, st));
-  if (d >= 2) CU(cudaMemsetAsync(s->w_stage, 0, 48 * (size_t)(d - 1), st));
   {
     ProfScope ps(p->prof, st, P_EQ);
     CU(bf::launch_eq_table(s->w_point, d - 1, s->w_heq, s->w_eq_lo, s->w_eq_hi, st));
@@ -600,7 +589,7 @@ int open_session_enqueue_start(bf_open_session* s) {
     CU(bf::launch_dot_xor(s->w_heq, s->first_poly(), (size_t)1 << (d - 1),
                           reinterpret_cast<uint32_t*>(s->stage(d - 1) + 32), st));
   }
-  CU(cudaMemcpyAsync(pin, s->stage(d - 1), 48, cudaMemcpyDeviceToHost, st));
+  if (!resident) CU(cudaMemcpyAsync(pin, s->stage(d - 1), 48, cudaMemcpyDeviceToHost, st));
   return BF_OK;
 }
 
@@ -615,10 +604,11 @@ cudaStream_t open_session_stream(const bf_open_session* s) { return s->st; }
 void open_session_set_stream(bf_open_session* s, cudaStream_t st) { s->st = st; }
 cudaEvent_t open_session_event(const bf_open_session* s) { return s->ev; }
 
-// bf_open_start; `values` may be null when a device-transcript open will
-// observe the evaluation on the device (width 1).
+// bf_open_start, or with `resident` the start of a device-transcript open from that
+// transcript, to be followed by open_resident_enqueue; `values` may be null when it
+// will observe the evaluation on the device (width 1).
 int open_start_impl(bf_pcs* p, const bf_commitment* cm, const uint8_t* point, const uint8_t* values,
-                    const uint8_t* scalars, void* stream, bf_open_session** out) {
+                    const uint8_t* scalars, void* stream, bf_open_session** out, const bfh::Challenger* resident) {
   if (!p || !cm || !out || (p->d > 0 && !point)) return fail(BF_ERR_ARG, "null argument");
   if (!values && cm->width != 1) return fail(BF_ERR_ARG, "null argument");
   if (cm->width > 1 && !scalars) return fail(BF_ERR_ARG, "width > 1 needs the eq scalars");
@@ -628,7 +618,8 @@ int open_start_impl(bf_pcs* p, const bf_commitment* cm, const uint8_t* point, co
   std::unique_ptr<bf_open_session> s(raw);
   DeviceGuard g(p->device);
   TRY(open_session_prepare(s.get(), point, values, scalars));
-  TRY(open_session_enqueue_start(s.get()));
+  if (resident) TRY(open_resident_prepare(s.get(), *resident));
+  TRY(open_session_enqueue_start(s.get(), resident != nullptr));
   CU(cudaEventRecord(s->ev, s->st));
   s->pending = true;
   *out = s.release();
@@ -763,16 +754,17 @@ int bf_open(bf_pcs* p, const bf_commitment* cm, const uint8_t* point, const uint
     scal.resize(16 * sc.size());
     for (size_t c = 0; c < sc.size(); ++c) bfh::store(scal.data() + 16 * c, sc[c]);
   }
+  if (!values) return fail(BF_ERR_ARG, "null argument");
+  const bool fits = ch.in.size() + 64 <= (size_t)bf::kTrMax && ch.out.size() <= 32;
   bf_open_session* s = nullptr;
-  TRY(bf_open_start(p, cm, point, values, scal.empty() ? nullptr : scal.data(), nullptr, &s));
+  TRY(open_start_impl(p, cm, point, values, scal.empty() ? nullptr : scal.data(), nullptr, &s, fits ? &ch : nullptr));
   std::unique_ptr<bf_open_session, void (*)(bf_open_session*)> guard(s, bf_open_session_free);
   // every round and the final polynomial with the transcript on the device
   // (basefold.rs:185-196, 335-369), then the queries on the host; a pending
   // transcript input too long for the device buffer drives the rounds from
   // the host instead (same kernels)
-  const bool fits = ch.in.size() + 64 <= (size_t)bf::kTrMax && ch.out.size() <= 32;
   if (fits) {
-    TRY(open_resident_enqueue(s, ch, nullptr, nullptr));
+    TRY(open_resident_enqueue(s, nullptr, nullptr));
     TRY(open_resident_complete(s, ch));
   } else {
     while (true) {

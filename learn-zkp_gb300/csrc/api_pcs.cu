@@ -283,7 +283,7 @@ int commit_alloc(bf_pcs* p, bf_commitment* cm, cudaStream_t st) {
   const size_t nd = p->n_d(), w = cm->width;
   const bool pairs = p->d > 0 && w == 1;
   if (!cm->cw.p) CU(cm->cw.alloc_async(16 * nd * w, p->pool, st));
-  if (!cm->tree.p) CU(cm->tree.alloc_async(32 * (2 * nd - 1), p->pool, st));
+  if (!cm->tree.p) CU(cm->tree.alloc_async(32 * (2 * nd - 1 + (pairs ? 1 : 0)), p->pool, st));
   if (pairs && !cm->pi_tree.p) CU(cm->pi_tree.alloc_async(32 * (nd - 1), p->pool, st));
   return BF_OK;
 }
@@ -301,6 +301,7 @@ int commit_enqueue(bf_pcs* p, bf_commitment* cm, const uint4* data, cudaStream_t
   uint4* cw = cm->cw.as<uint4>();
   uint4* tree = cm->tree.as<uint4>();
   uint4* pit = cm->pi_tree.as<uint4>();
+  uint4* roots = tree + 2 * (2 * nd - 2);  // the tree's, and behind it a copy of the pair tree's
   {
     // encode; for width 1 and d >= 1 the last NTT pass also hashes the leaves
     ProfScope ps(p->prof, st, P_ENCODE);
@@ -329,17 +330,16 @@ int commit_enqueue(bf_pcs* p, bf_commitment* cm, const uint4* data, cudaStream_t
     ProfScope ps(p->prof, st, P_TREE);  // one scope from the fork to the join
     CU(cudaEventRecord(p->ev_fork, st));
     CU(cudaStreamWaitEvent(p->aux, p->ev_fork, 0));
-    CU(bf::launch_tree(pit, nd / 2, p->aux, nullptr, p->tune));
+    CU(bf::launch_tree(pit, nd / 2, p->aux, roots + 2, p->tune));
     CU(bf::launch_tree(tree, nd, st, nullptr, p->tune));
     CU(cudaEventRecord(p->ev_join, p->aux));
     CU(cudaStreamWaitEvent(st, p->ev_join, 0));
   } else {
     ProfScope ps(p->prof, st, P_TREE);
     CU(bf::launch_tree(tree, nd, st, nullptr, p->tune));
-    if (pairs) CU(bf::launch_tree(pit, nd / 2, st, nullptr, p->tune));
+    if (pairs) CU(bf::launch_tree(pit, nd / 2, st, roots + 2, p->tune));
   }
-  CU(cudaMemcpyAsync(roots_pin, tree + 2 * (2 * nd - 2), 32, cudaMemcpyDeviceToHost, st));
-  if (pairs) CU(cudaMemcpyAsync(roots_pin + 32, pit + 2 * (nd - 2), 32, cudaMemcpyDeviceToHost, st));
+  CU(cudaMemcpyAsync(roots_pin, roots, pairs ? 64 : 32, cudaMemcpyDeviceToHost, st));
   return BF_OK;
 }
 

@@ -111,7 +111,7 @@ struct alignas(8) BbTranscript {
 };
 // Per sumcheck round ri (< num_vars): the point coordinate, its inverse and
 // the correcting factor prod_{k >= ri} (1 - r_k)^-1 (eval_impr.rs:83-90).
-struct BbRoundConsts {
+struct alignas(8) BbRoundConsts {
   bb::E5 r[kBbMaxRounds], r_inv[kBbMaxRounds], cf[kBbMaxRounds];
 };
 // One folding-sumcheck round's transcript (sumcheck round ri): observe the

@@ -65,7 +65,7 @@ int sumcheck_run(cudaStream_t st, DevBuf& scratch, PinnedBuf& pinned, int k, int
     int ri = 0, round = n - 1;
     const uint4* const* src = in;
     for (; round >= bf::kSumcheckTailLog; --round, ++ri) {
-      CU(bf::launch_sumcheck_round(S, k, acc, rec + rec_sz * (size_t)ri, st));
+      CU(bf::launch_sumcheck_round(S, k, ri == 0, acc, rec + rec_sz * (size_t)ri, st));
       const size_t half = (size_t)1 << round;
       CU(bf::launch_prod_fix(work, src, k, half, uint4{}, half / 2, acc, st, &S->x));
       src = work;
@@ -73,6 +73,7 @@ int sumcheck_run(cudaStream_t st, DevBuf& scratch, PinnedBuf& pinned, int k, int
     bf::SumcheckTail tp{};
     for (int j = 0; j < k; ++j) tp.in[j] = src[j];
     tp.m = round + 1;
+    tp.first = ri == 0;
     tp.acc = acc;
     tp.state = S;
     tp.rec = rec + rec_sz * (size_t)ri;

@@ -178,12 +178,16 @@ struct alignas(16) DevTranscript {
 // Device-resident state of one open (basefold.rs:133-232): the transcript,
 // the claim of the first sumcheck round (`outer`, the evaluation), the
 // EvalProver claim of the later rounds (`inner`), the product of delta
-// scalars (eval_impr.rs:45-51) and the last challenge.  status bit 0: the
+// scalars (eval_impr.rs:45-51) and the last challenge.  c holds what the last
+// round's claim update needs (c0, c1, 1 + r; a product sumcheck's coefficients):
+// that update is left to the next step, where it waits for nothing (`inner`,
+// `delta` and a sumcheck's `outer` are those before it).  status bit 0: the
 // transcript input outgrew kTrMax; bit 1: the last folded codeword is not
 // encode0 of the final polynomial (basefold.rs:198).
 struct alignas(16) OpenState {
   DevTranscript tr;
   uint4 outer, inner, delta, x;
+  uint4 c[3];
   int status, pad_[3];
 };
 // Observes the commitment root (32 bytes at `root`) and the evaluation
@@ -199,11 +203,11 @@ cudaError_t launch_open_round(OpenState* s, int i, int d, const uint4* scal, con
 // One round of the product sumcheck's transcript on the device (warp):
 // from the sums acc = [c0, c2, c3] (sumcheck/src/function/quadratic.rs
 // 116-127 for k = 2; its k = 3 extension), observe the compressed round
-// polynomial, sample the challenge into s->x, and advance the claim
-// s->outer to the round polynomial at x (lib.rs:95-103).  `rec` receives
-// the compressed polynomial (16 k bytes) and the challenge (16 bytes); acc
-// (48 bytes) is cleared once read.
-cudaError_t launch_sumcheck_round(OpenState* s, int k, uint32_t* acc, uint8_t* rec, cudaStream_t st);
+// polynomial and sample the challenge into s->x; the claim s->outer becomes the
+// round polynomial at x (lib.rs:95-103) in the next step.  `first`: no round was
+// launched before.  `rec` receives the compressed polynomial (16 k bytes) and the
+// challenge (16 bytes); acc (48 bytes) is cleared once read.
+cudaError_t launch_sumcheck_round(OpenState* s, int k, bool first, uint32_t* acc, uint8_t* rec, cudaStream_t st);
 
 // The last m rounds of the product sumcheck in one block, from the first of
 // them's sums (acc, 48 bytes) and its k input polynomials of 2^m elements.
@@ -213,6 +217,7 @@ constexpr int kSumcheckTailLog = 9;
 struct SumcheckTail {
   const uint4* in[3];
   int m;
+  bool first;  // no round was launched before
   const uint32_t* acc;
   OpenState* state;
   uint8_t* rec;

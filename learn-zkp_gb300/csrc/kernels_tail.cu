@@ -130,8 +130,8 @@ __device__ uint4 warp_sample_elem(const WarpKeccak& wk, OpenState& o) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Transcript step of round i, warp-collective.  S = sum_b half_eq[b] poly_lo[b].
-// `rec` (global, 16-byte aligned) receives root, c0, c2.
+// The transcript step of round i in three parts, each warp-collective, so that only
+// the middle one stands between a round's root and its challenge.
 //
 // EvalImprProver::compute_round_poly gives [c0, c1] (eval_impr.rs:116-127);
 // EvalProver lifts it by delta = d * [1 - r, r - (1 - r)] = d * [1 + r, 1]
@@ -140,45 +140,59 @@ __device__ uint4 warp_sample_elem(const WarpKeccak& wk, OpenState& o) {
 // challenge x the EvalProver claim is c0 + c1 x and d becomes d (1 + r + x);
 // the sumcheck claim (the round polynomial at x) is only read in the first
 // round, so it is not carried.
-__device__ void round_step(const WarpKeccak& wk, OpenState& o, int i, int d, const uint4* scal, uint4 root_lo_bi,
-                           uint4 root_hi_bi, uint4 S, uint4* rec) {
-  Digest rt;  // the round's root is a tree digest (interleaved): its bytes
-  rt.lo = root_lo_bi;
-  rt.hi = root_hi_bi;
-  rt = digest_bytes(rt);
-  const uint4 root_lo = rt.lo, root_hi = rt.hi;
-  // Every lane computes the same scalars; the products are spread over the
-  // warp (gf_mul_warp2), two independent ones at a time.
-  const uint4 ONE = one_dev();
-  const uint4 r = scal[3 * i], r_inv = scal[3 * i + 1], corr = scal[3 * i + 2];
-  const uint4 claim = (i == d - 1) ? o.outer : o.inner;
+//
+// round_message: c0', c2' from S = sum_b half_eq[b] poly_lo[b] and the claim.
+// Every lane computes the same scalars; the products are spread over the warp
+// (gf_mul_warp2), two independent ones at a time.
+__device__ void round_message(OpenState& o, bool first, uint4 r, uint4 r_inv, uint4 corr, uint4 S, uint4& rp0,
+                              uint4& rp2) {
+  const uint4 claim = first ? o.outer : o.inner;
   const uint4 delta = o.delta;
-  const uint4 one_r = gf_add(ONE, r);
-  uint4 c0, d0, t, rp0, c1, rp2;
+  const uint4 one_r = gf_add(one_dev(), r);
+  uint4 c0, d0, t, c1;
   gf_mul_warp2(corr, S, delta, one_r, c0, d0);  // c0 = corr * S; d0 = delta (1 + r)
   gf_mul_warp2(one_r, c0, c0, d0, t, rp0);      // rp0 = c0 d0
   c1 = gf_add(gf_mul_warp(gf_add(claim, t), r_inv), c0);
   rp2 = gf_mul_warp(c1, delta);
   __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
+    o.c[0] = c0;
+    o.c[1] = c1;
+    o.c[2] = one_r;
+  }
+  __syncwarp();
+}
+
+// round_challenge: observes the root (a tree digest, interleaved) and the message,
+// samples o.x; `rec` (global, 16-byte aligned) receives root, c0', c2'.
+__device__ void round_challenge(const WarpKeccak& wk, OpenState& o, uint4 root_lo_bi, uint4 root_hi_bi, uint4 rp0,
+                                uint4 rp2, uint4* rec) {
   if (wk.lane == 0) {
-    rec[0] = root_lo;
-    rec[1] = root_hi;
+    Digest rt;
+    rt.lo = root_lo_bi;
+    rt.hi = root_hi_bi;
+    rt = digest_bytes(rt);
+    rec[0] = rt.lo;
+    rec[1] = rt.hi;
     rec[2] = rp0;
     rec[3] = rp2;
-    const uint4 m[4] = {root_lo, root_hi, rp0, rp2};
+    const uint4 m[4] = {rt.lo, rt.hi, rp0, rp2};
     tr_observe(o, m);  // root (basefold.rs:356), then [c0, c2] (sumcheck/src/lib.rs:97)
   }
-  uint4 x = warp_sample_elem(wk, o);  // valid on lane 0
-  x.x = __shfl_sync(0xffffffffu, x.x, 0);
-  x.y = __shfl_sync(0xffffffffu, x.y, 0);
-  x.z = __shfl_sync(0xffffffffu, x.z, 0);
-  x.w = __shfl_sync(0xffffffffu, x.w, 0);
+  const uint4 x = warp_sample_elem(wk, o);
+  if (wk.lane == 0) o.x = x;
+  __syncwarp();
+}
+
+// round_claim: the claim and delta after the challenge.
+__device__ void round_claim(OpenState& o) {
+  const uint4 x = o.x, delta = o.delta, c0 = o.c[0], c1 = o.c[1], one_r = o.c[2];
   uint4 c1x, delta_next;
   gf_mul_warp2(c1, x, delta, gf_add(one_r, x), c1x, delta_next);
-  if (wk.lane == 0) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
     o.inner = gf_add(c1x, c0);  // EvalProver::fix_last_var (eval.rs:108-111)
     o.delta = delta_next;
-    o.x = x;
   }
   __syncwarp();
 }
@@ -188,7 +202,7 @@ constexpr int kStateVecs = (int)(sizeof(OpenState) / sizeof(uint4));
 __device__ __forceinline__ void state_load(OpenState& sh, const OpenState* g) {
   const uint4* src = reinterpret_cast<const uint4*>(g);
   uint4* dst = reinterpret_cast<uint4*>(&sh);
-  for (int k = threadIdx.x; k < kStateVecs; k += blockDim.x) dst[k] = src[k];
+  for (int k = threadIdx.x; k < kStateVecs; k += blockDim.x) dst[k] = __ldcg(src + k);
 }
 __device__ __forceinline__ void state_store(OpenState* g, const OpenState& sh) {
   const uint4* src = reinterpret_cast<const uint4*>(&sh);
@@ -218,15 +232,26 @@ __global__ void __launch_bounds__(32) open_observe_kernel(OpenState* S, const ui
   state_store(S, sh);
 }
 
+// From the second round on, the launch before this one is a tree's, and a block of
+// this grid starts only after every block of that one has waited for all launches
+// before it: the state and the reduction S, which those wrote, are read (past L1)
+// and the message made before the wait, which is left for the root alone.  From the
+// tree's end to this kernel's end measured 3.9 us on GB300, 7.2 with everything after
+// the wait.
 __global__ void __launch_bounds__(32) open_round_kernel(OpenState* S, int i, int d, const uint4* scal,
                                                         const uint4* root, const uint4* Sred, uint8_t* rec) {
   __shared__ OpenState sh;
   const WarpKeccak wk;
-  chain_wait();
+  const bool first = i == d - 1;
+  if (first) chain_wait();
   state_load(sh, S);
-  __syncthreads();
-  round_step(wk, sh, i, d, scal, root[0], root[1], Sred[0], reinterpret_cast<uint4*>(rec));
-  __syncthreads();
+  __syncwarp();
+  if (!first) round_claim(sh);
+  uint4 rp0, rp2;
+  round_message(sh, first, __ldcg(scal + 3 * i), __ldcg(scal + 3 * i + 1), __ldcg(scal + 3 * i + 2), __ldcg(Sred), rp0,
+                rp2);
+  if (!first) chain_wait();
+  round_challenge(wk, sh, root[0], root[1], rp0, rp2, reinterpret_cast<uint4*>(rec));
   state_store(S, sh);
 }
 
@@ -235,13 +260,16 @@ __global__ void __launch_bounds__(32) open_round_kernel(OpenState* S, int i, int
 // levels in shared memory (a level read back from global memory costs an L2
 // round trip), hash each level in the form that is fastest for its count
 // (hash_level_block), and multiply by the twiddles, which need no challenge,
-// on warps 1..7 while warp 0 runs the transcript step: after the challenge a
-// fold output is one product.  Bound by the chain of dependent permutations
-// (one per level, leaf and transcript step).  Measured at 2^8 leaves and below,
-// GB300: 195 us for the last eight rounds, 262 us with one thread per
-// leaf, the codeword and the levels in global memory and both products after
-// the challenge.
-constexpr int kTailShared = 512;
+// on warps 1..7 while warp 0 samples the challenge: after it a fold output is one
+// product, and the next reduction is a + x b of two sums that are ready.  The claim
+// and the next round's message are made while the leaves are hashed, by a warp
+// that has no hash there.  Bound by the chain of dependent permutations
+// (one per level, leaf and transcript step).  Measured on GB300 for the last nine
+// rounds of an open (fold outputs from 2^9): 172 us, 191 with the message and the
+// claim between root and challenge and a second product in the next reduction;
+// with one thread per leaf and the codeword and levels in global memory, 262 for
+// the last eight.
+constexpr int kTailShared = 512, kTailPoly = 128;
 
 __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P) {
   static_assert(kTailThreads == kTreeThreads, "the tail hashes levels with hash_level_block");
@@ -249,16 +277,35 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
   __shared__ uint4 pi_a[2 * kTailShared], pi_b[kTailShared];  // (lo', hi' - lo') pairs of a fold's input
   __shared__ uint4 msg[kTailShared];                          // a fold's outputs as interleaved lanes
   __shared__ TreeShared ts;
-  __shared__ __align__(16) uint32_t sums[2][4];  // the round's reduction and the next one's
+  __shared__ uint4 poly_s[kTailPoly];            // the polynomial once it fits
+  __shared__ __align__(16) uint32_t sums[2][4];  // the next reduction is sums[0] + x sums[1]
+  __shared__ uint4 rp[2];                        // the round's message
   const int d = P.d;
   const size_t c = (size_t)1 << P.log2_c;
   const WarpKeccak wk;
   const int warp = threadIdx.x >> 5;
-  chain_wait();
+  const bool early = P.i0 >= 0 && P.i0 < d - 1;  // after launched rounds: see open_round_kernel
+  if (!early) chain_wait();
   state_load(sh, P.state);
-  if (threadIdx.x == 0 && P.i0 >= 0) *reinterpret_cast<uint4*>(sums[0]) = P.S_i0[0];
+  if (threadIdx.x < 8) sums[threadIdx.x >> 2][threadIdx.x & 3] = 0;
+  __syncthreads();
+  auto message = [&](int i, uint4 S) {  // one warp
+    uint4 rp0, rp2;
+    round_message(sh, i == d - 1, __ldcg(P.scal + 3 * i), __ldcg(P.scal + 3 * i + 1), __ldcg(P.scal + 3 * i + 2), S, rp0,
+                  rp2);
+    if (wk.lane == 0) {
+      rp[0] = rp0;
+      rp[1] = rp2;
+    }
+  };
+  if (warp == 0 && P.i0 >= 0) {
+    if (early) round_claim(sh);
+    message(P.i0, __ldcg(P.S_i0));
+  }
+  if (early) chain_wait();
   const uint4* root = P.root_i0;  // the round's tree root
   const uint4* pi_s = nullptr;    // the round's folded codeword in shared memory, if it is there
+  const uint4* poly = P.i0 == d - 1 ? P.poly_first : P.poly;
   __syncthreads();
   int k = 0;
   for (int i = P.i0; i >= 0; --i, ++k) {
@@ -270,12 +317,12 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
     const uint4* thi = P.tw->hi[d - 1 - i];
     uint4* pairs = pi_s == pi_b ? pi_b : pi_a;
     uint4* next = pairs == pi_a ? pi_b : pi_a;
-    // ---- transcript step (warp 0); meanwhile the other warps interpolate ----
+    const uint32_t half = 1u << i, next_half = half >> 1;
+    // ---- the challenge (warp 0); meanwhile the other warps interpolate and add up
+    //      sum heq lo and sum heq (hi + lo) over the next round's range ----
     if (warp == 0) {
-      round_step(wk, sh, i, d, P.scal, root[0], root[1], *reinterpret_cast<const uint4*>(sums[k & 1]),
-                 reinterpret_cast<uint4*>(P.result + 64 * (size_t)k));
+      round_challenge(wk, sh, root[0], root[1], rp[0], rp[1], reinterpret_cast<uint4*>(P.result + 64 * (size_t)k));
     } else {
-      if (threadIdx.x == 32) *reinterpret_cast<uint4*>(sums[(k + 1) & 1]) = make_uint4(0, 0, 0, 0);
       if (small) {
         const uint4* src = pi_s ? pi_s : pi_in;
         for (uint32_t t = threadIdx.x - 32; t < ni; t += blockDim.x - 32) {
@@ -284,6 +331,24 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
           const uint4 l = gf_add(lo, gf_mul(hi, tw));
           pairs[2 * t] = l;
           pairs[2 * t + 1] = gf_add(hi, l);
+        }
+      }
+      uint4 part[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+      for (uint32_t e = blockDim.x - 1 - threadIdx.x; e < 2 * next_half; e += blockDim.x - 32) {
+        const uint32_t q = e & 1u, b = e >> 1;
+        const uint4 lo = poly[b];
+        part[0] = gf_add(part[0], gf_mul(P.heq[b], q ? gf_add(poly[b + half], lo) : lo));
+      }
+      // a thread's items all have the parity of its first (the stride is even)
+      if ((threadIdx.x & 1u) == 0) {
+        part[1] = part[0];
+        part[0] = make_uint4(0, 0, 0, 0);
+      }
+      if (next_half) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          part[q] = warp_xor(part[q]);
+          if (wk.lane == 0) atomic_xor4(sums[q], part[q]);
         }
       }
     }
@@ -311,26 +376,41 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
         pi_out[t] = gf_add(lo, gf_mul(gf_add(hi, lo), x));
       }
     }
-    const uint4* poly_in = (i == d - 1) ? P.poly_first : P.poly;
-    const size_t half = (size_t)1 << i, next_half = i > 0 ? half / 2 : 0;
-    uint4 part = make_uint4(0, 0, 0, 0);
-    for (size_t b = blockDim.x - 1 - threadIdx.x; b < half; b += blockDim.x) {
-      const uint4 lo = poly_in[b], hi = poly_in[b + half];
-      const uint4 v = gf_add(lo, gf_mul(x, gf_add(hi, lo)));
-      P.poly[b] = v;
-      if (b < next_half) part = gf_add(part, gf_mul(P.heq[b], v));
+    uint4* fixed = half <= (uint32_t)kTailPoly ? poly_s : P.poly;
+    for (uint32_t b = blockDim.x - 1 - threadIdx.x; b < half; b += blockDim.x) {
+      const uint4 lo = poly[b], hi = poly[b + half];
+      fixed[b] = gf_add(lo, gf_mul(x, gf_add(hi, lo)));
     }
-    part = warp_xor(part);
-    if (wk.lane == 0) atomic_xor4(sums[(k + 1) & 1], part);
+    poly = fixed;
     __syncthreads();
     // ---- the next round's leaves and Merkle tree ----
     if (i > 0) {
       size_t n = ni / 2;
+      auto next_message = [&] {  // by the last warp, which hashes nothing unless 8 or 256 hashes are due
+        if (warp != kTailThreads / 32 - 1) return;
+        round_claim(sh);
+        uint4* a = reinterpret_cast<uint4*>(sums);
+        const uint4 S = gf_add(a[0], gf_mul_warp(a[1], x));
+        __syncwarp();
+        if (wk.lane < 2) a[wk.lane] = make_uint4(0, 0, 0, 0);
+        message(i - 1, S);
+      };
       if (small) {
+        int levels = P.log2_c + i - 1;
+        const bool busy = n == 8 || n == 256;
+        if (!busy) next_message();
         hash_level_block<4>(wk, msg, 1, (uint32_t)n, ts.a, leaves, 1);
         __syncthreads();
-        root = tree_block(wk, ts.b, ts.a, ts.a, 1, leaves + 2 * n, n, 0, P.log2_c + i - 1);
+        if (!busy) {
+          root = tree_block(wk, ts.b, ts.a, ts.a, 1, leaves + 2 * n, n, 0, levels);
+        } else {
+          next_message();
+          hash_level_block<8>(wk, ts.a, 1, (uint32_t)n / 2, ts.b, leaves + 2 * n, 1);
+          __syncthreads();
+          root = tree_block(wk, ts.a, ts.b, ts.b, 1, leaves + 3 * n, n / 2, 0, levels - 1);
+        }
       } else {
+        next_message();
         for (size_t s = threadIdx.x; s < n; s += blockDim.x)
           store_digest(leaves, s, hash_pair(pi_out[2 * s], pi_out[2 * s + 1]));
         __syncthreads();
@@ -350,7 +430,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) open_tail_kernel(TailParams P
   }
   // ---- final polynomial (basefold.rs:196) ----
   if (threadIdx.x == 0) {
-    const uint4 fin = (k == 0) ? P.poly_first[0] : P.poly[0];
+    const uint4 fin = poly[0];
     reinterpret_cast<uint4*>(P.result + 64 * (size_t)k)[0] = fin;
     const uint4 m[1] = {fin};
     tr_observe(sh, m);
@@ -374,10 +454,8 @@ namespace {
 // launch_sumcheck_round): the sums c0, c2, c3 are the same in every lane.
 __device__ __forceinline__ void sumcheck_step(const WarpKeccak& wk, OpenState& sh, int k, uint4 c0, uint4 c2, uint4 c3,
                                               uint8_t* rec) {
-  const uint4 sc = sh.outer;
-  // k = 2: compressed [c0, c2] (the pair scalar is ONE, quadratic.rs:118),
-  // round polynomial [c0, sc - 2 c0 - c2 = sc + c2, c2]; k = 3: compressed
-  // [c0, c2, c3], round polynomial [c0, sc + c2 + c3, c2, c3]
+  // k = 2: compressed [c0, c2] (the pair scalar is ONE, quadratic.rs:118); k = 3:
+  // [c0, c2, c3]
   if (wk.lane == 0) {
     uint4* r = reinterpret_cast<uint4*>(rec);
     r[0] = c0;
@@ -391,22 +469,30 @@ __device__ __forceinline__ void sumcheck_step(const WarpKeccak& wk, OpenState& s
       tr_observe(sh, m);
     }
   }
-  uint4 x = warp_sample_elem(wk, sh);  // valid on lane 0
-  x.x = __shfl_sync(0xffffffffu, x.x, 0);
-  x.y = __shfl_sync(0xffffffffu, x.y, 0);
-  x.z = __shfl_sync(0xffffffffu, x.z, 0);
-  x.w = __shfl_sync(0xffffffffu, x.w, 0);
-  // horner over the round polynomial at x
+  const uint4 x = warp_sample_elem(wk, sh);  // valid on lane 0
+  if (wk.lane == 0) {
+    reinterpret_cast<uint4*>(rec)[k] = x;
+    sh.x = x;
+    sh.c[0] = c0;
+    sh.c[1] = c2;
+    sh.c[2] = c3;
+  }
+  __syncwarp();
+}
+
+// The claim after the challenge: horner over the round polynomial at x.  The message
+// does not need it, so this is left to the next step (one warp).
+__device__ __forceinline__ void sumcheck_claim(OpenState& sh, int k) {
+  // k = 2: round polynomial [c0, sc - 2 c0 - c2 = sc + c2, c2]; k = 3: [c0, sc + c2 +
+  // c3, c2, c3]
+  const uint4 sc = sh.outer, x = sh.x, c0 = sh.c[0], c2 = sh.c[1], c3 = sh.c[2];
   const uint4 c1 = (k == 3) ? gf_add(sc, gf_add(c2, c3)) : gf_add(sc, c2);
   uint4 acc_h = (k == 3) ? c3 : c2;
   if (k == 3) acc_h = gf_add(gf_mul_warp(acc_h, x), c2);
   acc_h = gf_add(gf_mul_warp(acc_h, x), c1);
   acc_h = gf_add(gf_mul_warp(acc_h, x), c0);
-  if (wk.lane == 0) {
-    reinterpret_cast<uint4*>(rec)[k] = x;
-    sh.outer = acc_h;
-    sh.x = x;
-  }
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) sh.outer = acc_h;
   __syncwarp();
 }
 
@@ -414,12 +500,20 @@ __device__ __forceinline__ void sumcheck_step(const WarpKeccak& wk, OpenState& s
 
 // Product sumcheck round (warp): c = [c0, c2, c3] from the device sums, which
 // it clears for the fix that accumulates the next round's.
-__global__ void __launch_bounds__(32) sumcheck_round_kernel(OpenState* S, int k, uint32_t* acc, uint8_t* rec) {
+// After the first round the launch before this one is a fix's, whose blocks wait for
+// the round's before it: the state is read, and its claim brought up to date, before
+// the wait (see open_round_kernel).
+__global__ void __launch_bounds__(32) sumcheck_round_kernel(OpenState* S, int k, bool first, uint32_t* acc,
+                                                            uint8_t* rec) {
   __shared__ OpenState sh;
   const WarpKeccak wk;
-  chain_wait();
+  if (first) chain_wait();
   state_load(sh, S);
-  __syncthreads();
+  __syncwarp();
+  if (!first) {
+    sumcheck_claim(sh, k);
+    chain_wait();
+  }
   uint4* a = reinterpret_cast<uint4*>(acc);
   const uint4 c0 = a[0], c2 = a[1], c3 = a[2];
   __syncwarp();
@@ -445,8 +539,13 @@ __global__ void __launch_bounds__(kTailThreads, 1) sumcheck_tail_kernel(Sumcheck
   __shared__ __align__(16) uint32_t sums[2][12];       // this round's c0, c2, c3 and the next one's
   const WarpKeccak wk;
   const uint32_t tid = threadIdx.x;
-  chain_wait();
+  if (p.first) chain_wait();
   state_load(sh, p.state);
+  __syncthreads();
+  if (!p.first) {
+    if (tid < 32) sumcheck_claim(sh, K);
+    chain_wait();
+  }
   if (tid < 12) sums[0][tid] = p.acc[tid];
   __syncthreads();
   // item i of a round's terms adds v to coefficient q; a warp whose items all
@@ -471,6 +570,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) sumcheck_tail_kernel(Sumcheck
     }
     __syncthreads();
     const uint4 x = sh.x;
+    if (tid >= kTailThreads - 32) sumcheck_claim(sh, K);  // the warp with the fewest outputs
     // fix: output b of polynomial j
     uint4 out[(K * kMax + kTailThreads - 1) / kTailThreads];
 #pragma unroll
@@ -529,9 +629,9 @@ cudaError_t launch_sumcheck_tail(const SumcheckTail& p, int k, cudaStream_t st) 
   return e;
 }
 
-cudaError_t launch_sumcheck_round(OpenState* s, int k, uint32_t* acc, uint8_t* rec, cudaStream_t st) {
+cudaError_t launch_sumcheck_round(OpenState* s, int k, bool first, uint32_t* acc, uint8_t* rec, cudaStream_t st) {
   if (k != 2 && k != 3) return cudaErrorInvalidValue;
-  const cudaError_t e = launch_chained(sumcheck_round_kernel, 1, 32, 0, st, s, k, acc, rec);
+  const cudaError_t e = launch_chained(sumcheck_round_kernel, 1, 32, 0, st, s, k, first, acc, rec);
   count_launch();
   return e;
 }

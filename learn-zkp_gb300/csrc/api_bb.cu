@@ -606,6 +606,8 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
         CU(cudaStreamWaitEvent(st, p->ev_dot, 0));
       }
       bf::BbTail tp{};
+      tp.early = fixed_here;
+      tp.first = k == 0;
       tp.i0 = i;
       tp.lk = lk;
       tp.log2_n0 = p->log2_n0();
@@ -641,7 +643,8 @@ int bf_bb_open(bf_bb_pcs* p, const bf_bb_commitment* cm, const uint8_t* point, c
       CU(cudaStreamWaitEvent(st, p->ev_dot, 0));
     }
     uint32_t* x_k = xs_dev + 5 * (size_t)k;
-    CU(bf::bb_launch_transcript_round(tdev, cdev, ri, root_dev, acc, base_k, x_k, rec_dev + 72 * (size_t)k, st));
+    CU(bf::bb_launch_transcript_round(tdev, cdev, ri, root_dev, acc, base_k, x_k, rec_dev + 72 * (size_t)k, k == 0,
+                                       fixed_here, st));
     const bb::E5 unused{};
     uint32_t* fixed = fixbuf[k & 1];  // the fix two rounds back and the sums since have read it (stream order)
     fixed_here = i > 0 && bf::bb_fold_takes_fix(ni);

@@ -108,6 +108,9 @@ struct alignas(8) BbTranscript {
   uint32_t pend_len, out_len;
   bb::E5 claim;         // the open's claim in the first round, then EvalImprProver's inner subclaim value
   bb::E5 delta;         // the delta factor eq_eval(r[ri+1 ..], challenges so far) (eval_impr.rs:45-51); 1 at the start
+  // what the last round's claim update needs (c0 + c1 X at x, r); that update is
+  // left to the next step, so claim and delta are those before it
+  bb::E5 c0, c1, r, x;
 };
 // Per sumcheck round ri (< num_vars): the point coordinate, its inverse and
 // the correcting factor prod_{k >= ri} (1 - r_k)^-1 (eval_impr.rs:83-90).
@@ -119,10 +122,12 @@ struct alignas(8) BbRoundConsts {
 // round polynomial from the GPU sum (Montgomery sums, or canonical ones when
 // `canonical`), observe its compressed form, sample the challenge into x_out
 // (Montgomery) and record the root and the compressed polynomial (72 canonical
-// bytes) at rec.
+// bytes) at rec.  first: no round was launched before; early: the sums come from a
+// launch before the tree's, so everything but the root may be read before that
+// one has ended.
 cudaError_t bb_launch_transcript_round(BbTranscript* t, const BbRoundConsts* c, int ri, const uint4* root_dev,
                                        unsigned long long* sums, int canonical, uint32_t* x_out, uint8_t* rec,
-                                       cudaStream_t st);
+                                       bool first, bool early, cudaStream_t st);
 
 // The last rounds i0 .. 0 of an open in one block: the rounds whose fold has
 // n_i <= kBbTailMax outputs.  The tree of round i0 is built before (its root
@@ -130,6 +135,7 @@ cudaError_t bb_launch_transcript_round(BbTranscript* t, const BbRoundConsts* c, 
 // `fold_out`, one after another.
 constexpr int kBbTailMax = 256;
 struct BbTail {
+  bool first, early;       // as bb_launch_transcript_round's
   int i0, lk, log2_n0;     // n_i = 2^(log2_n0 + i); the sumcheck round of round i is i + lk
   const uint32_t* pi;      // 2 n_i0 entries: extension, or base-field Montgomery when pi_base
   int pi_base;

@@ -59,7 +59,6 @@ struct ELane {
 struct BbStepShared {
   BbTranscript t;
   uint32_t msg[18];
-  uint32_t x[5];  // out: the challenge
 };
 
 // keccak256's last block: the first `len` < 136 bytes at `p` (8-byte aligned)
@@ -79,25 +78,21 @@ __device__ __forceinline__ uint2 padded_word(const WarpKeccak& wk, const uint8_t
   return w;
 }
 
-// S: this lane's coefficient of the round's sum (Montgomery, the same in every
-// group).  Bound by two chains: four extension products before the message and
-// the permutation; every load of the round's constants is issued at the start.
-// One lane doing the products one after another, with the delta factor
-// rebuilt from all challenges and the challenge popped byte by byte, took
-// 20.9 us per launch at 2^13 rows on GB300 (device time); this form takes 7.9 us.
-__device__ __forceinline__ void bb_round_step(const WarpKeccak& wk, BbStepShared& sh, const BbRoundConsts* c, int ri,
-                                              const uint4* root, uint32_t S, uint8_t* rec) {
+// The step in three parts, each by one warp, so that only the challenge stands
+// between a round's root and its fold.  From the tree's end to the step's end it
+// measured 4.0 us on GB300, 5.3 with all three after the root, 20.9 with one lane
+// doing the products one after another, the delta factor rebuilt from all challenges
+// and the challenge popped byte by byte.
+//
+// bb_message: the round polynomial from S, this lane's coefficient of the round's
+// sum (Montgomery, the same in every group).
+__device__ __forceinline__ void bb_message(BbStepShared& sh, const BbRoundConsts* c, int ri, uint32_t S) {
   const ELane el;
-  const int lane = wk.lane, k = el.k, g = el.group();
+  const int lane = threadIdx.x & 31, k = el.k, g = el.group();
   BbTranscript& t = sh.t;
-  const uint32_t cf = c->cf[ri].c[k], rinv = c->r_inv[ri].c[k], r = c->r[ri].c[k];
-  const uint32_t one = el.one(), omr = bb::sub(one, r);
+  const uint32_t cf = __ldcg(&c->cf[ri].c[k]), rinv = __ldcg(&c->r_inv[ri].c[k]), r = __ldcg(&c->r[ri].c[k]);
+  const uint32_t omr = bb::sub(el.one(), r);
   const uint32_t claim = t.claim.c[k], delta = t.delta.c[k];
-  if (lane >= 28) {  // the root's 32 bytes
-    const uint2 v = bi_to_lane(reinterpret_cast<const uint2*>(root)[lane - 28]);
-    sh.msg[2 * (lane - 28)] = v.x;
-    sh.msg[2 * (lane - 28) + 1] = v.y;
-  }
   // c0 = cf S, c1 = (claim - (1 - r) c0) / r - c0; the round polynomial is
   // (c0 + c1 X)(d0 + d1 X) with d0 = delta (1 - r), d1 = delta (2 r - 1)
   const uint32_t m1 = el.mul(g == 0 ? cf : delta, g == 0 ? S : g == 1 ? omr : bb::sub(r, omr));
@@ -106,8 +101,46 @@ __device__ __forceinline__ void bb_round_step(const WarpKeccak& wk, BbStepShared
   const uint32_t rp0 = el.from(m2, 1);
   const uint32_t c1 = bb::sub(el.mul(bb::sub(claim, el.from(m2, 0)), rinv), c0);
   const uint32_t rp2 = el.mul(c1, d1);
-  if (lane < 5) sh.msg[8 + lane] = bb::from_mont(rp0);  // Eval::compress_round_poly keeps c0 and c2
-  else if (lane < 10) sh.msg[13 + k] = bb::from_mont(rp2);
+  if (lane < 5) {
+    sh.msg[8 + lane] = bb::from_mont(rp0);  // Eval::compress_round_poly keeps c0 and c2
+    t.c0.c[k] = c0;
+    t.c1.c[k] = c1;
+    t.r.c[k] = r;
+  } else if (lane < 10) {
+    sh.msg[13 + k] = bb::from_mont(rp2);
+  }
+  __syncwarp();
+}
+
+// bb_claim: EvalProver's claim c0 + c1 x (eval.rs:108-111) and the next delta:
+// delta (2 r x + 1 - r - x) (multilinear.rs:224-229).
+__device__ __forceinline__ void bb_claim(BbStepShared& sh) {
+  const ELane el;
+  const int lane = threadIdx.x & 31, k = el.k, g = el.group();
+  BbTranscript& t = sh.t;
+  const uint32_t r = t.r.c[k], x = t.x.c[k], c0 = t.c0.c[k], delta = t.delta.c[k];
+  const uint32_t m = el.mul(g == 0 ? t.c1.c[k] : r, x);
+  const uint32_t rx = el.from(m, 1);
+  const uint32_t f = bb::sub(bb::sub(bb::add(bb::add(rx, rx), el.one()), r), x);
+  const uint32_t nd = el.mul(delta, f);
+  __syncwarp();
+  if (lane < 5) {
+    t.claim.c[k] = bb::add(c0, m);
+    t.delta.c[k] = nd;
+  }
+  __syncwarp();
+}
+
+// bb_challenge: observes the root and the message, samples t.x.
+__device__ __forceinline__ void bb_challenge(const WarpKeccak& wk, BbStepShared& sh, const uint4* root, uint8_t* rec) {
+  const ELane el;
+  const int lane = wk.lane, k = el.k;
+  BbTranscript& t = sh.t;
+  if (lane >= 28) {  // the root's 32 bytes
+    const uint2 v = bi_to_lane(reinterpret_cast<const uint2*>(root)[lane - 28]);
+    sh.msg[2 * (lane - 28)] = v.x;
+    sh.msg[2 * (lane - 28) + 1] = v.y;
+  }
   __syncwarp();
   // observe the root and the polynomial (challenger.rs:51-60): appended to the
   // pending input, whole blocks absorbed, the output cleared
@@ -163,17 +196,7 @@ __device__ __forceinline__ void bb_round_step(const WarpKeccak& wk, BbStepShared
     if (lane == 16) a.y = 0x80000000u;
     a = wk.permute<false>(a);
   }
-  // EvalProver's claim c0 + c1 x (eval.rs:108-111) and the next delta:
-  // delta (2 r x + 1 - r - x) (multilinear.rs:224-229)
-  const uint32_t m5 = el.mul(g == 0 ? c1 : r, x);
-  const uint32_t rx = el.from(m5, 1);
-  const uint32_t f = bb::sub(bb::sub(bb::add(bb::add(rx, rx), one), r), x);
-  const uint32_t nd = el.mul(delta, f);
-  if (lane < 5) {
-    t.claim.c[k] = bb::add(c0, m5);
-    t.delta.c[k] = nd;
-    sh.x[k] = x;
-  }
+  if (lane < 5) t.x.c[k] = x;
   if (lane < 4) {
     reinterpret_cast<uint2*>(t.pend)[lane] = a;
     reinterpret_cast<uint2*>(t.out)[lane] = a;
@@ -191,6 +214,10 @@ __device__ __forceinline__ void tr_copy(BbTranscript* dst, const BbTranscript* s
   for (int q = threadIdx.x; q < kTrWords; q += blockDim.x)
     reinterpret_cast<uint2*>(dst)[q] = reinterpret_cast<const uint2*>(src)[q];
 }
+__device__ __forceinline__ void tr_load(BbTranscript* dst, const BbTranscript* src) {  // past L1
+  for (int q = threadIdx.x; q < kTrWords; q += blockDim.x)
+    reinterpret_cast<uint2*>(dst)[q] = __ldcg(reinterpret_cast<const uint2*>(src) + q);
+}
 
 __device__ __forceinline__ E5 ld_e5(const uint32_t* p, size_t i) {
   E5 e;
@@ -205,31 +232,40 @@ __device__ __forceinline__ void st_e5(uint32_t* p, size_t i, const E5& e) {
 
 }  // namespace
 
+// early: the launch before this one is a tree's, and a block of this grid starts
+// only after every block of that one has waited for all launches before it, among
+// them the ones that wrote the transcript and the sums: those are read (past L1) and
+// the message is made before the wait, which is left for the root alone.
 __global__ void __launch_bounds__(32) bb_transcript_round_kernel(BbTranscript* t, const BbRoundConsts* c, int ri,
                                                                 const uint4* root_dev, unsigned long long* sums,
-                                                                int canonical, uint32_t* x_out, uint8_t* rec) {
+                                                                int canonical, uint32_t* x_out, uint8_t* rec,
+                                                                bool first, bool early) {
   __shared__ BbStepShared sh;
   const WarpKeccak wk;
-  chain_wait();
-  tr_copy(&sh.t, t);
-  const uint32_t v = (uint32_t)(sums[threadIdx.x % 5] % bb::P);
+  if (!early) chain_wait();
+  tr_load(&sh.t, t);
+  const uint32_t v = (uint32_t)(__ldcg(sums + threadIdx.x % 5) % bb::P);
   __syncwarp();
+  if (!first) bb_claim(sh);
+  bb_message(sh, c, ri, canonical ? bb::to_mont(v) : v);
+  if (early) chain_wait();
   if (threadIdx.x < 5) sums[threadIdx.x] = 0;  // for the fix that adds up the next round's
-  bb_round_step(wk, sh, c, ri, root_dev, canonical ? bb::to_mont(v) : v, rec);
-  if (threadIdx.x < 5) x_out[threadIdx.x] = sh.x[threadIdx.x];
+  bb_challenge(wk, sh, root_dev, rec);
+  if (threadIdx.x < 5) x_out[threadIdx.x] = sh.t.x.c[threadIdx.x];
   tr_copy(t, &sh.t);
 }
 
 // The last rounds in one block of eight warps, everything but the outputs in
-// shared memory.  While warp 0 runs the transcript step the others interpolate:
+// shared memory.  While warp 0 samples the challenge the others interpolate:
 // l = (lo + hi) / 2 and h - l with h = (lo - hi) t need no challenge, so a fold
-// output is one product after it.  Each level of hashes runs in the form that is
-// fastest for its count (hash_level_block).  Bound by the chain of dependent
-// permutations (one per level, leaf and transcript step); a round took a
-// launch each for fold, fix, sums, transcript and two for the tree before.
-// Measured on GB300: 143 us for the last eight rounds of a 2^13 x 5 open,
-// whose commit, evaluation and open take 916 us (1,127 with a launch per step
-// and the transcript step on one lane).
+// output is one product after it.  The claim and the next round's message are made
+// while the leaves are hashed, by a warp that has no hash there.  Each level of
+// hashes runs in the form that is fastest for its count (hash_level_block).  Bound by
+// the chain of dependent permutations (one per level, leaf and challenge); a round
+// took a launch each for fold, fix, sums, transcript and two for the tree before.
+// Measured on GB300: 127 us for the last eight rounds of a 2^13 x 5 open (131 with
+// claim and message between root and challenge), whose commit, evaluation and open
+// took 1,127 us with a launch per step and 916 with this kernel alone.
 __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
   __shared__ BbStepShared sh;
   __shared__ uint32_t pi_a[2 * kBbTailMax * 5], pi_b[kBbTailMax * 5];  // l, then h - l of a fold's input
@@ -239,8 +275,8 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
   __shared__ unsigned long long sums[2][5];  // this round's sum and the next one's
   const WarpKeccak wk;
   const int warp = threadIdx.x >> 5;
-  chain_wait();
-  tr_copy(&sh.t, p.t);
+  if (!p.early) chain_wait();
+  tr_load(&sh.t, p.t);
   if (threadIdx.x < 10) sums[threadIdx.x / 5][threadIdx.x % 5] = 0;
   __syncthreads();
   // sum over the block of h[b] v for the thread's b, into acc (Montgomery sums)
@@ -254,15 +290,25 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
     }
   };
   auto ld_poly = [&](size_t b) {  // the polynomial before the first fix
-    return p.poly_base ? bb::e_from(bb::to_mont(p.poly[b])) : ld_e5(p.poly, b);
+    if (p.poly_base) return bb::e_from(bb::to_mont(p.poly[b]));
+    E5 e;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) e.c[q] = __ldcg(p.poly + 5 * b + q);
+    return e;
   };
-  {  // round i0's sum
+  {  // round i0's sum, as early as the transcript round's
     const size_t n = (size_t)1 << (p.i0 + p.lk);
     E5 part = bb::e_zero();
     for (size_t b = threadIdx.x; b < n; b += kTreeThreads)
       part = bb::e_add(part, bb::e_mul(ld_e5(p.heq, b), ld_poly(b)));
     add_sums(part, sums[0]);
   }
+  __syncthreads();
+  if (warp == 0) {
+    if (!p.first) bb_claim(sh);
+    bb_message(sh, p.c, p.i0 + p.lk, (uint32_t)(sums[0][wk.lane % 5] % bb::P));
+  }
+  if (p.early) chain_wait();
   __syncthreads();
   const uint4* root = p.root;
   const uint32_t* pi_s = nullptr;  // the round's folded codeword in shared memory, after round i0
@@ -273,8 +319,7 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
     uint32_t* pairs = pi_s == pi_b ? pi_b : pi_a;
     uint32_t* next = pairs == pi_a ? pi_b : pi_a;
     if (warp == 0) {
-      bb_round_step(wk, sh, p.c, i + p.lk, root, (uint32_t)(sums[it & 1][wk.lane % 5] % bb::P),
-                    p.rec + 72 * (size_t)it);
+      bb_challenge(wk, sh, root, p.rec + 72 * (size_t)it);
     } else {
       if (threadIdx.x >= 32 && threadIdx.x < 37) sums[(it + 1) & 1][threadIdx.x - 32] = 0;
       const uint32_t* tinv = p.tinv + (((size_t)1 << (p.log2_n0 + i)) - ((size_t)1 << p.log2_n0));
@@ -294,7 +339,7 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
       }
     }
     __syncthreads();
-    const E5 x = ld_e5(sh.x, 0);
+    const E5 x = sh.t.x;
     // fold from the first thread up: row s of the next round's matrix is (out[s], out[s + n/2])
     const uint32_t rows = n > 1 ? n / 2 : 1;
     const int bits = p.log2_n0 + i - 1;
@@ -331,9 +376,25 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
     pi_s = next;
     if (i > 0) {
       const uint32_t leaves = n / 2;
+      // the claim and the next message by the last warp, which has no leaf to hash
+      // unless there are eight of them
+      auto next_message = [&] {
+        if (warp != kTreeThreads / 32 - 1) return;
+        bb_claim(sh);
+        bb_message(sh, p.c, i - 1 + p.lk, (uint32_t)(sums[(it + 1) & 1][wk.lane % 5] % bb::P));
+      };
+      const bool busy = leaves == 8;
+      if (!busy) next_message();
       hash_level_block<5>(wk, reinterpret_cast<const uint4*>(msg), 1, leaves, ts.a, tree, 1);
       __syncthreads();
-      root = tree_block(wk, ts.b, ts.a, ts.a, 1, tree + 2 * (size_t)leaves, leaves, 0, bits);
+      if (!busy) {
+        root = tree_block(wk, ts.b, ts.a, ts.a, 1, tree + 2 * (size_t)leaves, leaves, 0, bits);
+      } else {
+        next_message();
+        hash_level_block<8>(wk, ts.a, 1, leaves / 2, ts.b, tree + 2 * (size_t)leaves, 1);
+        __syncthreads();
+        root = tree_block(wk, ts.a, ts.b, ts.b, 1, tree + 3 * (size_t)leaves, leaves / 2, 0, bits - 1);
+      }
       tree += 2 * (size_t)(2 * leaves);
     }
   }
@@ -343,9 +404,9 @@ __global__ void __launch_bounds__(kTreeThreads, 1) bb_tail_kernel(BbTail p) {
 
 cudaError_t bb_launch_transcript_round(BbTranscript* t, const BbRoundConsts* c, int ri, const uint4* root_dev,
                                        unsigned long long* sums, int canonical, uint32_t* x_out, uint8_t* rec,
-                                       cudaStream_t st) {
+                                       bool first, bool early, cudaStream_t st) {
   const cudaError_t e =
-      launch_chained(bb_transcript_round_kernel, 1, 32, 0, st, t, c, ri, root_dev, sums, canonical, x_out, rec);
+      launch_chained(bb_transcript_round_kernel, 1, 32, 0, st, t, c, ri, root_dev, sums, canonical, x_out, rec, first, early);
   count_launch();
   return e;
 }

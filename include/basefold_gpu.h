@@ -169,13 +169,16 @@ void bf_open_session_free(bf_open_session* s);
  * A pcs's launch shapes are six integers: threads per block of the
  * shared-memory NTT pass (128, 256, 512), butterfly layers per NTT pass
  * (6..12, a tile of 2^T elements: the NTT radix per pass), the largest
- * Merkle level run by the single-block top kernel (64..4096, a power of
- * two), the single-block open tail (rounds whose next tree has
- * <= 2^tail_log leaves, 1..11), the Merkle levels per launch (levels of
- * 2^10 .. 2^subtree_log nodes run as one launch, 10..20), and the NTT pass
+ * Merkle level that the tree's last launch starts from (64..4096, a power of
+ * two; one block up to 128 nodes, a cluster of eight above), the single-block
+ * open tail (rounds whose next tree has <= 2^tail_log leaves, 1..11), the
+ * Merkle levels per launch (from 2^subtree_log nodes down up to nine levels
+ * run as one launch, 10..20), and the NTT pass
  * kind (0: layer by layer in shared memory; 1: tiles of 2^9..2^13 elements
  * register-blocked; 2: as 0 with the last pass and its leaf hashing
- * warp-specialized, butterfly warps and hashing warps on two tile buffers;
+ * warp-specialized, butterfly warps and hashing warps on two tile buffers,
+ * and, for large codewords, the leading layers two per pass over columns with
+ * tables of the twiddles;
  * 3: as 0 with the cosets of a two-pass encode pipelined, the next cosets'
  * first pass on a high-priority stream beside a coset's last pass).
  * They change how work is launched, never the proof bytes.  bf_pcs_autotune times `reps` whole proofs (commit + eval + open)

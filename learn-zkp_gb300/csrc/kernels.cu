@@ -588,8 +588,8 @@ __global__ void __launch_bounds__(kQuadTabThreads, 1) ntt_quad_tab_kernel(const 
 // one block's build runs beside the others' products.  The two products by t come
 // from a small table (64 KB, 4-bit groups), the two others from the multiplier with
 // their factors split beforehand (gf_prepare; 80 registers a thread, 670 us below
-// against 809 with the factors in registers and spills, 762 at two blocks).  Bound
-// by the ALU pipe.  Measured on GB300, a pass of 2^25 elements with 256 columns
+// against 809 with the factors in registers and spills, 762 at two blocks).  Held by
+// the ALU (62% busy), shared memory (57%) and the wide multiplier together.  Measured on GB300, a pass of 2^25 elements with 256 columns
 // per group: 670 us, 800 multiplied; with 1024: 460, 525 with the large tables.
 constexpr int kQuadMixThreads = 256, kQuadMixBlocks = 3;
 using QuadTabM = GfTab<8>;

@@ -35,6 +35,10 @@ __host__ __device__ __forceinline__ uint32_t sub(uint32_t a, uint32_t b) {
   const uint32_t d = a - b;
   return umin(d, d + P);
 }
+// a + b and a - b mod p for a, b < p, left below 2p (2p < 2^32): what mul_shoup, which
+// takes any 32-bit word, multiplies next.
+__host__ __device__ __forceinline__ uint32_t add_lazy(uint32_t a, uint32_t b) { return a + b; }
+__host__ __device__ __forceinline__ uint32_t sub_lazy(uint32_t a, uint32_t b) { return a - b + P; }
 // Montgomery product a b R^-1 mod p of a, b < p (R = 2^32): with t = a b and
 // m = t p^-1 mod R, m p has the low word of t, so (t - m p) / R is
 // hi(t) - hi(m p), in (-p, p); a negative difference wraps and gets p added.

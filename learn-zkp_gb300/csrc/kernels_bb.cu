@@ -352,6 +352,20 @@ __global__ void __launch_bounds__(256) bb_dft_pass_kernel(const uint32_t* __rest
   bb_tile_store(tile, cw, p, tl);
 }
 
+// The sum and difference of a register group's butterfly at layer l.  Outputs that
+// layer l + 1 of the group multiplies (bit l + 1 of their index) stay below 2p:
+// four of a butterfly's 19 instructions less for half of the butterflies.
+template <int R>
+__device__ __forceinline__ void bb_butterfly(uint32_t (&v)[1 << R], int l, int j0, int j1, uint32_t x0, uint32_t x1) {
+  if (l + 1 < R && (j0 & (2 << l))) {
+    v[j0] = bb::add_lazy(x0, x1);
+    v[j1] = bb::sub_lazy(x0, x1);
+  } else {
+    v[j0] = bb::add(x0, x1);
+    v[j1] = bb::sub(x0, x1);
+  }
+}
+
 // Register-blocked form of the same pass for tiles whose (u, column) slots
 // fill a warp (lu + lc = 5): lane = slot, and a warp takes 2^R rows of its
 // slots into registers and runs R layers there per round trip through
@@ -381,8 +395,7 @@ __device__ __forceinline__ void bb_reg_group(uint32_t* tile, uint32_t q, int l0,
       if (j0 & (1 << l)) continue;
       const int j1 = j0 | (1 << l);
       const uint32_t x1 = bb::mul_shoup(v[j1], tf[j0 & ((1 << l) - 1)]), x0 = v[j0];
-      v[j0] = bb::add(x0, x1);
-      v[j1] = bb::sub(x0, x1);
+      bb_butterfly<R>(v, l, j0, j1, x0, x1);
     }
   }
 #pragma unroll
@@ -435,10 +448,11 @@ __host__ __device__ constexpr int bb_wide_group(int T, int l0) {  // layers of t
 }
 
 // One register group: layers L0 .. L0 + R - 1 of the tile.  Warp q of the
-// 2^(T - R) groups takes rows a_base | j 2^L0 (j < 2^R) into registers.
-template <int T, int L0, int R>
+// 2^(T - R) groups takes rows a_base | j 2^L0 (j < 2^R) into registers.  The first
+// `zero` layers of a first pass were done by its load.
+template <int T, int L0, int R, int FIRST>
 __device__ __forceinline__ void bb_wide_layers(uint32_t* tile, int s_lo, uint32_t u, uint32_t lane, uint32_t warp,
-                                               const uint2* __restrict__ tw) {
+                                               const uint2* __restrict__ tw, int zero) {
   constexpr uint32_t kWork = 1u << (T - R);
   constexpr uint32_t kIters = kWork >= 8 ? kWork / 8 : 1;
 #pragma unroll
@@ -457,6 +471,8 @@ __device__ __forceinline__ void bb_wide_layers(uint32_t* tile, int s_lo, uint32_
     const uint32_t step = 1u << (L0 + s_lo);
 #pragma unroll
     for (int l = 0; l < R; ++l) {
+      if (FIRST == 1 && L0 + l < 1) continue;
+      if (FIRST == 2 && L0 + l < zero) continue;
       const uint2* tl = tq + ((1u << (s_lo + L0 + l)) - 1u);
       uint2 tf[1 << (R - 1)];
 #pragma unroll
@@ -466,8 +482,7 @@ __device__ __forceinline__ void bb_wide_layers(uint32_t* tile, int s_lo, uint32_
         if (j0 & (1 << l)) continue;
         const int j1 = j0 | (1 << l);
         const uint32_t x1 = bb::mul_shoup(v[j1], tf[j0 & ((1 << l) - 1)]), x0 = v[j0];
-        v[j0] = bb::add(x0, x1);
-        v[j1] = bb::sub(x0, x1);
+        bb_butterfly<R>(v, l, j0, j1, x0, x1);
       }
     }
 #pragma unroll
@@ -475,22 +490,28 @@ __device__ __forceinline__ void bb_wide_layers(uint32_t* tile, int s_lo, uint32_
   }
 }
 
-template <int T, int L0>
+template <int T, int L0, int FIRST>
 struct BbWideGroups {
   static __device__ __forceinline__ void run(uint32_t* tile, int s_lo, uint32_t u, uint32_t lane, uint32_t warp,
-                                             const uint2* __restrict__ tw) {
+                                             const uint2* __restrict__ tw, int zero) {
     constexpr int R = bb_wide_group(T, L0);
-    bb_wide_layers<T, L0, R>(tile, s_lo, u, lane, warp, tw);
+    bb_wide_layers<T, L0, R, FIRST>(tile, s_lo, u, lane, warp, tw, zero);
     __syncthreads();
-    BbWideGroups<T, L0 + R>::run(tile, s_lo, u, lane, warp, tw);
+    BbWideGroups<T, L0 + R, FIRST>::run(tile, s_lo, u, lane, warp, tw, zero);
   }
 };
-template <int T>
-struct BbWideGroups<T, T> {
-  static __device__ __forceinline__ void run(uint32_t*, int, uint32_t, uint32_t, uint32_t, const uint2*) {}
+template <int T, int FIRST>
+struct BbWideGroups<T, T, FIRST> {
+  static __device__ __forceinline__ void run(uint32_t*, int, uint32_t, uint32_t, uint32_t, const uint2*, int) {}
 };
 
-template <int T>
+// FIRST: 0 a later pass; the first one with blowup 2 (1) or another (2).  The first
+// pass's load makes the copies that its first log2_c layers would; with blowup 2
+// which layers are left is known at compile time.  Measured on GB300, 2^20 rows x
+// 256, seven layers: first pass 813 us with zero rows loaded, converted and
+// multiplied, 652 with the copies and a runtime test per layer, 538 as it is; a
+// later pass 505 and, with outputs left below 2p (bb_butterfly), 501.
+template <int T, int FIRST>
 __global__ void __launch_bounds__(256) bb_dft_wide_kernel(const uint32_t* __restrict__ m, uint32_t* cw, BbPass p,
                                                          const uint2* __restrict__ tw, uint32_t* bad) {
   extern __shared__ uint32_t tile[];
@@ -508,23 +529,31 @@ __global__ void __launch_bounds__(256) bb_dft_wide_kernel(const uint32_t* __rest
   const bool col_ok = c < p.w;
   const size_t w = p.w;
   const size_t step = ((size_t)8 << s_lo) * w;  // words between a thread's consecutive tile rows
-  if (p.first) {  // spread rows: tile row a holds data row (x0 + a) >> log2_c when its low log2_c bits are 0
-    const uint32_t cmask = (1u << p.log2_c) - 1u;
+  int zero = 0;
+  if (FIRST) {
+    // Spread rows: row x holds data row x >> log2_c where its low log2_c bits are 0,
+    // else zero, so each of the first log2_c layers adds a zero row: it copies row a
+    // to a + 2^l.  The load writes those copies (s_lo = 0).
+    zero = FIRST == 1 ? 1 : p.log2_c < T ? p.log2_c : T;
+    const uint32_t nsrc = kRows >> zero, rep = 1u << zero;
+    const uint64_t cmask = ((uint64_t)1 << p.log2_c) - 1;
 #pragma unroll 1
-    for (uint32_t k0 = 0; k0 < kPer; k0 += kBatch) {
+    for (uint32_t i0 = warp; i0 < nsrc; i0 += 8 * kBatch) {
       uint32_t v[kBatch];
 #pragma unroll
       for (uint32_t k = 0; k < kBatch; ++k) {
-        const uint32_t a = warp + 8u * (k0 + k);
-        const uint64_t x = x0 + a;
-        v[k] = 0;
-        if ((kRows >= 8 || a < kRows) && col_ok && ((uint32_t)x & cmask) == 0) v[k] = m[(x >> p.log2_c) * w + c];
+        const uint32_t i = i0 + 8u * k;
+        const uint64_t x = x0 + ((uint64_t)i << zero);
+        v[k] = (i < nsrc && col_ok && (x & cmask) == 0) ? m[(x >> p.log2_c) * w + c] : 0u;
       }
 #pragma unroll
       for (uint32_t k = 0; k < kBatch; ++k) {
-        const uint32_t a = warp + 8u * (k0 + k);
+        const uint32_t i = i0 + 8u * k;
+        if (i >= nsrc) break;
         if (v[k] >= bb::P) atomicOr(bad, 1u);
-        if (kRows >= 8 || a < kRows) tile[(a << 5) | lane] = bb::to_mont(v[k]);
+        const uint32_t y = bb::to_mont(v[k]);
+        uint32_t* dst = tile + ((i << zero) << 5) + lane;
+        for (uint32_t q = 0; q < rep; ++q) dst[q << 5] = y;
       }
     }
   } else {
@@ -546,7 +575,7 @@ __global__ void __launch_bounds__(256) bb_dft_wide_kernel(const uint32_t* __rest
     }
   }
   __syncthreads();
-  BbWideGroups<T, 0>::run(tile, s_lo, u, lane, warp, tw);
+  BbWideGroups<T, 0, FIRST>::run(tile, s_lo, u, lane, warp, tw, zero);
   if (col_ok) {
     uint32_t* dst = cw + (x0 + ((size_t)warp << s_lo)) * w + c;
 #pragma unroll 4
@@ -994,6 +1023,17 @@ cudaError_t bb_launch_tinv(const uint32_t* ts, uint32_t* tinv, size_t n, uint32_
   return cudaGetLastError();
 }
 
+template <int T>
+static void bb_dft_wide(unsigned grid, size_t sh, cudaStream_t st, const uint32_t* m, uint32_t* cw, const BbPass& p,
+                        const uint2* tw, uint32_t* bad) {
+  if (!p.first)
+    bb_dft_wide_kernel<T, 0><<<grid, 256, sh, st>>>(m, cw, p, tw, bad);
+  else if (p.log2_c == 1)
+    bb_dft_wide_kernel<T, 1><<<grid, 256, sh, st>>>(m, cw, p, tw, bad);
+  else
+    bb_dft_wide_kernel<T, 2><<<grid, 256, sh, st>>>(m, cw, p, tw, bad);
+}
+
 cudaError_t bb_launch_encode(const uint32_t* m, uint32_t* cw, int d, int log2_c, int log2_k0, int generic, size_t w,
                              const uint2* tw, uint32_t* bad, cudaStream_t st, const cudaEvent_t* slice_ready,
                              int slices) {
@@ -1078,14 +1118,14 @@ cudaError_t bb_launch_encode(const uint32_t* m, uint32_t* cw, int d, int log2_c,
     const size_t sh = pp.words * sizeof(uint32_t);
     if (p.lc == 5) {  // wider than 16 columns: tiles of whole 32-column runs (T <= 8)
       switch (p.T) {
-        case 1: bb_dft_wide_kernel<1><<<grid, 256, sh, st>>>(m, cw, p, tw, bad); break;
-        case 2: bb_dft_wide_kernel<2><<<grid, 256, sh, st>>>(m, cw, p, tw, bad); break;
-        case 3: bb_dft_wide_kernel<3><<<grid, 256, sh, st>>>(m, cw, p, tw, bad); break;
-        case 4: bb_dft_wide_kernel<4><<<grid, 256, sh, st>>>(m, cw, p, tw, bad); break;
-        case 5: bb_dft_wide_kernel<5><<<grid, 256, sh, st>>>(m, cw, p, tw, bad); break;
-        case 6: bb_dft_wide_kernel<6><<<grid, 256, sh, st>>>(m, cw, p, tw, bad); break;
-        case 7: bb_dft_wide_kernel<7><<<grid, 256, sh, st>>>(m, cw, p, tw, bad); break;
-        case 8: bb_dft_wide_kernel<8><<<grid, 256, sh, st>>>(m, cw, p, tw, bad); break;
+        case 1: bb_dft_wide<1>(grid, sh, st, m, cw, p, tw, bad); break;
+        case 2: bb_dft_wide<2>(grid, sh, st, m, cw, p, tw, bad); break;
+        case 3: bb_dft_wide<3>(grid, sh, st, m, cw, p, tw, bad); break;
+        case 4: bb_dft_wide<4>(grid, sh, st, m, cw, p, tw, bad); break;
+        case 5: bb_dft_wide<5>(grid, sh, st, m, cw, p, tw, bad); break;
+        case 6: bb_dft_wide<6>(grid, sh, st, m, cw, p, tw, bad); break;
+        case 7: bb_dft_wide<7>(grid, sh, st, m, cw, p, tw, bad); break;
+        case 8: bb_dft_wide<8>(grid, sh, st, m, cw, p, tw, bad); break;
         default: return cudaErrorInvalidValue;
       }
     } else if (p.lu + p.lc == 5) {  // a warp's lanes are one row run: registers take 4 layers per round trip

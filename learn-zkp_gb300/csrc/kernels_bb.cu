@@ -687,53 +687,77 @@ __global__ void __launch_bounds__(kCombRows, 6) bb_combine_kernel(const uint32_t
 }
 
 // ---- column evaluations (basefold.rs:126-131) ---------------------------------
-// Lane = column (32 per blockIdx.y), warps and blocks over the rows; the data
-// stay canonical and the eq table is Montgomery.
-// Products are summed unreduced: a word v is first brought below 2^32 - p by
-// one conditional subtraction (v mod p for every 32-bit word), each product
-// eq R v (eq in Montgomery form) is then below 4.6e18, and a 64-bit sum is
-// folded to hi (2^32 mod p) + lo (below 1.2e18) after every two rows, so three
-// products never overflow it.  A thread's sum is congruent to R sum eq v;
-// one reduction mod p and one Montgomery reduction give its canonical part.
-__global__ void __launch_bounds__(256) bb_eval_cols_kernel(const uint32_t* __restrict__ eq,
+// Lane = COLS columns (32 COLS per blockIdx.y), warps and blocks over the rows; the
+// data stay canonical and the eq table is Montgomery.
+// Products are summed unreduced: a word v is first brought below p by two
+// conditional subtractions (v mod p for every 32-bit word), each product eq R v (eq
+// in Montgomery form) is then below 4.1e18, and a 64-bit sum is folded to
+// hi (2^32 mod p) + lo (below 1.2e18) after every four rows, so four products
+// never overflow it.  A thread's sum is congruent to R sum eq v; one reduction mod p
+// and one Montgomery reduction give its canonical part.  Bound by the wide
+// multiplier (6.25 products and folds a word); with one column a lane the five eq
+// words a row, loaded by every warp, and the addresses cost as much.  Measured on
+// GB300, 2^19 rows x 256: 187 us, 334 with one column a lane, eight rows in flight and
+// a fold every two; without the three blocks per SM (80 registers) 262, with four
+// 206, with eight rows in flight 183 (but 2^16 rows 36.6 instead of 34.8).
+template <int COLS>
+__global__ void __launch_bounds__(256, COLS == 1 ? 6 : 3) bb_eval_cols_kernel(const uint32_t* __restrict__ eq,
                                                           const uint32_t* __restrict__ data, size_t rows, uint32_t w,
                                                           unsigned long long* acc) {
+  constexpr int kFlight = COLS == 1 ? 8 : 4;  // rows whose loads are in flight before they are used
   __shared__ unsigned long long part[8][5][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t c = blockIdx.y * 32 + lane;
-  unsigned long long s[5] = {0, 0, 0, 0, 0};
-  auto fold = [&]() {
-#pragma unroll
-    for (int k = 0; k < 5; ++k) s[k] = (s[k] >> 32) * (unsigned long long)bb::MONT_ONE + (uint32_t)s[k];
-  };
+  const uint32_t c = (blockIdx.y * 32 + lane) * COLS;
+  unsigned long long s[COLS][5] = {};
   if (c < w) {
     const size_t step = (size_t)gridDim.x * 8;
-    for (size_t r = (size_t)blockIdx.x * 8 + warp; r < rows; r += 8 * step) {
-      uint32_t v[8];  // eight rows' loads in flight before they are used
+    for (size_t r = (size_t)blockIdx.x * 8 + warp; r < rows; r += kFlight * step) {
+      uint32_t v[kFlight][COLS];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = r + q * step < rows ? data[(r + q * step) * w + c] : 0u;
+      for (int q = 0; q < kFlight; ++q) {
+        const bool there = r + q * step < rows;
+        const uint32_t* p = data + (there ? r + q * step : r) * w + c;
+        if (COLS == 4) {
+          const uint4 t = *reinterpret_cast<const uint4*>(p);
+          v[q][0] = t.x, v[q][COLS > 1 ? 1 : 0] = t.y, v[q][COLS > 2 ? 2 : 0] = t.z, v[q][COLS > 3 ? 3 : 0] = t.w;
+        } else {
+          v[q][0] = *p;
+        }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        if (r + q * step >= rows) break;
-        const size_t rr = r + q * step;
-        const uint32_t x = bb::umin(v[q], v[q] - bb::P);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) s[k] += (unsigned long long)eq[5 * rr + k] * x;
-        if (q & 1) fold();
+        for (int m = 0; m < COLS; ++m) v[q][m] = there ? v[q][m] : 0u;
       }
-      fold();
+#pragma unroll
+      for (int q = 0; q < kFlight; ++q) {
+        const size_t rr = r + q * step < rows ? r + q * step : r;
+        uint32_t e[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) e[k] = eq[5 * rr + k];
+#pragma unroll
+        for (int m = 0; m < COLS; ++m) {
+          uint32_t x = bb::umin(v[q][m], v[q][m] - bb::P);
+          x = bb::umin(x, x - bb::P);
+#pragma unroll
+          for (int k = 0; k < 5; ++k) {
+            s[m][k] += (unsigned long long)e[k] * x;
+            if ((q & 3) == 3) s[m][k] = (s[m][k] >> 32) * (unsigned long long)bb::MONT_ONE + (uint32_t)s[m][k];
+          }
+        }
+      }
     }
   }
 #pragma unroll
-  for (int k = 0; k < 5; ++k) part[warp][k][lane] = bb::reduce(s[k] % bb::P);
-  __syncthreads();
-  if (warp == 0 && c < w) {
+  for (int m = 0; m < COLS; ++m) {
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
+    for (int k = 0; k < 5; ++k) part[warp][k][lane] = bb::reduce(s[m][k] % bb::P);
+    __syncthreads();
+    for (int t = threadIdx.x; t < 5 * 32; t += blockDim.x) {
+      const int k = t >> 5, l = t & 31;
+      const uint32_t col = (blockIdx.y * 32 + l) * COLS + m;
       unsigned long long v = 0;
-      for (int q = 0; q < 8; ++q) v += part[q][k][lane];
-      if (v) atomicAdd(acc + 5 * (size_t)c + k, v);
+      for (int q = 0; q < 8; ++q) v += part[q][k][l];
+      if (col < w && v) atomicAdd(acc + 5 * (size_t)col + k, v);
     }
+    __syncthreads();
   }
 }
 
@@ -1223,15 +1247,16 @@ cudaError_t bb_launch_combine(const uint32_t* src, size_t rows, size_t w, const 
   return cudaGetLastError();
 }
 
-cudaError_t bb_launch_eval_cols(const uint32_t* eq, const uint32_t* data, size_t rows, size_t w,
-                                unsigned long long* acc, cudaStream_t st) {
+template <int COLS>
+static cudaError_t bb_eval_cols(const uint32_t* eq, const uint32_t* data, size_t rows, size_t w, unsigned long long* acc,
+                                cudaStream_t st) {
   size_t bx = (rows + 63) / 64;  // at least 8 rows per warp
-  const size_t by = (w + 31) / 32;
+  const size_t by = (w + 32 * COLS - 1) / (32 * COLS);
   // one wave: as many blocks as the SMs hold at once, spread over the column
   // groups (blocks per SM depend on the kernel only; SMs on the current device)
   static const int per_sm = [] {
     int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, bb_eval_cols_kernel, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, bb_eval_cols_kernel<COLS>, 256, 0);
     return b > 0 ? b : 4;
   }();
   int dev = 0, sms = 0;
@@ -1241,9 +1266,16 @@ cudaError_t bb_launch_eval_cols(const uint32_t* eq, const uint32_t* data, size_t
   if (cap < 1) cap = 1;
   if (bx > cap) bx = cap;
   if (bx < 1) bx = 1;
-  bb_eval_cols_kernel<<<dim3((unsigned)bx, (unsigned)by), 256, 0, st>>>(eq, data, rows, (uint32_t)w, acc);
+  bb_eval_cols_kernel<COLS><<<dim3((unsigned)bx, (unsigned)by), 256, 0, st>>>(eq, data, rows, (uint32_t)w, acc);
   count_launch();
   return cudaGetLastError();
+}
+
+cudaError_t bb_launch_eval_cols(const uint32_t* eq, const uint32_t* data, size_t rows, size_t w,
+                                unsigned long long* acc, cudaStream_t st) {
+  // four columns a lane where every row starts on 16 bytes and fills a warp
+  const bool wide = w % 4 == 0 && w >= 128 && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
+  return wide ? bb_eval_cols<4>(eq, data, rows, w, acc, st) : bb_eval_cols<1>(eq, data, rows, w, acc, st);
 }
 
 cudaError_t bb_launch_eq_table(uint32_t* ev, const bb::E5* x, int n, cudaStream_t st) {

@@ -286,7 +286,11 @@ int bf_verify(const bf_pcs* pcs, const uint8_t root[32], const uint8_t* point, c
  * of every query run on the GPU (the pcs must be on a device).  Each job's
  * `result` and challenger end exactly as bf_verify's would.  Returns BF_OK or
  * a negative BF_ERR_* (nothing is verified then).  Calls on one pcs are
- * serialized. */
+ * serialized.  Where the device shares the host's page tables it reads the
+ * paths of an 8-byte aligned proof in the caller's memory: every proof must
+ * stay mapped and readable until the call returns.  Bytes changed meanwhile
+ * (a shared mapping) cannot make a false opening pass: no two checks of an
+ * opening read the same byte of the caller's memory. */
 typedef struct bf_verify_job {
   const uint8_t* root;        /* 32-byte commitment */
   const uint8_t* point;       /* num_vars field elements */

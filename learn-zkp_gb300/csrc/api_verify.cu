@@ -285,9 +285,15 @@ struct VJob {
   std::vector<uint64_t> idx;   // query positions
   size_t nq_dev = 0;
   int after = BF_VERIFY_OK;  // status of query nq_dev, decided by its structure (or OK: none left)
-  uint64_t elems = 0;  // device image offset
-  // where the kernels read the proof: the caller's bytes in place, or (staged)
-  // their copy at this device image offset
+  // The folded-codeword roots and the final polynomial, copied out of the proof
+  // once: what the transcript observed is what the queries are checked against,
+  // whatever happens to the caller's bytes meanwhile.
+  std::vector<uint8_t> bound;
+  const uint8_t* roots() const { return bound.data(); }
+  const uint8_t* final_poly() const { return bound.data() + 32 * lay.pi_n; }
+  uint64_t elems = 0, rows = 0;  // device image and scratch offsets
+  // where the kernels read rows, paths and siblings: the caller's bytes in place, or
+  // (staged) their copy at this device image offset
   uint64_t proof = 0;
   bool staged = false;
 };
@@ -301,6 +307,9 @@ void verify_host_part(const bf_pcs* p, const bf_verify_job& jb, VJob& v) {
     return;
   }
   const Layout& lay = v.lay;
+  v.bound.resize(32 * lay.pi_n + 16 * lay.final_n);
+  if (lay.pi_n) std::memcpy(v.bound.data(), pf + lay.pi_off, 32 * lay.pi_n);
+  if (lay.final_n) std::memcpy(v.bound.data() + 32 * lay.pi_n, pf + lay.final_off, 16 * lay.final_n);
   bfh::Challenger& ch = jb.challenger->c;
   const u128 ONE = bfh::one();
   const int d = p->d, L = p->L, log2_c = p->log2_c;
@@ -320,7 +329,7 @@ void verify_host_part(const bf_pcs* p, const bf_verify_job& jb, VJob& v) {
   u128 sc = claim;
   v.rounds_x.resize(d);
   for (int k = 0; k < d; ++k) {
-    ch.observe(pf + lay.pi_off + 32 * (size_t)k, 32);
+    ch.observe(v.roots() + 32 * (size_t)k, 32);
     if (lay.rp_n[k] != 2) {
       v.status = BF_VERIFY_MALFORMED;
       return;
@@ -333,14 +342,14 @@ void verify_host_part(const bf_pcs* p, const bf_verify_job& jb, VJob& v) {
     sc = horner(rp, 3, x);
     v.rounds_x[k] = x;
   }
-  for (uint64_t i = 0; i < lay.final_n; ++i) ch.observe_elem(bfh::load(pf + lay.final_off + 16 * i));
+  for (uint64_t i = 0; i < lay.final_n; ++i) ch.observe_elem(bfh::load(v.final_poly() + 16 * i));
   if (lay.final_n != 1) {
     v.status = BF_VERIFY_MALFORMED;
     return;
   }
   u128 eqv = ONE;  // eq_eval(point, r) with r[k] the challenge of round d-1-k
   for (int k = 0; k < d; ++k) eqv = bfh::mul(eqv, ONE ^ bfh::load(jb.point + 16 * k) ^ v.rounds_x[d - 1 - k]);
-  if (bfh::mul(bfh::load(pf + lay.final_off), eqv) != sc) {
+  if (bfh::mul(bfh::load(v.final_poly()), eqv) != sc) {
     v.status = BF_VERIFY_INVALID_FINAL_POLY;
     return;
   }
@@ -389,6 +398,8 @@ void parallel_jobs(size_t count, F&& f) {
   for (auto& x : th) x.join();
 }
 
+inline void touch(const uint8_t* p) { (void)*static_cast<const volatile uint8_t*>(p); }
+
 inline uint64_t align16(uint64_t x) { return (x + 15) & ~(uint64_t)15; }
 
 }  // namespace
@@ -412,11 +423,18 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
   // scratch and flags.  Every job owns Q query slots and a fixed element range,
   // so one pass over the jobs fills it; slots a job does not use (queries decided
   // on the host) are marked inactive.  A device that shares the host's page
-  // tables reads the proofs where the caller has them (8-byte aligned; every
+  // tables reads the openings where the caller has the proof (8-byte aligned; every
   // field of a proof then is): each byte crosses once, as the paths are hashed,
   // instead of being copied to pinned memory and from there to the device
-  // (64 proofs of 2^14, 83 MB, GB300: 3.5 -> 2.9 ms a batch, 7.2 -> 3.5 ms the
-  // first one of a pcs, which no longer pins 83 MB).
+  // (GB300: 64 proofs of 2^14, 83 MB, 2.1 ms a batch in place, 2.3 copied; 16 of 2^12
+  // x 256, 36 MB, 1.4 and 1.7; the first batch of a pcs, which pins no proof, 3.6 and
+  // 7.2 ms).
+  // Whoever can still write the proof must not be able to show two checks two
+  // values, so each byte that a check depends on is fetched once: the lengths by the
+  // host (parse_layout), the roots and the final polynomial by the host too, which
+  // hands what the transcript observed to the device; an opened row and a sibling by
+  // the fold, which hands them to the path checks (rows, pairs); a path digest by its
+  // path's check.
   const uint64_t nq = count * Q;
   if (nq > 0xffffffffull / (uint64_t)(d + 2)) return fail(BF_ERR_ARG, "too many queries in one batch");
   std::vector<VJob> v(count);
@@ -425,8 +443,8 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
   const uint64_t off_rounds = align16(off_queries + sizeof(bf::VerifyQuery) * nq);
   uint64_t cur = align16(off_rounds + sizeof(bf::VerifyRound) * nq * d);
   for (size_t j = 0; j < count; ++j) {
-    v[j].elems = cur;
-    cur += 32 + 16 * (uint64_t)d + (jobs[j].width > 1 ? 16 * (uint64_t)jobs[j].width : 0);
+    v[j].elems = cur;  // root, challenges, final polynomial, folded-codeword roots, scalars
+    cur += 32 + 16 * (uint64_t)d + 16 + 32 * (uint64_t)d + (jobs[j].width > 1 ? 16 * (uint64_t)jobs[j].width : 0);
   }
   const uint64_t header = align16(cur);  // what the kernels read besides the proofs
   cur = header;
@@ -437,7 +455,13 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
     cur = align16(cur + jobs[j].proof_len);
   }
   const uint64_t image = cur;
-  const uint64_t off_pairs = image, off_flags = off_pairs + 32 * nq * d;
+  const uint64_t off_pairs = image;
+  cur = off_pairs + 32 * nq * d;
+  for (size_t j = 0; j < count; ++j) {
+    v[j].rows = cur;  // of the opened rows that are read, all in the proof
+    cur = align16(cur + std::min<uint64_t>(16 * (uint64_t)jobs[j].width * Q, jobs[j].proof_len));
+  }
+  const uint64_t off_flags = cur;
   const uint64_t flag_bytes = nq * (uint64_t)(d + 2);
   const uint64_t dev_bytes = align16(off_flags + flag_bytes);
   if (nq > 0) {
@@ -459,18 +483,22 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
     const uint64_t proof = x.staged ? dev + x.proof : reinterpret_cast<uint64_t>(jb.proof);
     bf::VerifyJob rec{};
     rec.root = dev + x.elems;
-    rec.challenges = dev + x.elems + 32;
-    rec.scalars = dev + x.elems + 32 + 16 * (uint64_t)d;
-    rec.pi_comms = proof + (active ? lay.pi_off : 0);
-    rec.final_poly = proof + (active ? lay.final_off : 0);
+    rec.challenges = rec.root + 32;
+    rec.final_poly = rec.challenges + 16 * (uint64_t)d;
+    rec.pi_comms = rec.final_poly + 16;
+    rec.scalars = rec.pi_comms + 32 * (uint64_t)d;
+    rec.rows = dev + x.rows;
     rec.width = (uint32_t)jb.width;
     std::memcpy(h + off_jobs + sizeof(rec) * j, &rec, sizeof(rec));
     if (active) {
       uint8_t* e = h + x.elems;
       std::memcpy(e, jb.root, 32);
       for (int k = 0; k < d; ++k) bfh::store(e + 32 + 16 * k, x.rounds_x[k]);
+      std::memcpy(e + (rec.final_poly - rec.root), x.final_poly(), 16);
+      std::memcpy(e + (rec.pi_comms - rec.root), x.roots(), 32 * (size_t)d);
       if (jb.width > 1)
-        for (size_t w = 0; w < jb.width; ++w) bfh::store(e + 32 + 16 * (size_t)d + 16 * w, x.scalars[w]);
+        for (size_t w = 0; w < jb.width; ++w) bfh::store(e + (rec.scalars - rec.root) + 16 * w, x.scalars[w]);
+      touch(jb.proof + jb.proof_len - 1);
     }
     for (uint64_t q = 0; q < Q; ++q) {
       bf::VerifyQuery vq{};
@@ -479,6 +507,11 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
       if (q < active) {
         const Layout::Open& o = lay.open[q];
         vq.idx = x.idx[q];
+        // Every page of the proof is read by the host before the device reads it, so
+        // memory that cannot be read fails here, as in a copy: of what parse_layout
+        // skips, only rows and the last path's end can hold a page's every byte.
+        for (uint64_t at = 0; at < 16 * (uint64_t)jb.width; at += 4096) touch(jb.proof + o.leaves + at);
+        vq.slot = (uint32_t)q;
         vq.leaves = proof + o.leaves;
         vq.path = proof + o.path;
         for (int k = 0; k < d; ++k) {
@@ -510,10 +543,12 @@ extern "C" int bf_verify_batch(bf_pcs* p, bf_verify_job* jobs, size_t count) {
     vp.nq = (uint32_t)nq;
     vp.d = d;
     vp.log2_c = p->log2_c;
-    CU(bf::launch_verify(vp, st));
     uint8_t* flags = h + image;
-    CU(cudaMemcpyAsync(flags, dv + off_flags, flag_bytes, cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
+    cudaError_t e = bf::launch_verify(vp, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(flags, dv + off_flags, flag_bytes, cudaMemcpyDeviceToHost, st);
+    const cudaError_t done = cudaStreamSynchronize(st);  // also after an error: the proofs are the caller's again
+    CU(e);
+    CU(done);
     // per job, the first query that fails decides (basefold.rs:284-322 checks
     // them in order): a bad path is an Mmcs error, a bad chain InvalidQuery
     for (size_t j = 0; j < count; ++j) {

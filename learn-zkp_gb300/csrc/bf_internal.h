@@ -245,22 +245,24 @@ struct TailParams {
 cudaError_t launch_open_tail(const TailParams& p, cudaStream_t st);
 
 // ---- Basefold::verify of many proofs (basefold.rs:284-320) on the device.
-// Fields are addresses the device can read, multiples of 8 (device memory, or the
-// caller's host memory where the device shares the host's page tables).  All
-// proofs share one pcs (num_vars d, blowup 2^log2_c) and are checked query by query.
+// Fields are addresses the device can read, multiples of 8: device memory, or for a
+// query's leaves, path and siblings the caller's host memory where the device shares
+// the host's page tables.  All proofs share one pcs (num_vars d, blowup 2^log2_c) and
+// are checked query by query.
 struct VerifyJob {
   uint64_t root;        // 32-byte commitment
   uint64_t pi_comms;    // the proof's d folded-codeword roots, 32 bytes apart
   uint64_t final_poly;  // the proof's final polynomial (one element)
   uint64_t challenges;  // round challenges in round order (16 bytes each)
   uint64_t scalars;     // width > 1: the eq scalars of the columns
+  uint64_t rows;        // scratch: the opened rows as the fold read them, query after query
   uint32_t width;
   uint32_t pad;
 };
 constexpr uint32_t kVerifyInactive = 0xffffffffu;  // a query slot with nothing to check
 struct VerifyQuery {
   uint32_t job;     // kVerifyInactive: an unused slot
-  uint32_t pad;
+  uint32_t slot;    // its number among the job's queries
   uint64_t idx;     // sampled position in the codeword
   uint64_t leaves;  // the opened row (16*width bytes)
   uint64_t path;    // its L sibling digests

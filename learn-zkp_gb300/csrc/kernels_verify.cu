@@ -10,7 +10,7 @@
 //  * verify_fold_kernel (one thread per query) runs the chain — the leaf row's
 //    scalar combination, then per round the pair [folded, sibling] placed by
 //    the index bit and the interpolation of binary_reed_solomon.rs:98-109 —
-//    writes each round's pair and compares the last value with the final
+//    writes the row and each round's pair for the path checks and compares the last value with the final
 //    polynomial (encode0 repeats it, binary_reed_solomon.rs:63-65);
 //  * verify_path_kernel (one thread per path) hashes a leaf and walks its
 //    sibling path to the root (MerkleTreeMmcs::verify_batch: leaf =
@@ -37,6 +37,19 @@ __device__ __forceinline__ uint4 load_elem8(uint64_t at) {
   return make_uint4(a.x, a.y, b.x, b.y);
 }
 
+// Rows, siblings and path digests may lie in memory that someone still writes: their
+// loads are volatile asm, which the compiler neither repeats nor splits, so a value
+// has been read once wherever it is used.
+__device__ __forceinline__ uint2 load8_once(uint64_t at) {
+  uint2 v;
+  asm volatile("ld.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(at));
+  return v;
+}
+__device__ __forceinline__ uint4 load_elem8_once(uint64_t at) {
+  const uint2 a = load8_once(at), b = load8_once(at + 8);
+  return make_uint4(a.x, a.y, b.x, b.y);
+}
+
 // A digest stored as bytes: its four lanes as they are, and interleaved as the
 // tree hashes use them.
 struct RawDigest {
@@ -49,8 +62,7 @@ struct RawDigest {
   }
 };
 __device__ __forceinline__ RawDigest load_digest_raw(uint64_t at) {
-  const uint2* p = reinterpret_cast<const uint2*>(at);
-  return RawDigest{{p[0], p[1], p[2], p[3]}};
+  return RawDigest{{load8_once(at), load8_once(at + 8), load8_once(at + 16), load8_once(at + 24)}};
 }
 __device__ __forceinline__ Digest load_digest_bytes(uint64_t at) { return load_digest_raw(at).interleaved(); }
 
@@ -97,12 +109,16 @@ __global__ void __launch_bounds__(128) verify_fold_kernel(VerifyParams P) {
   }
   const VerifyJob J = P.jobs[Q.job];
   uint4 folded;
+  uint4* row = reinterpret_cast<uint4*>(J.rows) + (uint64_t)J.width * Q.slot;  // for the path's leaf
   if (J.width == 1) {
-    folded = load_elem8(Q.leaves);  // scalars = [ONE] (basefold.rs:253-254)
+    row[0] = folded = load_elem8_once(Q.leaves);  // scalars = [ONE] (basefold.rs:253-254)
   } else {
     folded = make_uint4(0, 0, 0, 0);
-    for (uint32_t w = 0; w < J.width; ++w)
-      folded = gf_add(folded, gf_mul(load_elem8(J.scalars + 16ull * w), load_elem8(Q.leaves + 16ull * w)));
+    for (uint32_t w = 0; w < J.width; ++w) {
+      const uint4 e = load_elem8_once(Q.leaves + 16ull * w);
+      row[w] = e;
+      folded = gf_add(folded, gf_mul(load_elem8(J.scalars + 16ull * w), e));
+    }
   }
   const int d = P.d;
   for (int k = 0; k < d; ++k) {
@@ -111,7 +127,7 @@ __global__ void __launch_bounds__(128) verify_fold_kernel(VerifyParams P) {
     const uint64_t ii = Q.idx & ((1ull << bits) - 1);
     const bool sib_left = ((Q.idx >> bits) & 1) != 0;  // the sibling is values[0]
     const VerifyRound R = P.rounds[(size_t)q * d + k];
-    const uint4 s = load_elem8(R.sibling);
+    const uint4 s = load_elem8_once(R.sibling);
     uint4 v0 = sib_left ? s : folded, v1 = sib_left ? folded : s;
     P.pairs[2 * ((size_t)q * d + k)] = v0;
     P.pairs[2 * ((size_t)q * d + k) + 1] = v1;
@@ -144,7 +160,8 @@ __global__ void __launch_bounds__(128) verify_path_kernel(VerifyParams P) {
     index = Q.idx;
     path = Q.path;
     root = load_digest_bytes(J.root);
-    cur = J.width == 1 ? hash_elem(load_elem8(Q.leaves)) : hash_row(Q.leaves, J.width);
+    const uint64_t row = J.rows + 16ull * J.width * Q.slot;
+    cur = J.width == 1 ? hash_elem(load_elem8(row)) : hash_row(row, J.width);
   } else {  // folded codeword of round k: leaf = keccak256(values[0] || values[1])
     const int k = (int)level - 1;
     log_h = P.log2_c + P.d - 1 - k;

@@ -35,7 +35,10 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, s
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  // reported here: left as the thread's last error, it would fail the next launch that reads that
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
 }
 
 }  // namespace bf

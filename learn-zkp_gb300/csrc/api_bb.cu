@@ -3,9 +3,9 @@
 // (poly-commit/src/basefold.rs, poly-commit/src/basefold/code/reed_solomon.rs).
 //
 // The GPU holds every array (evaluations, codeword, folded codewords, trees,
-// eq tables); the host runs the transcript and the O(num_vars) sumcheck
-// scalars, reading 96 bytes back per open round (the folded-codeword root and
-// the round's sum).
+// eq tables) and runs an open's rounds with their transcript (kernels_bb_tail.cu)
+// without a wait; the host makes the batching scalars and the rounds' constants
+// before them and reads the records back once, then samples the query positions.
 #include <cuda_runtime.h>
 
 #include <algorithm>

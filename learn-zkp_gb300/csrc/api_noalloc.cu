@@ -1,7 +1,7 @@
 // libbasefold_gpu.so: multilinear evaluation without any allocation.
 //
-// bf_eval needs scratch for the chain of variable fixings and takes it from
-// device memory it allocates.  Some callers cannot allocate at that point:
+// bf_eval needs scratch (eq tables, or a chain of variable fixings) and takes it
+// from device memory it allocates.  Some callers cannot allocate at that point:
 // a proving service that has carved all device memory into fixed per-request
 // slots for admission control (an extra cudaMalloc would fail or break its
 // accounting), or a latency-critical loop where cudaMalloc/cudaFree would
@@ -78,8 +78,9 @@ extern "C" int bf_eval_noalloc(const void* d_evals, int num_vars, const uint8_t*
   TRY(scratch_for_current_device(&scratch));
   // MultiPoly::evaluate (multilinear.rs:124-141): fix the top variable with
   // the last coordinate, repeatedly — the large levels one launch each, the
-  // last (at most kEvalTailMaxVars) in one block, as bf_eval does.  Every
-  // level writes the entries the next one reads, so nothing in the scratch
+  // last (at most kEvalTailMaxVars) in one block, as bf_eval does below
+  // kEvalSplitMin variables (from there on it sums against the point's eq table: the
+  // same value).  Every level writes the entries the next one reads, so nothing in the scratch
   // needs clearing between calls.
   auto coord = [&](int k) {
     uint4 r;

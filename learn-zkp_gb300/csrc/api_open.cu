@@ -66,8 +66,9 @@ struct bf_open_session {
   uint8_t* w_rec = nullptr;
   bool resident_pending = false;   // a device-transcript open is in flight
   bool gather_pending = false;     // query openings in flight
-  std::unique_ptr<PinnedBuf> pin;  // [0,64) staging, [64,64+16(w+d)) scalars and point, indices,
-                                   // openings, device-transcript results; inputs at tail_in_off()
+  std::unique_ptr<PinnedBuf> pin;  // [0,64) staging, [64,64+16(w+d)) scalars and point; then indices,
+                                   // openings, device-transcript results; before them, from byte 64
+                                   // on, the inputs (point_off() and on)
   uint64_t* idx_pin = nullptr;
   uint8_t* open_pin = nullptr;
   uint8_t* res_pin = nullptr;

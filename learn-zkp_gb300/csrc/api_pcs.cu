@@ -344,9 +344,12 @@ int commit_enqueue(bf_pcs* p, bf_commitment* cm, const uint4* data, cudaStream_t
 }
 
 // MultiPoly::evaluate (multilinear.rs:124-141) of the commitment's data at
-// `point` (host, d elements) on stream `st`: fix the top variable with the
-// last coordinate, repeatedly, in `scratch` (2^(d-1) elements).  The value
-// lands in value_pin[0..16).
+// `point` (host, d elements; or point_dev) on stream `st`, in `scratch` (2^(d-1)
+// elements).  One polynomial of kEvalSplitMin .. kEvalSplitMax variables: one sum
+// against the point's eq table in two factors, which take 2^((d+1)/2) + 2^(d/2)
+// elements of the scratch, below its last, the value (from d = 5 on).  Otherwise (fewer
+// variables; matrices of more than kEqTableMaxVars): fix the top variable with the
+// last coordinate, repeatedly.  The values land in value_pin.
 int eval_enqueue(bf_pcs* p, const bf_commitment* cm, const uint8_t* point, uint4* scratch, cudaStream_t st,
                  uint8_t* value_pin, const uint4** value_dev, const uint4* point_dev) {
   const int d = p->d;

@@ -1,5 +1,5 @@
-// Internal interface between the host orchestration (api.cu) and the
-// kernels (kernels.cu).  Not part of the public C ABI.
+// Internal interface between the host orchestration (api_*.cu) and the
+// kernels (kernels.cu, kernels_tail.cu, kernels_verify.cu).  Not part of the public C ABI.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -26,12 +26,15 @@ constexpr int kNttMaxT = 12;  // largest shared-memory tile of an NTT pass: 2^12
 struct Tune {
   int ntt_threads = 256;  // threads per block of the shared-memory NTT pass: 128, 256 or 512
   int ntt_max_T = 12;     // butterfly layers per NTT pass (tile 2^T), 6 .. kNttMaxT
-  int top_nodes = 512;    // Merkle levels at or below this many nodes run in one block (64 .. 4096)
+  int top_nodes = 512;    // the tree's last launch takes levels of at most this many nodes (64 .. 4096): one
+                          // block up to 128 nodes, a cluster of eight above
   int tail_log = 8;       // open rounds whose next tree has <= 2^tail_log leaves run in one block (1 .. 11)
-  int subtree_log = 16;   // Merkle levels of 2^10 .. 2^subtree_log nodes run as one launch (10 .. 20)
+  int subtree_log = 16;   // from 2^subtree_log nodes down to top_nodes six to nine levels run as one launch,
+                          // above it each level is a launch (10 .. 20)
   // NTT pass kind: 0 every pass layer by layer in shared memory; 1 tiles of
   // 2^9 .. 2^13 register-blocked; 2 as 0, with the last pass (and its leaf
-  // hashing) warp-specialized; 3 as 0, two-pass encodes with the cosets
+  // hashing) warp-specialized and, for large codewords, the leading layers two
+  // per pass over columns; 3 as 0, two-pass encodes with the cosets
   // pipelined (the next cosets' first pass beside a coset's last pass)
   int ntt_kind = 2;
   int gf_mix = 0;        // NTT passes without hashing: 32 x 32 products per field product from 16-bit pieces (0 .. 4)
@@ -46,9 +49,9 @@ bool tune_valid(const Tune& t);
 // leaves and the first folded-codeword leaves.
 // With `slices` > 0, slice k of the input (rows [k N/slices, (k+1) N/slices))
 // is ready once slice_ready[k] has completed: the first pass waits for each
-// slice before the blocks that read it, its launches alternating between st
-// and st2 (joined back to st through the events ev_a, ev_b) when those are
-// given.  last_a / last_b (when given) are recorded on st around the last
+// slice before the blocks that read it.  Where that pass is a tile pass its
+// launches alternate between st and st2 (joined back to st through the events ev_a,
+// ev_b) when those are given; a column pass's all run on st.  last_a / last_b (when given) are recorded on st around the last
 // pass (the kernel-class timing of the last pass with its leaf hashing).
 cudaError_t launch_encode(const uint4* m, uint4* cw, int n, int log2_c, size_t width, const TwiddleView* tw,
                           cudaStream_t st, uint4* leaves = nullptr, uint4* pair_leaves = nullptr,

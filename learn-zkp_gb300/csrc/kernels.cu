@@ -1780,8 +1780,8 @@ __global__ void __launch_bounds__(64 * K) prod_fix_kernel(PolyPtrs p, size_t hal
 // + 2 (K = 2) or + 7 (K = 3) products of an element pair, come from a
 // shared-memory table of r (GfTab), so the wide multiplier, which bounds
 // prod_fix_kernel in large rounds, is left with the sums' products, and the table's loads run
-// beside it.  One persistent block per SM builds the table (about 3 us) and
-// walks the pairs.  Measured on GB300, clocks per pair and SM: K = 3 67 at 512
+// beside it.  One persistent block per SM builds the table and walks the pairs
+// (start, build and reductions: see prod_tab_min).  Measured on GB300, clocks per pair and SM: K = 3 67 at 512
 // threads (68 at 384, 77 at 256; 95 without the table); K = 2 22 at 768
 // threads (24 at 512; 44).
 using ProdTab = GfTab<6>;
@@ -1832,8 +1832,8 @@ cudaError_t launch_prod_round_sums(const uint4* const* polys, int k, size_t half
   return cudaGetLastError();
 }
 
-// Pairs from which a fix uses the table, whose build takes a launch of few pairs to
-// 18 us (k = 2) or 26 us (k = 3).  Measured on GB300, without and with the table: k =
+// Pairs from which a fix uses the table.  A launch of few pairs takes 18 us (k = 2) or
+// 26 us (k = 3) with it: start, table and reductions.  Measured on GB300, without and with the table: k =
 // 2 18.1 and 18.2 us at 2^16 pairs, 26.9 and 27.2 at 2^17, 47.3 and 35.8 at 2^18; k = 3
 // 19.9 and 26.3 us at 2^15, 30.2 and 26.4 at 2^16, 56.1 and 43.2 at 2^17.
 constexpr size_t prod_tab_min(int k) { return (size_t)1 << (k == 2 ? 18 : 16); }

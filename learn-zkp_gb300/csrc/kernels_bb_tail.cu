@@ -235,7 +235,8 @@ __device__ __forceinline__ void st_e5(uint32_t* p, size_t i, const E5& e) {
 // early: the launch before this one is a tree's, and a block of this grid starts
 // only after every block of that one has waited for all launches before it, among
 // them the ones that wrote the transcript and the sums: those are read (past L1) and
-// the message is made before the wait, which is left for the root alone.
+// the message is made before the wait, which is left for the root alone (the rules:
+// launch.cuh).
 __global__ void __launch_bounds__(32) bb_transcript_round_kernel(BbTranscript* t, const BbRoundConsts* c, int ri,
                                                                 const uint4* root_dev, unsigned long long* sums,
                                                                 int canonical, uint32_t* x_out, uint8_t* rec,
